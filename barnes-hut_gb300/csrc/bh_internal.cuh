@@ -497,8 +497,9 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
 int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2, double kick_h, bool fp64,
                            bool group = false);
 int launch_traverse_learned(bh_context* ctx, double theta, double G, double soft2, double kick_h);
-// FP32 node records (hi/lo centres, G m, topology) from the FP64 records.
-int launch_fp32_nodes(bh_context* ctx, double G);
+// FP32 node records (hi/lo centres, G m, topology) from the FP64 records;
+// fp64: also the FP64 walks' {centre, G m} records (d4).
+int launch_fp32_nodes(bh_context* ctx, double G, bool fp64 = false);
 
 // Device-wide exclusive scan of n int32 values (in may equal out); the
 // total is written to *total (device pointer).  n is read from n_dev when

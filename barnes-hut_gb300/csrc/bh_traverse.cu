@@ -1,35 +1,47 @@
 // Warp-cooperative Barnes-Hut traversal.
 //
-// Replaces computeAccelerations (src/traversal.cpp:13-103).  Each warp owns
-// 32 Morton-consecutive bodies (one per lane) and walks the compressed
-// octree once for all of them.
+// Replaces computeAccelerations (src/traversal.cpp:13-103).
 //
-// BH_MODE_PLAIN_FP64 (exact): the warp runs the reference's depth-first walk
-// over the union of the nodes its lanes need.  Children are pushed in octant
-// order and popped last-in-first-out, exactly as the reference's per-body
-// stack does, so every lane meets its own nodes in the reference's order.
-// A lane that accepts a node the warp still opens marks the stack height;
-// it sits out every node popped above that height (the node's subtree) and
-// rejoins when the stack falls back below it.  Each lane applies the
-// reference's test to its own body: leaf -> accept (own leaf -> skip),
-// else side(depth)^2 < theta^2 r^2 with r the distance to the centre of
-// mass.  Because every lane sees the same node, the node is first classified
-// against the group's bounding box in FP32 (with allowances for rounding):
-// accepted by all, opened by all, or undecided -- only then does each lane
-// run the FP64 test.  Accepted nodes go to a per-lane list in walk order;
-// the lists are evaluated in lockstep (each lane its own next node) with
-// IEEE sqrt and division and no contraction, so every lane adds its terms in
-// the reference's order and the result equals the reference bit for bit.
+// BH_MODE_PLAIN_FP64 (exact): a warp owns 32 / P Morton-consecutive bodies, P
+// lanes to a body, and walks the compressed octree once for all of them.
+//
+// Walk.  The reference's per-body stack pops children last-in-first-out, in
+// descending octant order, so a body meets the nodes it accepts in descending
+// key order.  The warp's stack holds items in that order, the next one on
+// top: nodes still to be tested, and nodes some bodies have accepted.  A pass
+// takes the top 32 items, one per lane, tests the untested ones all at once
+// and puts the children of an opened node in its place; the accepted items in
+// front of the first opened node are next for every body, and go to the
+// bodies' lists.  (One node per pass, as a plain depth-first walk takes them,
+// left the warp waiting on one node record at a time: 34 passes instead of
+// about 950 at 100,003 bodies.)  A node is classified against the bodies' box
+// in FP32 with allowances for rounding: accepted by all, opened by all, or
+// undecided; an undecided one each body tests itself, in FP32 and, where that
+// cannot tell either, in FP64 with the reference's rounding.
+//
+// Evaluation.  Every term is rounded as the reference rounds it and every body
+// adds its terms in the reference's order, so the accelerations are the
+// reference's bit for bit.  P lanes evaluate P consecutive terms of a body;
+// then one lane per component adds them one after the other.  The FP64 pipe
+// bounds this (two lanes per cycle: 16 to 19 cycles of the SM per warp
+// instruction), so the products, the square root and the reciprocal run as
+// integer code beside it (bh_soft64.cuh): 11 FP64 instructions per 32 terms
+// are left (the differences, two squares, the sum of squares and the P
+// additions) instead of 36.
+//
+// Measured (theta 1.05, ms of forces; before: one node per pass, 32 bodies
+// per warp, IEEE operations on the FP64 pipe):
+//   300,149 bodies 12.66 -> 2.96, 19,054 7.71 -> 1.21, 1,000 1.23 -> 0.071.
+#include <climits>
+
 #include "bh_internal.cuh"
+#include "bh_soft64.cuh"
 
 namespace bh {
 namespace {
 
 constexpr int kTravWarps = 4;
 constexpr int kTravThreads = 32 * kTravWarps;
-// A root-to-leaf path has at most 22 nodes (depths strictly increase), each
-// leaving at most 7 siblings behind, plus 8 children of the last node.
-constexpr int kStackCap = 22 * 7 + 8 + 2;
 
 struct TravParams {
     int64_t n;
@@ -38,6 +50,7 @@ struct TravParams {
     const double* pz;
     const int32_t* body_leaf;
     const TreeRec* rec;
+    const double4_32a* d4;  // {cx, cy, cz, G m} per slot
     const float4* A;        // FP32 node records (group tests)
     const float4* B;
     const uint32_t* meta;
@@ -46,6 +59,7 @@ struct TravParams {
     double G;
     double soft2;
     double kick_h;  // > 0: also apply the second half kick v += kick_h * a
+    double one;        // 1.0, as a run-time value: RN(a 1 + b) stays an FMA
     int64_t max_pops;  // upper bound on tree slots (2n)
     double* ax;
     double* ay;
@@ -73,49 +87,106 @@ __device__ inline void fill_side2(const double* bbox, double* side2)
     }
 }
 
-__device__ inline TreeRec load_rec(const TreeRec* __restrict__ rec, int s)
+// Stack items {node | kDecided, lane mask}: a node still to be tested by the
+// lanes of its mask, or (kDecided) one those lanes have accepted.
+constexpr int kDecided = 1 << 31;
+constexpr int kStk = 384;
+// Nodes other than the first undecided one are opened only while the stack
+// stays below this; the first one always may, which adds at most 8 items per
+// level of one root path (21 levels), so the stack never passes kStk.
+constexpr int kSoftStk = kStk - 21 * 8 - 8;
+// FP32 tests: a relative margin on the squares (eight roundings of 2^-24
+// each are below 5e-7) with an absolute one against underflow, and the error
+// of a group-relative distance relative to the coordinates' magnitudes: each
+// component of a difference is off by at most 2^-24 (3 |c| + 2 |r|), so the
+// distance by sqrt(3) times that, below 3.2e-7 (|c| + |r|); the hi + lo
+// split of an absolute coordinate adds 2^-46 of it, so sqrt(3) 2^-46, below
+// 2.5e-14, of the group's distance from the origin (and of |c|).
+constexpr float kMargin = 2e-6f, kTiny = 1e-36f;
+constexpr float kAbsErr = 4e-7f;
+__device__ __forceinline__ bool sure_below(float side2, float theta2, float dist2)  // side^2 < theta^2 dist^2
 {
-    const double2* p = reinterpret_cast<const double2*>(rec + s);
-    const double2 a = __ldg(p);
-    const double2 b = __ldg(p + 1);
-    const int4 c = __ldg(reinterpret_cast<const int4*>(reinterpret_cast<const char*>(rec + s) + 32));
-    TreeRec r;
-    r.cx = a.x; r.cy = a.y; r.cz = b.x; r.m = b.y;
-    r.child = c.x;
-    r.leaf = c.y;
-    r.nchild = (uint8_t)(c.z & 0xFF);
-    r.depth = (uint8_t)((c.z >> 8) & 0xFF);
-    r.top = (uint8_t)((c.z >> 16) & 0xFF);
-    return r;
+    return fmaf(side2, 1.0f + kMargin, kTiny) < theta2 * dist2;
+}
+__device__ __forceinline__ bool sure_above(float side2, float theta2, float dist2)  // side^2 > theta^2 dist^2
+{
+    return side2 * (1.0f - kMargin) > fmaf(theta2, dist2, kTiny);
 }
 
-// Per-lane ordered interaction lists of the exact walk (slots).
-constexpr int kPList = 48;
-constexpr float kMargin = 1e-5f;
-constexpr float kAbsErr = 1e-6f;
+// Shared memory of a block.  Per-body ordered interaction lists: kCap entries
+// per body (P lanes to a body), slots modulo kCap.
+template <int P>
+struct ExactSmem {
+    static constexpr int kBodies = 32 / P;
+    // The first lane of each body: masks of bodies have their bits there.
+    static constexpr unsigned kFirst = 0xffffffffu / ((1u << (P - 1) << 1) - 1u);
+    static constexpr int kCap = 128;  // a power of two, over 33
+    int2 stack[kTravWarps][kStk];
+    int plist[kTravWarps][kCap][kBodies];
+    double term[kTravWarps][3][32];  // the terms of one step of an evaluation
+    // Nodes the box cannot decide: {centre, allowance}, {depth of the test,
+    // node, leaf id or -1}.
+    float4 und[kTravWarps][32];
+    int4 und2[kTravWarps][32];
+    double side2[kMaxDepth + 1];
+    float side2f[kMaxDepth + 1];
+};
 
+// The factor G m / r^3 with the reference's operations, for the terms whose
+// exponents soft::term leaves out.  A call of its own: inlined, it becomes
+// predicated instructions that take the FP64 pipe although no lane needs them.
+__device__ __noinline__ double ieee_scale(double dx, double dy, double dz, double soft2, double gm)
+{
+    const double r2 =
+        __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
+    const double invR = __drcp_rn(__dsqrt_rn(r2));
+    return __dmul_rn(gm, __dmul_rn(__dmul_rn(invR, invR), invR));
+}
+
+// One interaction term with the reference's rounding (src/traversal.cpp:
+// 80-88): displacement, r^2 and the three products sc d.
+template <bool kSoft>
+__device__ __forceinline__ void exact_term(const double4_32a& r, double px, double py, double pz, double soft2,
+                                           bool on, double one, double& tx, double& ty, double& tz)
+{
+    const double dx = fma(r.x, one, -px), dy = fma(r.y, one, -py), dz = fma(r.z, one, -pz);
+    // One of the three squares on the integer pipes balances them with the
+    // FP64 pipe (300,149 bodies: none 3.05 ms, one 2.96, two 2.96, three 3.06).
+    const double zz = soft::square(soft::bits_of(dz));
+    double r2 = fma(fma(__dmul_rn(dx, dx), one, __dmul_rn(dy, dy)), one, zz);
+    if (kSoft) r2 = fma(r2, one, soft2);
+    if (!soft::term(dx, dy, dz, r2, r.w, tx, ty, tz) && on) {
+        const double sc = ieee_scale(dx, dy, dz, soft2, r.w);
+        tx = __dmul_rn(sc, dx);
+        ty = __dmul_rn(sc, dy);
+        tz = __dmul_rn(sc, dz);
+    }
+}
+
+template <int P, bool kSoft>
 __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams p)
 {
-    __shared__ int stack[kTravWarps][kStackCap];
-    __shared__ int plist[kTravWarps][kPList][32];
-    __shared__ double side2[kMaxDepth + 1];
-    __shared__ float side2f[kMaxDepth + 1];
-    fill_side2(p.bbox, side2);
+    using Smem = ExactSmem<P>;
+    constexpr int kBodies = Smem::kBodies;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+    fill_side2(p.bbox, sm.side2);
     __syncthreads();
-    if (threadIdx.x <= kMaxDepth) side2f[threadIdx.x] = (float)side2[threadIdx.x];
+    if (threadIdx.x <= kMaxDepth) sm.side2f[threadIdx.x] = (float)sm.side2[threadIdx.x];
     __syncthreads();
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t group = (int64_t)blockIdx.x * kTravWarps + w;
-    const int64_t base = group * 32;
+    const int64_t base = group * kBodies;
     if (base >= p.n) return;  // whole warp past the end
-    const int64_t i = base + lane;
+    const int body = lane / P, phase = lane % P;
+    const int64_t i = base + body;
     const bool valid = i < p.n;
     const int64_t ii = valid ? i : base;
     const double px = p.px[ii], py = p.py[ii], pz = p.pz[ii];
     const int my_leaf = valid ? p.body_leaf[i] : -2;
-    const double theta2 = p.theta2, G = p.G, soft2 = p.soft2;
-    const float theta2f = (float)theta2;
+    const double theta2 = p.theta2, soft2 = p.soft2;
+    const float theta2f = (float)theta2, soft2f = (float)soft2;
     // Group box in group-relative FP32 coordinates (for the group tests).
     const float gx = __double2float_rn(__shfl_sync(0xffffffffu, px, 0));
     const float gy = __double2float_rn(__shfl_sync(0xffffffffu, py, 0));
@@ -124,6 +195,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
     const float ry = __double2float_rn(py - (double)gy);
     const float rz = __double2float_rn(pz - (double)gz);
     float bminx = rx, bminy = ry, bminz = rz, bmaxx = rx, bmaxy = ry, bmaxz = rz;
+    int leaf_lo = valid ? my_leaf : INT_MAX, leaf_hi = valid ? my_leaf : INT_MIN;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         bminx = fminf(bminx, __shfl_xor_sync(0xffffffffu, bminx, off));
@@ -132,145 +204,255 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
         bmaxx = fmaxf(bmaxx, __shfl_xor_sync(0xffffffffu, bmaxx, off));
         bmaxy = fmaxf(bmaxy, __shfl_xor_sync(0xffffffffu, bmaxy, off));
         bmaxz = fmaxf(bmaxz, __shfl_xor_sync(0xffffffffu, bmaxz, off));
+        leaf_lo = min(leaf_lo, __shfl_xor_sync(0xffffffffu, leaf_lo, off));
+        leaf_hi = max(leaf_hi, __shfl_xor_sync(0xffffffffu, leaf_hi, off));
     }
     const float bmag = fmaxf(fmaxf(fmaxf(fabsf(bminx), fabsf(bmaxx)), fmaxf(fabsf(bminy), fabsf(bmaxy))),
-                             fmaxf(fabsf(bminz), fabsf(bmaxz)));
-    int* stk = stack[w];
-    int (*PL)[32] = plist[w];
+                             fmaxf(fabsf(bminz), fabsf(bmaxz))) +
+                       (5e-14f / kAbsErr) * fmaxf(fmaxf(fabsf(gx), fabsf(gy)), fabsf(gz));
+    int2* stk = sm.stack[w];
+    int (*PL)[kBodies] = sm.plist[w];
+    const unsigned lt = (1u << lane) - 1u;
 
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    unsigned cnt = 0;
-    int mine = 0;  // entries in this lane's list
+    // Lane l < 3 kBodies sums the component l / kBodies of body l % kBodies.
+    double sum = 0.0;
+    // This body's list: entries done .. cnt - 1, in slots modulo kCap.
+    int cnt = 0, done = 0;
     int sp = 1;
-    int skip_sp = 0x7fffffff;
-    if (lane == 0) stk[0] = 0;
+    const unsigned full = __ballot_sync(0xffffffffu, valid) & Smem::kFirst;
+    const double one = __shfl_sync(0xffffffffu, p.one, 0);
+    if (lane == 0) stk[0] = make_int2(0, (int)full);
     __syncwarp();
     bool overflow = false;
-    int64_t pops = 0;
+    int64_t passes = 0;
 
-    // Evaluates every lane's list in order with the reference's arithmetic.
-    auto flush = [&]() {
-        int most = mine;
+    // Evaluates the bodies' lists in order until none holds more than `left`
+    // entries.  P lanes evaluate P consecutive terms of a body; the sums run
+    // over them one after the other.
+    auto flush = [&](int left) {
+        int most = cnt - done;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
-        for (int q = 0; q < most; ++q) {
-            const bool on = q < mine;
-            const int s = on ? PL[q][lane] : 0;
-            const TreeRec r = load_rec(p.rec, s);
-            const double dx = __dsub_rn(r.cx, px), dy = __dsub_rn(r.cy, py), dz = __dsub_rn(r.cz, pz);
-            const double r2 =
-                __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
-            const double invR = __drcp_rn(__dsqrt_rn(r2));
-            const double invR3 = __dmul_rn(__dmul_rn(invR, invR), invR);
-            const double sc = __dmul_rn(__dmul_rn(G, r.m), invR3);
-            if (on) {
-                ax = __dadd_rn(ax, __dmul_rn(sc, dx));
-                ay = __dadd_rn(ay, __dmul_rn(sc, dy));
-                az = __dadd_rn(az, __dmul_rn(sc, dz));
+        const int sum_body = lane % kBodies;
+        for (; most > left; most -= P) {
+            const int q = done + phase;
+            const bool on = q < cnt;
+            const double4_32a r = p.d4[on ? PL[q & (Smem::kCap - 1)][body] : 0];
+            double tx, ty, tz;
+            exact_term<kSoft>(r, px, py, pz, soft2, on, one, tx, ty, tz);
+            auto T = sm.term[w];
+            T[0][lane] = tx;
+            T[1][lane] = ty;
+            T[2][lane] = tz;
+            const int terms = __shfl_sync(0xffffffffu, cnt - done, sum_body * P);
+            if (lane < 3 * kBodies) {
+                const double* t = &T[lane / kBodies][sum_body * P];
+#pragma unroll
+                for (int k = 0; k < P; ++k)
+                    if (k < terms) sum = fma(sum, one, t[k]);
             }
+            __syncwarp();
+            done = min(done + P, cnt);
         }
-        mine = 0;
         __syncwarp();
     };
 
     while (sp > 0) {
-        if (++pops > p.max_pops) {
+        if (++passes > p.max_pops) {
             overflow = true;
             break;
         }
-        --sp;
-        const int s = stk[sp];
-        __syncwarp();
-        const float4 a = __ldg(p.A + s);
-        const float4 b = __ldg(p.B + s);
-        const uint32_t mt = __ldg(p.meta + s);
-        if (sp < skip_sp) skip_sp = 0x7fffffff;
-        if ((mt >> 17) & 1u) continue;  // massless: skipped with its subtree (traversal.cpp:66)
-        const bool active = valid && skip_sp == 0x7fffffff;
-        const bool leaf = (mt >> 16) & 1u;
-        const int depth = (mt >> 8) & 0xFF;
-        bool accept = false, open = false;
-        if (leaf) {
-            if (active) {
-                if (__float_as_int(b.w) != my_leaf) {
-                    accept = true;
+        // The window: the top items of the stack, lane 0 the first in walk
+        // order.
+        const int m = sp < 32 ? sp : 32;
+        int node = 0, nc = 0, ref = 0, depth = 0;
+        unsigned M = 0, A = 0;
+        bool test = false, leaf = false, mixed = false;
+        float cx = 0.f, cy = 0.f, cz = 0.f, nerr = 0.f;  // group-relative centre, its allowance
+        if (lane < m) {
+            const int2 it = stk[sp - 1 - lane];
+            node = it.x & ~kDecided;
+            M = (unsigned)it.y;
+            if (it.x & kDecided) {
+                A = M;
+            } else {
+                test = true;
+                const float4 a = __ldg(p.A + node);
+                const float4 b = __ldg(p.B + node);
+                const uint32_t mt = __ldg(p.meta + node);
+                cx = (a.x - gx) + b.x;
+                cy = (a.y - gy) + b.y;
+                cz = (a.z - gz) + b.z;
+                ref = __float_as_int(b.w);
+                leaf = (mt >> 16) & 1u;
+                depth = (mt >> 8) & 0xFF;
+                nerr = kAbsErr * (fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + bmag);
+                if ((mt >> 17) & 1u) {
+                    M = 0;  // massless: skipped with its subtree (traversal.cpp:66)
+                } else if (leaf) {
+                    A = M;
                 } else {
-                    // Own leaf: the reference skips it at depth 21, but a chain
-                    // cell above it (depths top..20) may already accept.
-                    const TreeRec r = load_rec(p.rec, s);
-                    const double dx = __dsub_rn(r.cx, px), dy = __dsub_rn(r.cy, py), dz = __dsub_rn(r.cz, pz);
-                    const double r2 = __dadd_rn(
-                        __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
-                    accept = r.top <= kMaxDepth - 1 && side2[kMaxDepth - 1] < __dmul_rn(theta2, r2);
-                }
-            }
-        } else {
-            // The same node for every lane: classify it against the group box
-            // (with allowances for FP32 rounding), test lane by lane in FP64
-            // only when the box cannot decide.
-            const float cx = (a.x - gx) + b.x, cy = (a.y - gy) + b.y, cz = (a.z - gz) + b.z;
-            const float ex = fmaxf(0.0f, fmaxf(bminx - cx, cx - bmaxx));
-            const float ey = fmaxf(0.0f, fmaxf(bminy - cy, cy - bmaxy));
-            const float ez = fmaxf(0.0f, fmaxf(bminz - cz, cz - bmaxz));
-            const float fx = fmaxf(fabsf(cx - bminx), fabsf(cx - bmaxx));
-            const float fy = fmaxf(fabsf(cy - bminy), fabsf(cy - bmaxy));
-            const float fz = fmaxf(fabsf(cz - bminz), fabsf(cz - bmaxz));
-            const float err = kAbsErr * (fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + bmag);
-            const float dlo = fmaxf(sqrtf(ex * ex + ey * ey + ez * ez) - err, 0.0f);
-            const float dhi = sqrtf(fx * fx + fy * fy + fz * fz) + err;
-            const float s2 = side2f[depth];
-            if (s2 * (1.0f + kMargin) < theta2f * dlo * dlo) {
-                accept = active;
-            } else if (s2 * (1.0f - kMargin) > theta2f * dhi * dhi) {
-                open = active;
-            } else if (__any_sync(0xffffffffu, active)) {
-                const TreeRec r = load_rec(p.rec, s);
-                if (active) {
-                    const double dx = __dsub_rn(r.cx, px), dy = __dsub_rn(r.cy, py), dz = __dsub_rn(r.cz, pz);
-                    const double r2 = __dadd_rn(
-                        __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
-                    accept = side2[depth] < __dmul_rn(theta2, r2);
-                    open = !accept;
+                    nc = (int)(mt & 0xFF);
+                    const float ex = fmaxf(0.0f, fmaxf(bminx - cx, cx - bmaxx));
+                    const float ey = fmaxf(0.0f, fmaxf(bminy - cy, cy - bmaxy));
+                    const float ez = fmaxf(0.0f, fmaxf(bminz - cz, cz - bmaxz));
+                    const float fx = fmaxf(fabsf(cx - bminx), fabsf(cx - bmaxx));
+                    const float fy = fmaxf(fabsf(cy - bminy), fabsf(cy - bmaxy));
+                    const float fz = fmaxf(fabsf(cz - bminz), fabsf(cz - bmaxz));
+                    const float dlo = fmaxf(sqrtf(ex * ex + ey * ey + ez * ez) - nerr, 0.0f);
+                    const float dhi = sqrtf(fx * fx + fy * fy + fz * fz) + nerr;
+                    const float s2 = sm.side2f[depth];
+                    if (sure_below(s2, theta2f, dlo * dlo + soft2f)) A = M;
+                    else mixed = !sure_above(s2, theta2f, dhi * dhi + soft2f);
                 }
             }
         }
-        if (accept) {
-            PL[mine++][lane] = s;
-            ++cnt;
-        }
-        const unsigned opened = __ballot_sync(0xffffffffu, open);
-        if (opened) {
-            if (accept) skip_sp = sp;  // sit out this node's subtree
-            const int nc = (int)(mt & 0xFF);
-            if (sp + nc > kStackCap) {
-                overflow = true;
-                break;
+        // Nodes the box cannot decide, and the leaves that may hold one of
+        // the bodies: each body tests them itself, P at a time, in FP32 with
+        // the same allowance and in FP64 with the reference's rounding where
+        // that cannot decide either.  A body skips its own leaf at depth 21,
+        // but a chain cell above it (depths top..20) may already accept it;
+        // any other leaf it accepts.
+        const bool own = test && leaf && A != 0 && ref >= leaf_lo && ref <= leaf_hi;
+        const unsigned ub = __ballot_sync(0xffffffffu, mixed || own);
+        if (ub) {
+            const int k = __popc(ub & lt);
+            if (mixed || own) {
+                sm.und[w][k] = make_float4(cx, cy, cz, nerr);
+                sm.und2[w][k] = make_int4(own ? kMaxDepth - 1 : depth, node, own ? ref : -1, 0);
             }
-            if (lane < nc) stk[sp + lane] = __float_as_int(b.w) + lane;
             __syncwarp();
-            sp += nc;
+            const int nu = __popc(ub);
+            for (int k0 = 0; k0 < nu; k0 += P) {
+                bool acc = false;
+                const int kk = k0 + phase;
+                if (kk < nu) {
+                    const float4 u = sm.und[w][kk];
+                    const int4 v = sm.und2[w][kk];
+                    const float dxf = u.x - rx, dyf = u.y - ry, dzf = u.z - rz;
+                    const float df = sqrtf(dxf * dxf + dyf * dyf + dzf * dzf);
+                    const float lo = fmaxf(df - u.w, 0.0f), hi = df + u.w;
+                    const float s2 = sm.side2f[v.x];
+                    if (v.z >= 0 ? v.z != my_leaf : sure_below(s2, theta2f, lo * lo + soft2f)) {
+                        acc = true;
+                    } else if (!sure_above(s2, theta2f, hi * hi + soft2f)) {
+                        const TreeRec r = p.rec[v.y];
+                        const double dx = __dsub_rn(r.cx, px), dy = __dsub_rn(r.cy, py), dz = __dsub_rn(r.cz, pz);
+                        const double r2 = __dadd_rn(
+                            __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
+                        acc = (v.z < 0 || r.top <= kMaxDepth - 1) && sm.side2[v.x] < __dmul_rn(theta2, r2);
+                    }
+                }
+                const unsigned res = __ballot_sync(0xffffffffu, acc);
+                if ((mixed || own) && k >= k0 && k < k0 + P) A = (res >> (k - k0)) & Smem::kFirst & M;
+            }
+            __syncwarp();
         }
-        if (__any_sync(0xffffffffu, mine == kPList)) flush();
+        // Opened nodes leave their children in their place.  Where they would
+        // not fit, the later ones wait (an untested item again).
+        const unsigned O = leaf ? 0u : M & ~A;
+        bool open = test && O != 0;
+        const unsigned opened = __ballot_sync(0xffffffffu, open);
+        const int first = opened ? __ffs(opened) - 1 : 32;
+        int out = (A != 0 ? 1 : 0) + (open ? nc : 0);
+        int incl = out;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += t;
+        }
+        const int below = sp - m;
+        if (__any_sync(0xffffffffu, open && lane > first && below + incl + (m - 1 - lane) > kSoftStk)) {
+            if (open && lane > first && below + incl + (m - 1 - lane) > kSoftStk) {
+                open = false;
+                A = M;
+                nc = -1;  // not decided: the item goes back as it was
+                out = 1;
+            }
+            incl = out;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) incl += t;
+            }
+        }
+        // Accepted items before the first opened node, and its own accepted
+        // part, are next in walk order: they go to the lists.  All else goes
+        // back on the stack.
+        const bool emit = A != 0 && lane <= first;
+        if (emit) --out;
+        const unsigned em = __ballot_sync(0xffffffffu, emit);
+        const int total = __shfl_sync(0xffffffffu, incl, 31) - __popc(em);
+        const int pos = incl - __popc(em & (lt | (1u << lane))) - out;  // outputs put back before this lane's
+        if (below + total > kStk) {
+            overflow = true;
+            break;
+        }
+        __syncwarp();
+        int top = below + total - 1 - pos;
+        if (A != 0 && !emit) stk[top--] = make_int2(nc < 0 ? node : node | kDecided, (int)A);
+        if (open)
+            for (int c = nc - 1; c >= 0; --c) stk[top--] = make_int2(ref + c, (int)O);
+        sp = below + total;
+        if (em) {
+            if (__any_sync(0xffffffffu, cnt - done > Smem::kCap - 33)) {
+                __syncwarp();
+                flush(Smem::kCap / 4);
+            }
+            // Body by body: the lanes whose item it takes append it.
+#pragma unroll
+            for (int b = 0; b < kBodies; ++b) {
+                const bool take = emit && ((A >> (b * P)) & 1u);
+                const unsigned tb = __ballot_sync(0xffffffffu, take);
+                const int at = __shfl_sync(0xffffffffu, cnt, b * P);
+                if (take) PL[(at + __popc(tb & lt)) & (Smem::kCap - 1)][b] = node;
+                if (body == b) cnt += __popc(tb);
+            }
+        }
+        __syncwarp();
     }
-    flush();
+    flush(0);
     if (overflow && lane == 0) atomicOr(p.err, kErrOverflow);
-    if (valid) {
-        p.ax[i] = ax;
-        p.ay[i] = ay;
-        p.az[i] = az;
-        if (p.body_count) p.body_count[i] = (int32_t)cnt;
-        if (p.kick_h > 0.0) {
-            p.vx[i] = __dadd_rn(p.vx[i], __dmul_rn(p.kick_h, ax));
-            p.vy[i] = __dadd_rn(p.vy[i], __dmul_rn(p.kick_h, ay));
-            p.vz[i] = __dadd_rn(p.vz[i], __dmul_rn(p.kick_h, az));
+    if (lane < 3 * kBodies) {
+        const int c = lane / kBodies;
+        const int64_t k = base + lane % kBodies;
+        if (k < p.n) {
+            double* a = c == 0 ? p.ax : c == 1 ? p.ay : p.az;
+            double* v = c == 0 ? p.vx : c == 1 ? p.vy : p.vz;
+            a[k] = sum;
+            if (p.kick_h > 0.0) v[k] = __dadd_rn(v[k], __dmul_rn(p.kick_h, sum));
         }
     }
+    const bool counts = valid && phase == 0;
+    if (counts && p.body_count) p.body_count[i] = cnt;
     if (p.inter_count) {
-        unsigned long long c = valid ? cnt : 0ull;
+        unsigned long long c = counts ? (unsigned long long)cnt : 0ull;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) c += __shfl_down_sync(0xffffffffu, c, off);
         if (lane == 0) atomicAdd(p.inter_count, c);
     }
+}
+
+template <int P, bool kSoft>
+int launch_exact(bh_context* ctx, const TravParams& p)
+{
+    auto kernel = traverse_exact_kernel<P, kSoft>;
+    const size_t smem = sizeof(ExactSmem<P>);
+    BH_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BH_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared));
+    const int64_t groups = (p.n + 32 / P - 1) / (32 / P);
+    const int64_t blocks = (groups + kTravWarps - 1) / kTravWarps;
+    kernel<<<(unsigned)blocks, kTravThreads, smem, ctx->stream>>>(p);
+    BH_LAUNCH_CHECK(ctx);
+    return BH_OK;
+}
+
+// soft2 = 0 leaves r^2 as it is (r^2 + 0 = r^2): one FP64 addition less.
+template <int P>
+int launch_exact_p(bh_context* ctx, const TravParams& p)
+{
+    return p.soft2 == 0.0 ? launch_exact<P, false>(ctx, p) : launch_exact<P, true>(ctx, p);
 }
 
 }  // namespace
@@ -284,12 +466,14 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
     p.px = ctx->px; p.py = ctx->py; p.pz = ctx->pz;
     p.body_leaf = ctx->body_leaf;
     p.rec = ctx->rec;
+    p.d4 = ctx->d4;
     p.A = ctx->fA; p.B = ctx->fB; p.meta = ctx->fmeta;
     p.bbox = ctx->bbox;
     p.theta2 = theta * theta;
     p.G = G;
     p.soft2 = soft2;
     p.kick_h = kick_h;
+    p.one = 1.0;
     p.max_pops = 2 * n + 2;
     p.ax = ctx->ax; p.ay = ctx->ay; p.az = ctx->az;
     p.vx = ctx->vx; p.vy = ctx->vy; p.vz = ctx->vz;
@@ -297,14 +481,21 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
     p.body_count = ctx->body_count;
     p.err = ctx->err;
     BH_CUDA_TRY(cudaMemsetAsync(ctx->inter_count, 0, sizeof(unsigned long long), ctx->stream));
-    const int64_t groups = (n + 31) / 32;
-    const int64_t blocks = (groups + kTravWarps - 1) / kTravWarps;
     switch (mode) {
     case BH_MODE_PLAIN_FP64: {
-        const int rc = launch_fp32_nodes(ctx, G);
+        const int rc = launch_fp32_nodes(ctx, G, true);
         if (rc) return rc;
-        traverse_exact_kernel<<<(unsigned)blocks, kTravThreads, 0, ctx->stream>>>(p);
-        break;
+        // Lanes to a body: 4 (the evaluation's sums fill 24 lanes and the
+        // bodies share a walk) while that gives the chip 12 warps per SM, and
+        // more below, where a warp's own latency counts: forces in ms with
+        // 4 / 8 / 16 / 32 lanes: 300,149 bodies 2.96 / 3.67 / 5.36 / -,
+        // 19,054 1.21 / 1.26 / 1.39 / -, 8,000 0.69 / 0.46 / - / -,
+        // 4,000 0.44 / 0.29 / 0.23 / 0.25, 1,000 0.20 / 0.13 / 0.095 / 0.070.
+        const int64_t want = 12 * (int64_t)num_sms() * 32;
+        if (n * 4 >= want) return launch_exact_p<4>(ctx, p);
+        if (n * 8 >= want) return launch_exact_p<8>(ctx, p);
+        if (n * 16 >= want) return launch_exact_p<16>(ctx, p);
+        return launch_exact_p<32>(ctx, p);
     }
     case BH_MODE_FP64_LIST:
         return launch_traverse_masked(ctx, theta, G, soft2, kick_h, true);
@@ -317,8 +508,6 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
     default:
         return bh_fail(BH_ERR_INVALID_ARGUMENT, "bh_compute_accelerations: mode not available");
     }
-    BH_LAUNCH_CHECK(ctx);
-    return BH_OK;
 }
 
 }  // namespace bh

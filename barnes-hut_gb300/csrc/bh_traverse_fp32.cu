@@ -731,11 +731,11 @@ int launch_walk(bh_context* ctx, const FParams& p)
 
 }  // namespace
 
-int launch_fp32_nodes(bh_context* ctx, double G)
+int launch_fp32_nodes(bh_context* ctx, double G, bool fp64)
 {
     if (ctx->n == 0) return BH_OK;
     fp32_nodes_kernel<<<grid_n(2 * ctx->n), 256, 0, ctx->stream>>>(ctx->counts, ctx->rec, G, ctx->fA, ctx->fB,
-                                                                    ctx->fmeta, nullptr);
+                                                                    ctx->fmeta, fp64 ? ctx->d4 : nullptr);
     BH_LAUNCH_CHECK(ctx);
     ctx->fnodes_fused = true;
     ctx->fnodes_G = G;
