@@ -481,24 +481,30 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
     p.body_count = ctx->body_count;
     p.err = ctx->err;
     BH_CUDA_TRY(cudaMemsetAsync(ctx->inter_count, 0, sizeof(unsigned long long), ctx->stream));
+    // Lanes to a body in the exact walk: 4 (the evaluation's sums fill 24 lanes
+    // and the bodies share a walk) while that gives the chip 12 warps per SM,
+    // and more below, where a warp's own latency counts.  Forces in ms with
+    // 4 / 8 / 16 / 32 lanes: 300,149 bodies 2.96 / 3.67 / 5.36 / -, 19,054
+    // 1.21 / 1.26 / 1.39 / -, 8,000 0.69 / 0.46 / - / -, 4,000 0.44 / 0.29 /
+    // 0.23 / 0.25, 1,000 0.20 / 0.13 / 0.095 / 0.070.
+    const int64_t want = 12 * (int64_t)num_sms() * 32;
+    const int lanes = n * 4 >= want ? 4 : n * 8 >= want ? 8 : n * 16 >= want ? 16 : 32;
+    // The FP64 list form meets its bounds with the exact walk's result, which
+    // small systems get sooner: 4,000 bodies 0.23 against 0.27 ms, 1,000 0.07
+    // against 0.12; 8,000 take the same time, 19,054 1.21 against 0.92.
+    if (mode == BH_MODE_FP64_LIST && lanes < 16) return launch_traverse_masked(ctx, theta, G, soft2, kick_h, true);
     switch (mode) {
-    case BH_MODE_PLAIN_FP64: {
+    case BH_MODE_PLAIN_FP64:
+    case BH_MODE_FP64_LIST: {
         const int rc = launch_fp32_nodes(ctx, G, true);
         if (rc) return rc;
-        // Lanes to a body: 4 (the evaluation's sums fill 24 lanes and the
-        // bodies share a walk) while that gives the chip 12 warps per SM, and
-        // more below, where a warp's own latency counts: forces in ms with
-        // 4 / 8 / 16 / 32 lanes: 300,149 bodies 2.96 / 3.67 / 5.36 / -,
-        // 19,054 1.21 / 1.26 / 1.39 / -, 8,000 0.69 / 0.46 / - / -,
-        // 4,000 0.44 / 0.29 / 0.23 / 0.25, 1,000 0.20 / 0.13 / 0.095 / 0.070.
-        const int64_t want = 12 * (int64_t)num_sms() * 32;
-        if (n * 4 >= want) return launch_exact_p<4>(ctx, p);
-        if (n * 8 >= want) return launch_exact_p<8>(ctx, p);
-        if (n * 16 >= want) return launch_exact_p<16>(ctx, p);
-        return launch_exact_p<32>(ctx, p);
+        switch (lanes) {
+        case 4: return launch_exact_p<4>(ctx, p);
+        case 8: return launch_exact_p<8>(ctx, p);
+        case 16: return launch_exact_p<16>(ctx, p);
+        default: return launch_exact_p<32>(ctx, p);
+        }
     }
-    case BH_MODE_FP64_LIST:
-        return launch_traverse_masked(ctx, theta, G, soft2, kick_h, true);
     case BH_MODE_FP32_FAR:
         return launch_traverse_masked(ctx, theta, G, soft2, kick_h, false);
     case BH_MODE_LEARNED:

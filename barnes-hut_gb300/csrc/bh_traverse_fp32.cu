@@ -20,8 +20,13 @@
 // walk at theta accepts.
 //
 // BH_MODE_FP64_LIST: per-lane tests in FP64 with the reference's rounding,
-//   interactions in FP64 (rcube_hh + FMA) from the FP64 node records, on the
-//   reference's tree.
+//   interactions in FP64 from the FP64 node records, on the reference's tree.
+//   The FP64 pipe bounds the evaluation (16 to 19 cycles of the SM per warp
+//   instruction), so r^2, r^-3 and the factor G m r^-3 are formed from the
+//   displacement's bits on the integer pipes, to within an ulp
+//   (soft::scale); six FP64 instructions per 32 pairs are left of 13 (the
+//   differences and the accumulating FMAs).  300,149 bodies, theta 1.05:
+//   3.27 -> 1.90 ms of forces.
 // BH_MODE_FP32_FAR: precision form.  The bodies with id < num_direct (Sun and
 //   planets) are taken out of the tree (masses zeroed before the build) and
 //   summed directly in FP64.  Far-field interactions run in FP32 on
@@ -36,6 +41,7 @@
 //   recording every candidate's group, slot, lane mask and raw features.
 #include <climits>
 
+#include "bh_soft64.cuh"
 #include "bh_walk.cuh"
 
 namespace bh {
@@ -84,6 +90,24 @@ __global__ void direct_extract_kernel(int64_t n, const double* __restrict__ px, 
 
 namespace {
 
+// G m r^-3 on the FP64 pipe, for the pairs soft::scale leaves out.  A call of
+// its own: inlined, it becomes predicated instructions that take the FP64 pipe
+// although no lane needs them.
+__device__ __noinline__ double fp64_scale(double dx, double dy, double dz, double soft2, double gm)
+{
+    return gm * rcube_hh(fma(dx, dx, fma(dy, dy, fma(dz, dz, soft2))));
+}
+
+// Whether a cell of depth 20 accepts, with the reference's rounding
+// (traversal.cpp:78); a call for the same reason.
+__device__ __noinline__ bool own_chain_accepts(double dx, double dy, double dz, double soft2, double theta2,
+                                               double side2)
+{
+    const double r2 =
+        __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
+    return side2 < __dmul_rn(theta2, r2);
+}
+
 template <bool kFP64, int kLearn, bool kGroup = false>
 __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
 {
@@ -117,10 +141,10 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t group = (int64_t)blockIdx.x * kWarps + w;
-    const int64_t base = group * 32;
+    const int64_t base = group * p.bodies;
     if (base >= p.n) return;
     const int64_t i = base + lane;
-    const bool valid = i < p.n;
+    const bool valid = lane < p.bodies && i < p.n;
     const int64_t ii = valid ? i : base;  // idle lanes shadow the group's first body
     const double x = p.px[ii], y = p.py[ii], z = p.pz[ii];
     // The group centre g: the first body's position truncated to FP32 on the
@@ -563,24 +587,21 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
                     bool take = on;
                     if (on && LL[j] == sm.bleaf[w][b]) {
                         // Own leaf: skipped at depth 21 unless a chain cell above
-                        // it (depths top..20) accepts (traversal.cpp:70,78).  At
-                        // zero displacement and no softening r^2 is 0 and no
-                        // cell accepts (decided on the bit patterns).
-                        if (nosoft && ((__double_as_longlong(dx) | __double_as_longlong(dy) |
-                                        __double_as_longlong(dz)) << 1) == 0) {
-                            take = false;
-                        } else {
-                            const double r2e = __dadd_rn(
-                                __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
+                        // it (depths top..20) accepts (traversal.cpp:70,78): in
+                        // FP32 where that can tell it does not (the margins hold
+                        // for any side^2 above 1e-30; at zero displacement and no
+                        // softening r^2 is 0 and no cell accepts), else in FP64.
+                        const float fx = narrow_trunc(dx), fy = narrow_trunc(dy), fz = narrow_trunc(dz);
+                        const float r2f = fmaf(fx, fx, fmaf(fy, fy, fmaf(fz, fz, (float)soft2)));
+                        const float s20 = sm.side2f[kMaxDepth - 1];
+                        take = false;
+                        if (!(s20 * (1.0f - kMargin) > theta2f * r2f && s20 > 1e-30f))
                             take = p.rec[LN[j]].top <= kMaxDepth - 1 &&
-                                   sm.side2d[kMaxDepth - 1] < __dmul_rn(theta2, r2e);
-                        }
+                                   own_chain_accepts(dx, dy, dz, soft2, theta2, sm.side2d[kMaxDepth - 1]);
                     }
-                    const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, soft2)));
-                    // A pair not taken (an own leaf at r2 = 0, or a lane past
-                    // its share) gets an argument on the fast path, so that no
-                    // lane diverges into the out-of-range branch for it.
-                    double sc = r.w * rcube_hh(take ? r2 : 1.0);
+                    double sc;
+                    if (!(soft::scale(dx, dy, dz, r.w, sc) && nosoft) && take)
+                        sc = fp64_scale(dx, dy, dz, soft2, r.w);
                     if (!take) sc = 0.0;
                     sx = fma(sc, dx, sx);
                     sy = fma(sc, dy, sy);
@@ -722,7 +743,7 @@ int launch_walk(bh_context* ctx, const FParams& p)
         BH_CUDA_TRY(cudaFuncSetAttribute(traverse_masked_kernel<kFP64, kLearn, kGroup>,
                                          cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared));
-    const int64_t groups = (p.n + 31) / 32;
+    const int64_t groups = (p.n + p.bodies - 1) / p.bodies;
     const int64_t blocks = (groups + kWarps - 1) / kWarps;
     traverse_masked_kernel<kFP64, kLearn, kGroup><<<(unsigned)blocks, kThreads, smem, ctx->stream>>>(p);
     BH_LAUNCH_CHECK(ctx);
@@ -771,6 +792,7 @@ int prepare_walk(bh_context* ctx, double theta, double G, double soft2, bool fp6
     }
     p = FParams{};
     p.n = n;
+    p.bodies = 32;
     p.px = ctx->px; p.py = ctx->py; p.pz = ctx->pz;
     p.id = ctx->id;
     p.body_leaf = ctx->body_leaf;
@@ -805,7 +827,15 @@ int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2
     int rc = prepare_walk(ctx, theta, G, soft2, fp64, p);
     if (rc) return rc;
     p.kick_h = kick_h;
-    if (fp64) return launch_walk<true, kLearnNone>(ctx, p);
+    if (fp64) {
+        // Bodies per warp: 32 while that gives the chip 12 warps per SM, and
+        // fewer below (the evaluation is balanced over the 32 threads however
+        // many bodies share it).  Forces in ms with 32 / 16 / 8 / 4 bodies:
+        // 65,537 bodies 0.54 / 0.55 / 0.52 / 0.62, 19,054 1.83 / 1.27 / 0.92 /
+        // 1.08, 8,000 1.29 / 0.80 / 0.59 / 0.46.
+        while (p.bodies > 4 && ctx->n < 12 * (int64_t)num_sms() * p.bodies) p.bodies >>= 1;
+        return launch_walk<true, kLearnNone>(ctx, p);
+    }
     return group ? launch_walk<false, kLearnNone, true>(ctx, p) : launch_walk<false, kLearnNone>(ctx, p);
 }
 

@@ -109,6 +109,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
 
 struct FParams {
     int64_t n;
+    int bodies;  // per warp group: a power of two up to 32
     const double* px;
     const double* py;
     const double* pz;

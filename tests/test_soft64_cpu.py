@@ -89,6 +89,27 @@ int main()
             if (w == 0 ? t[k] != 0 : bits_of((double)w) != bits_of(t[k])) ++bad;
         }
     }
+    // The list form's factor: within an ulp of the value in long double.
+    long in = 0;
+    for (long i = 0; i < 4000000; ++i) {
+        double d[3], got;
+        const int e = (int)(rnd() % 160) - 80;
+        for (double& v : d) {
+            v = value(e - (int)(rnd() % 20));
+            if (rnd() & 1) v = -v;
+            if ((rnd() & 31) == 0) v = 0.0;
+            if ((rnd() & 31) == 0) v = value(e - 60 - (int)(rnd() % 60));
+        }
+        const double gm = value((int)(rnd() % 200) - 150);
+        if (!scale(d[0], d[1], d[2], gm, got)) continue;
+        ++in;
+        const long double r2 = (long double)d[0] * d[0] + (long double)d[1] * d[1] + (long double)d[2] * d[2];
+        const long double want = gm / (r2 * sqrtl(r2));
+        // 0.53 ulp, and what the long double itself is off by where it has no
+        // more than 53 bits (Arm's has 113, x86's 64)
+        if (!(fabsl((long double)got - want) <= 0.55L * 0x1p-52L * want)) ++bad;
+    }
+    if (in < 1000000) ++bad;
     // Out of range: refused, not wrong.
     double t[3];
     const double out[][5] = {{1, 1, 1, 0x1p-250, 1}, {1, 1, 1, 0x1p+250, 1}, {1, 1, 1, 0.0, 1}, {1, 1, 1, 3, 0.0},
@@ -96,6 +117,10 @@ int main()
                              {1, 1, 1, HUGE_VAL, 1}, {1, 1, 1, 3, HUGE_VAL}, {1, 1, 1, NAN, 1}, {1, 1, 1, -1.0, 1}};
     for (auto& o : out)
         if (term(o[0], o[1], o[2], o[3], o[4], t[0], t[1], t[2])) ++bad;
+    const double far[][4] = {{0, 0, 0, 1}, {0x1p-120, 0, 0, 1}, {0x1p+120, 1, 1, 1}, {1, HUGE_VAL, 0, 1},
+                             {1, 1, NAN, 1}, {1, 1, 1, 0.0}, {1, 1, 1, -1.0}, {1, 1, 1, 0x1p-320}};
+    for (auto& o : far)
+        if (scale(o[0], o[1], o[2], o[3], t[0])) ++bad;
     std::printf("%ld %ld %ld\n", bad, odd, taken);
     return bad != 0;
 }
