@@ -489,13 +489,8 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
     // 0.23 / 0.25, 1,000 0.20 / 0.13 / 0.095 / 0.070.
     const int64_t want = 12 * (int64_t)num_sms() * 32;
     const int lanes = n * 4 >= want ? 4 : n * 8 >= want ? 8 : n * 16 >= want ? 16 : 32;
-    // The FP64 list form meets its bounds with the exact walk's result, which
-    // small systems get sooner: 4,000 bodies 0.23 against 0.27 ms, 1,000 0.07
-    // against 0.12; 8,000 take the same time, 19,054 1.21 against 0.92.
-    if (mode == BH_MODE_FP64_LIST && lanes < 16) return launch_traverse_masked(ctx, theta, G, soft2, kick_h, true);
     switch (mode) {
-    case BH_MODE_PLAIN_FP64:
-    case BH_MODE_FP64_LIST: {
+    case BH_MODE_PLAIN_FP64: {
         const int rc = launch_fp32_nodes(ctx, G, true);
         if (rc) return rc;
         switch (lanes) {
@@ -505,6 +500,8 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
         default: return launch_exact_p<32>(ctx, p);
         }
     }
+    case BH_MODE_FP64_LIST:
+        return launch_traverse_masked(ctx, theta, G, soft2, kick_h, true);
     case BH_MODE_FP32_FAR:
         return launch_traverse_masked(ctx, theta, G, soft2, kick_h, false);
     case BH_MODE_LEARNED:

@@ -108,13 +108,22 @@ __device__ __noinline__ bool own_chain_accepts(double dx, double dy, double dz, 
     return side2 < __dmul_rn(theta2, r2);
 }
 
-template <bool kFP64, int kLearn, bool kGroup = false>
-__global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
+// kTeam > 1: a block of kTeam warps walks one group, for systems with too few
+// groups to fill the chip.  The warps take ranges from one stack in rounds
+// (kTeamPop each from its top, eight lanes to a range), push the opened nodes'
+// ranges behind one another's, and evaluate the entries each of them staged
+// for all 32 bodies; the bodies' sums over the warps are added in warp order.
+// Every body meets the nodes it meets with one warp, and the result does not
+// depend on timing.
+template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1>
+__global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_masked_kernel(FParams p)
 {
+    static_assert(kTeam == 1 || kLearn == kLearnNone, "collection records one warp per group");
+    using Smem = WalkSmem<kFP64, kLearn, kGroup, kTeam>;
     static_assert(kLearn != kLearnInfer, "the learned walk is traverse_learned_kernel");
     static_assert(!kGroup || (!kFP64 && kLearn == kLearnNone), "the group test is an FP32 far-field walk");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    WalkSmem<kFP64, kLearn, kGroup>& sm = *reinterpret_cast<WalkSmem<kFP64, kLearn, kGroup>*>(smem_raw);
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     if (threadIdx.x <= kMaxDepth) {
         const double dx = __dsub_rn(p.bbox[3], p.bbox[0]);
         const double dy = __dsub_rn(p.bbox[4], p.bbox[1]);
@@ -140,11 +149,11 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
     __syncthreads();
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t group = (int64_t)blockIdx.x * kWarps + w;
-    const int64_t base = group * p.bodies;
-    if (base >= p.n) return;
+    const int64_t group = kTeam > 1 ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kWarps + w;
+    const int64_t base = group * 32;
+    if (base >= p.n) return;  // (a team's grid is exact)
     const int64_t i = base + lane;
-    const bool valid = lane < p.bodies && i < p.n;
+    const bool valid = i < p.n;
     const int64_t ii = valid ? i : base;  // idle lanes shadow the group's first body
     const double x = p.px[ii], y = p.py[ii], z = p.pz[ii];
     // The group centre g: the first body's position truncated to FP32 on the
@@ -184,10 +193,10 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
         sm.bleaf[w][lane] = my_leaf;
         __syncwarp();
     }
-    int2* stk = sm.stack[w];
+    int2* stk = sm.stack[kTeam > 1 ? 0 : w];
     float4* L = kFP64 ? nullptr : sm.lst[w];
     int* LN = sm.lst_node[w];
-    int* LL = WalkSmem<kFP64, kLearn, kGroup>::kLL ? sm.lst_leaf[w] : nullptr;
+    int* LL = Smem::kLL ? sm.lst_leaf[w] : nullptr;
     unsigned* LM = sm.lst_mask[w];
     const unsigned me = 1u << lane;
     const unsigned lt = me - 1u;
@@ -202,7 +211,7 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
     float ascale = 0.0f;
     if (!kFP64) {
         const uint64_t my_id = valid ? p.id[i] : ~0ull;
-        for (int kk = 0; kk < p.nd; ++kk) {
+        for (int kk = kTeam > 1 ? w : 0; kk < p.nd; kk += kTeam) {
             if (!p.present[kk] || my_id == (uint64_t)kk) continue;
             const double dx = p.direct[4 * kk] - x, dy = p.direct[4 * kk + 1] - y, dz = p.direct[4 * kk + 2] - z;
             const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, soft2)));
@@ -233,52 +242,74 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
 
     int nlist = 0;
     int sp = 1;
-    if (lane == 0) stk[0] = make_int2(0, (int)full);  // the root: a range of one slot
+    if (lane == 0 && (kTeam == 1 || w == 0)) stk[0] = make_int2(0, (int)full);  // the root: a range of one slot
+    if (kTeam > 1) __syncthreads();
     __syncwarp();
     bool overflow = false;
     int64_t pops = 0;
 
-    while (sp > 0 || nlist > 0) {
-        if (sp > 0) {
-            // Pop whole ranges from the top while they fit in 32 lanes.
-            const int avail = sp < 32 ? sp : 32;
-            int rfirst = 0, rcnt = 0;
-            unsigned rmask = 0;
-            if (lane < avail) {
-                const int2 ent = stk[sp - 1 - lane];
-                rfirst = ent.x & ((1 << kSlotBits) - 1);
-                rcnt = (int)((unsigned)ent.x >> kSlotBits) + 1;
-                rmask = (unsigned)ent.y;
-            }
-            int incl = rcnt;
+    // (The list is empty whenever the stack is: the last round evaluates it.)
+    while (sp > 0) {
+        bool flush_now;
+        {
+            int R, node = -1;  // ranges taken off the stack; this lane's node
+            unsigned m_r = 0;
+            bool has;
+            if (kTeam > 1) {
+                R = sp < kTeamPop * kTeam ? sp : kTeamPop * kTeam;
+                const int r = sp - 1 - (kTeamPop * w + (lane >> 3));
+                has = false;
+                if (r >= 0) {
+                    const int2 ent = stk[r];
+                    has = (lane & 7) <= (int)((unsigned)ent.x >> kSlotBits);
+                    node = (ent.x & ((1 << kSlotBits) - 1)) + (lane & 7);
+                    m_r = (unsigned)ent.y;
+                }
+                pops += 1;
+                if (pops > p.max_pops) {  // the same in every warp
+                    overflow = true;
+                    break;
+                }
+            } else {
+                // Pop whole ranges from the top while they fit in 32 lanes.
+                const int avail = sp < 32 ? sp : 32;
+                int rfirst = 0, rcnt = 0;
+                unsigned rmask = 0;
+                if (lane < avail) {
+                    const int2 ent = stk[sp - 1 - lane];
+                    rfirst = ent.x & ((1 << kSlotBits) - 1);
+                    rcnt = (int)((unsigned)ent.x >> kSlotBits) + 1;
+                    rmask = (unsigned)ent.y;
+                }
+                int incl = rcnt;
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, off);
-                if (lane >= off) incl += t;
+                for (int off = 1; off < 32; off <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, incl, off);
+                    if (lane >= off) incl += t;
+                }
+                const bool take = lane < avail && incl <= 32;
+                R = __popc(__ballot_sync(0xffffffffu, take));
+                const int T = __shfl_sync(0xffffffffu, incl, R - 1);
+                const int rstart = incl - rcnt;
+                const unsigned starts = __reduce_or_sync(0xffffffffu, take ? (1u << rstart) : 0u);
+                const int rj = __popc(starts & ((2u << lane) - 1u)) - 1;
+                const int f_r = __shfl_sync(0xffffffffu, rfirst, rj);
+                const int s_r = __shfl_sync(0xffffffffu, rstart, rj);
+                m_r = __shfl_sync(0xffffffffu, rmask, rj);
+                pops += T;
+                if (sp - R + T > Smem::kStk || pops > p.max_pops) {
+                    overflow = true;
+                    break;
+                }
+                has = lane < T;
+                node = f_r + (lane - s_r);
             }
-            const bool take = lane < avail && incl <= 32;
-            const int R = __popc(__ballot_sync(0xffffffffu, take));
-            const int T = __shfl_sync(0xffffffffu, incl, R - 1);
-            const int rstart = incl - rcnt;
-            const unsigned starts = __reduce_or_sync(0xffffffffu, take ? (1u << rstart) : 0u);
-            const int rj = __popc(starts & ((2u << lane) - 1u)) - 1;
-            const int f_r = __shfl_sync(0xffffffffu, rfirst, rj);
-            const int s_r = __shfl_sync(0xffffffffu, rstart, rj);
-            const unsigned m_r = __shfl_sync(0xffffffffu, rmask, rj);
-            pops += T;
-            if (sp - R + T > WalkSmem<kFP64, kLearn, kGroup>::kStk || pops > p.max_pops) {
-                overflow = true;
-                break;
-            }
-            const int k = T;
-            int node = -1;
             unsigned M = 0, A = 0;
             int nc = 0, ref = 0, depth = 0;
             bool leaf = false, mixed = false, cand = false;
             float dmin2 = 0.f, dmax2 = 0.f, s2 = 0.f, nerr = 0.f;
             float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (lane < k) {
-                node = f_r + (lane - s_r);
+            if (has) {
                 M = m_r;
                 const float4 a = __ldg(p.A + node);
                 const float4 b = __ldg(p.B + node);
@@ -510,7 +541,7 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
                     P[6] = e.w;
                 }
                 if (kFP64) LN[pos] = node;
-                if (WalkSmem<kFP64, kLearn, kGroup>::kLL) LL[pos] = leaf ? ref : -1;  // for the own-leaf test
+                if (Smem::kLL) LL[pos] = leaf ? ref : -1;  // for the own-leaf test
                 LM[pos] = A;
             }
             nlist += __popc(am);
@@ -519,11 +550,27 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
             const unsigned rest = M & ~A;
             const bool push = !leaf && nc > 0 && rest != 0;
             const unsigned pm = __ballot_sync(0xffffffffu, push);
-            if (push) stk[sp + __popc(pm & lt)] = make_int2(ref | ((nc - 1) << kSlotBits), (int)rest);
-            sp += __popc(pm);
+            int at = sp, np = __popc(pm);
+            if (kTeam > 1) {
+                if (lane == 0) sm.pushed[w] = np;
+                __syncthreads();  // and every warp has read its ranges
+                const int v = lane < kTeam ? sm.pushed[lane] : 0;
+                at += __reduce_add_sync(0xffffffffu, lane < w ? v : 0);
+                np = __reduce_add_sync(0xffffffffu, v);
+                if (sp + np > Smem::kStk) {  // the same in every warp
+                    overflow = true;
+                    break;
+                }
+            }
+            if (push) stk[at + __popc(pm & lt)] = make_int2(ref | ((nc - 1) << kSlotBits), (int)rest);
+            sp += np;
+            // A team evaluates its lists together, when one is full: an
+            // evaluation is long, and the others would wait for it below.
+            if (kTeam > 1) flush_now = __syncthreads_or(nlist > Smem::kLst - 32);
+            else flush_now = nlist > Smem::kLst - 32;
             __syncwarp();
         }
-        if (nlist > WalkSmem<kFP64, kLearn, kGroup>::kLst - 32 || (sp == 0 && nlist > 0)) {
+        if (nlist > 0 && (flush_now || sp == 0)) {
             if (kLearn == kLearnCollect) {
                 nlist = 0;  // collection evaluates nothing
                 __syncwarp();
@@ -702,6 +749,29 @@ __global__ void __launch_bounds__(kThreads) traverse_masked_kernel(FParams p)
         ady += widen(oy);
         adz += widen(oz);
     }
+    if (kTeam > 1) {
+        // The team's sums, through the warps' list (FP64: run) tables.
+        __syncthreads();
+        auto table = [&](int u) {
+            return kFP64 ? &sm.seg[kFP64 ? u : 0][0][0] : reinterpret_cast<double*>(sm.lst[kFP64 ? 0 : u]);
+        };
+        double* T = table(w);
+        T[lane] = adx;
+        T[32 + lane] = ady;
+        T[64 + lane] = adz;
+        sm.lst_node[w][lane] = (int)cnt;
+        __syncthreads();
+        if (w > 0) return;
+        adx = ady = adz = 0.0;
+        cnt = 0;
+        for (int u = 0; u < kTeam; ++u) {
+            const double* U = table(u);
+            adx += U[lane];
+            ady += U[32 + lane];
+            adz += U[64 + lane];
+            cnt += (unsigned)sm.lst_node[u][lane];
+        }
+    }
 
     if (valid) {
         p.ax[i] = adx;
@@ -729,23 +799,22 @@ int grid_n(int64_t n)
     return (int)(b > 8 * bh::num_sms() ? 8 * bh::num_sms() : b);
 }
 
-template <bool kFP64, int kLearn, bool kGroup = false>
+template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1>
 int launch_walk(bh_context* ctx, const FParams& p)
 {
-    const size_t smem = sizeof(WalkSmem<kFP64, kLearn, kGroup>);
-    BH_CUDA_TRY(cudaFuncSetAttribute(traverse_masked_kernel<kFP64, kLearn, kGroup>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto kernel = traverse_masked_kernel<kFP64, kLearn, kGroup, kTeam>;
+    const size_t smem = sizeof(WalkSmem<kFP64, kLearn, kGroup, kTeam>);
+    BH_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // The plain walks keep their working set in shared memory and L2 (L1
     // hit rates are low): shared memory takes the whole carveout, for more
     // resident blocks.  The learned walk reads the network's weights through
     // L1 and keeps the default split.
     if (kLearn == kLearnNone)
-        BH_CUDA_TRY(cudaFuncSetAttribute(traverse_masked_kernel<kFP64, kLearn, kGroup>,
-                                         cudaFuncAttributePreferredSharedMemoryCarveout,
+        BH_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared));
-    const int64_t groups = (p.n + p.bodies - 1) / p.bodies;
-    const int64_t blocks = (groups + kWarps - 1) / kWarps;
-    traverse_masked_kernel<kFP64, kLearn, kGroup><<<(unsigned)blocks, kThreads, smem, ctx->stream>>>(p);
+    const int64_t groups = (p.n + 31) / 32;
+    const int64_t blocks = kTeam > 1 ? groups : (groups + kWarps - 1) / kWarps;
+    kernel<<<(unsigned)blocks, kTeam > 1 ? 32 * kTeam : kThreads, smem, ctx->stream>>>(p);
     BH_LAUNCH_CHECK(ctx);
     return BH_OK;
 }
@@ -792,7 +861,6 @@ int prepare_walk(bh_context* ctx, double theta, double G, double soft2, bool fp6
     }
     p = FParams{};
     p.n = n;
-    p.bodies = 32;
     p.px = ctx->px; p.py = ctx->py; p.pz = ctx->pz;
     p.id = ctx->id;
     p.body_leaf = ctx->body_leaf;
@@ -827,16 +895,35 @@ int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2
     int rc = prepare_walk(ctx, theta, G, soft2, fp64, p);
     if (rc) return rc;
     p.kick_h = kick_h;
+    // Warps per group, by the groups of 32 bodies each SM gets: one where they
+    // fill the chip, a team where they do not (forces in ms, theta 1.05, with
+    // teams of 1 / 4 / 8 / 16):
+    //   FP64 list: 45,000 bodies 0.49 / 0.45 / 0.64 / 1.10 (65,537: 0.54 /
+    //     0.62), 19,054 1.83 / 0.76 / 0.83 / 0.87, 12,000 1.50 / 0.59 / 0.59 /
+    //     0.53, 1,000 0.40 / 0.16 / 0.12 / 0.08;
+    //   FP32: 200,000 0.285 / 0.275 / 0.36 / 0.64 (300,149: 0.370 / 0.395),
+    //     30,000 0.128 / 0.069 / 0.083 / 0.118, 19,054 0.45 / 0.20 / 0.15 /
+    //     0.16, 8,000 0.32 / 0.14 / 0.09 / 0.08, 1,000 0.11 / 0.06 / 0.045 /
+    //     0.039;
+    //   FP32 group: 65,537 0.115 / 0.107 / 0.14 / 0.22 (100,003: 0.141 /
+    //     0.145), 30,000 0.100 / 0.063 / 0.083 / 0.119, 8,000 0.22 / 0.11 /
+    //     0.083 / 0.072.
+    const int64_t per_sm = (ctx->n + 32 * (int64_t)num_sms() - 1) / (32 * (int64_t)num_sms());
     if (fp64) {
-        // Bodies per warp: 32 while that gives the chip 12 warps per SM, and
-        // fewer below (the evaluation is balanced over the 32 threads however
-        // many bodies share it).  Forces in ms with 32 / 16 / 8 / 4 bodies:
-        // 65,537 bodies 0.54 / 0.55 / 0.52 / 0.62, 19,054 1.83 / 1.27 / 0.92 /
-        // 1.08, 8,000 1.29 / 0.80 / 0.59 / 0.46.
-        while (p.bodies > 4 && ctx->n < 12 * (int64_t)num_sms() * p.bodies) p.bodies >>= 1;
+        if (per_sm <= 2) return launch_walk<true, kLearnNone, false, 16>(ctx, p);
+        if (per_sm <= 10) return launch_walk<true, kLearnNone, false, 4>(ctx, p);
         return launch_walk<true, kLearnNone>(ctx, p);
     }
-    return group ? launch_walk<false, kLearnNone, true>(ctx, p) : launch_walk<false, kLearnNone>(ctx, p);
+    if (group) {
+        if (per_sm <= 2) return launch_walk<false, kLearnNone, true, 16>(ctx, p);
+        if (per_sm <= 5) return launch_walk<false, kLearnNone, true, 8>(ctx, p);
+        if (per_sm <= 18) return launch_walk<false, kLearnNone, true, 4>(ctx, p);
+        return launch_walk<false, kLearnNone, true>(ctx, p);
+    }
+    if (per_sm <= 2) return launch_walk<false, kLearnNone, false, 16>(ctx, p);
+    if (per_sm <= 5) return launch_walk<false, kLearnNone, false, 8>(ctx, p);
+    if (per_sm <= 42) return launch_walk<false, kLearnNone, false, 4>(ctx, p);
+    return launch_walk<false, kLearnNone>(ctx, p);
 }
 
 int launch_collect(bh_context* ctx, double theta, double G, double theta_max, int32_t* c_group, int32_t* c_slot,

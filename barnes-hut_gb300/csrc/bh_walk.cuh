@@ -30,17 +30,25 @@ constexpr float kAbsErr = 1e-6f;  // bound on FP32 coordinate error, relative to
 
 enum { kLearnNone = 0, kLearnInfer = 1, kLearnCollect = 2 };
 
+// A team of warps sharing one group's walk (see traverse_masked_kernel): its
+// sibling ranges, of which the warps take kTeamPop each per round.
+constexpr int kTeamStack = 2048;
+constexpr int kTeamPop = 4;
+
 // Per-block shared memory of the walk.  Tables a variant does not use shrink
 // to one element, so that the FP32 walk fits 8 blocks (32 warps) per SM; the
 // FP64 walk fits 5 (6 ran slower: the FP64 pipe is already 86 % busy).
-template <bool kFP64, int kLearn, bool kGroup = false>
+template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1>
 struct WalkSmem {
+    static constexpr int kWarps = kTeam > 1 ? kTeam : bh::kWarps;  // per block
     static constexpr int kW64 = kFP64 ? kWarps : 1;      // FP64-only tables
     static constexpr bool kLL = kFP64;                    // leaf ids kept for the evaluation's own-leaf test
     static constexpr bool kF = kLearn == 1;              // network input rows
-    static constexpr int kStk = kFP64 ? kStack64 : kStack;  // stack entries per warp
+    static constexpr int kStk = kTeam > 1 ? kTeamStack : kFP64 ? kStack64 : kStack;  // stack entries
     static constexpr int kLst = kFP64 ? kList64 : kGroup ? kListGroup : kList;  // staged entries per warp
-    int2 stack[kWarps][kStk];  // sibling ranges: {first | (count - 1) << 28, lane mask}
+    // sibling ranges: {first | (count - 1) << 28, lane mask}, per warp or team
+    int2 stack[kTeam > 1 ? 1 : kWarps][kStk];
+    int pushed[kTeam > 1 ? kTeam : 1];  // ranges each warp of a team pushes in a round
     // FP32 node data of the staged entries: {x, y, z, G m} per entry, or in
     // the plain FP32 walk entry pairs {x0, x1, y0, y1}, {z0, z1, w0, w1}
     float4 lst[kFP64 ? 1 : kWarps][kFP64 ? 1 : kLst];
@@ -109,7 +117,6 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
 
 struct FParams {
     int64_t n;
-    int bodies;  // per warp group: a power of two up to 32
     const double* px;
     const double* py;
     const double* pz;
