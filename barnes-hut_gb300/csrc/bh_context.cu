@@ -197,6 +197,17 @@ int download_vec3(bh_context* ctx, double* host_aos, double* stage, const double
     return BH_OK;
 }
 
+}  // namespace
+
+int bh::download_accelerations(bh_context* ctx, double* acc_out)
+{
+    if (int rc = download_vec3(ctx, acc_out, ctx->px2, ctx->ax, ctx->ay, ctx->az, ctx->n)) return rc;
+    BH_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    return BH_OK;
+}
+
+namespace {
+
 cudaEvent_t next_event(bh_context* ctx)
 {
     if (ctx->ev_used == ctx->ev_pool.size()) {

@@ -401,7 +401,7 @@ struct bh_context {
     // and the topology word; 2n entries each.
     float4* fA = nullptr;   // {hi.x, hi.y, hi.z, G m}
     float4* fB = nullptr;   // {lo.x, lo.y, lo.z, bits of ref (child or leaf id)}
-    uint32_t* fmeta = nullptr;  // nchild | depth << 8 | leaf << 16
+    uint32_t* fmeta = nullptr;  // nchild | depth << 8 | leaf << 16 | massless << 17 | chain above the leaf << 18
     double4_32a* d4 = nullptr;  // FP64 walk: {cx, cy, cz, G m} per slot
     bool fnodes_fused = false;  // fA / fB / fmeta are current for rec and fnodes_G
     double fnodes_G = 0.0;
@@ -487,6 +487,8 @@ int launch_build(bh_context* ctx, const double* mass, bool moments = false, bool
 // The FP64 records of the current tree, written by a rebuild of its node
 // values where the last build left them out (no-op otherwise).
 int ensure_rec(bh_context* ctx);
+// The accelerations in the current body order to the host (n*3); waits.
+int download_accelerations(bh_context* ctx, double* acc_out);
 // Waits for the context's stream and turns a raised device error word into
 // a status (clearing the word).
 int finish(bh_context* ctx, const char* fn);
@@ -494,6 +496,20 @@ int finish(bh_context* ctx, const char* fn);
 int launch_direct_extract(bh_context* ctx, double G);
 
 int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int mode, double kick_h);
+// The exact walk (BH_MODE_PLAIN_FP64) over node records: A {hi.x, hi.y, hi.z,
+// G m}, B {lo.x, lo.y, lo.z, bits of first child or leaf id}, meta (nchild |
+// depth << 8 | leaf << 16 | massless << 17 | chain above the leaf << 18), d4
+// {cx, cy, cz, G m}; node 0 is the root, a node's children are consecutive in
+// octant order.  Accelerations into ctx; the counters may be null.
+struct ExactTree {
+    int64_t nodes;
+    const float4* A;
+    const float4* B;
+    const uint32_t* meta;
+    const double4_32a* d4;
+};
+int launch_exact_walk(bh_context* ctx, const ExactTree& tree, double theta, double soft2, double kick_h,
+                      int32_t* body_count, unsigned long long* inter_count, unsigned* err);
 int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2, double kick_h, bool fp64,
                            bool group = false);
 int launch_traverse_learned(bh_context* ctx, double theta, double G, double soft2, double kick_h);

@@ -49,18 +49,13 @@ struct TravParams {
     const double* py;
     const double* pz;
     const int32_t* body_leaf;
-    const TreeRec* rec;
-    const double4_32a* d4;  // {cx, cy, cz, G m} per slot
-    const float4* A;        // FP32 node records (group tests)
-    const float4* B;
-    const uint32_t* meta;
+    ExactTree tree;
     const double* bbox;
     double theta2;
-    double G;
     double soft2;
     double kick_h;  // > 0: also apply the second half kick v += kick_h * a
     double one;        // 1.0, as a run-time value: RN(a 1 + b) stays an FMA
-    int64_t max_pops;  // upper bound on tree slots (2n)
+    int64_t max_passes;  // above the nodes a walk can meet
     double* ax;
     double* ay;
     double* az;
@@ -125,7 +120,7 @@ struct ExactSmem {
     int plist[kTravWarps][kCap][kBodies];
     double term[kTravWarps][3][32];  // the terms of one step of an evaluation
     // Nodes the box cannot decide: {centre, allowance}, {depth of the test,
-    // node, leaf id or -1}.
+    // node, leaf id or -1, a chain above the leaf}.
     float4 und[kTravWarps][32];
     int4 und2[kTravWarps][32];
     double side2[kMaxDepth + 1];
@@ -237,7 +232,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
         for (; most > left; most -= P) {
             const int q = done + phase;
             const bool on = q < cnt;
-            const double4_32a r = p.d4[on ? PL[q & (Smem::kCap - 1)][body] : 0];
+            const double4_32a r = p.tree.d4[on ? PL[q & (Smem::kCap - 1)][body] : 0];
             double tx, ty, tz;
             exact_term<kSoft>(r, px, py, pz, soft2, on, one, tx, ty, tz);
             auto T = sm.term[w];
@@ -258,7 +253,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
     };
 
     while (sp > 0) {
-        if (++passes > p.max_pops) {
+        if (++passes > p.max_passes) {
             overflow = true;
             break;
         }
@@ -267,7 +262,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
         const int m = sp < 32 ? sp : 32;
         int node = 0, nc = 0, ref = 0, depth = 0;
         unsigned M = 0, A = 0;
-        bool test = false, leaf = false, mixed = false;
+        bool test = false, leaf = false, chain = false, mixed = false;
         float cx = 0.f, cy = 0.f, cz = 0.f, nerr = 0.f;  // group-relative centre, its allowance
         if (lane < m) {
             const int2 it = stk[sp - 1 - lane];
@@ -277,14 +272,15 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
                 A = M;
             } else {
                 test = true;
-                const float4 a = __ldg(p.A + node);
-                const float4 b = __ldg(p.B + node);
-                const uint32_t mt = __ldg(p.meta + node);
+                const float4 a = __ldg(p.tree.A + node);
+                const float4 b = __ldg(p.tree.B + node);
+                const uint32_t mt = __ldg(p.tree.meta + node);
                 cx = (a.x - gx) + b.x;
                 cy = (a.y - gy) + b.y;
                 cz = (a.z - gz) + b.z;
                 ref = __float_as_int(b.w);
                 leaf = (mt >> 16) & 1u;
+                chain = (mt >> 18) & 1u;
                 depth = (mt >> 8) & 0xFF;
                 nerr = kAbsErr * (fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + bmag);
                 if ((mt >> 17) & 1u) {
@@ -319,7 +315,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
             const int k = __popc(ub & lt);
             if (mixed || own) {
                 sm.und[w][k] = make_float4(cx, cy, cz, nerr);
-                sm.und2[w][k] = make_int4(own ? kMaxDepth - 1 : depth, node, own ? ref : -1, 0);
+                sm.und2[w][k] = make_int4(own ? kMaxDepth - 1 : depth, node, own ? ref : -1, chain ? 1 : 0);
             }
             __syncwarp();
             const int nu = __popc(ub);
@@ -336,11 +332,11 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
                     if (v.z >= 0 ? v.z != my_leaf : sure_below(s2, theta2f, lo * lo + soft2f)) {
                         acc = true;
                     } else if (!sure_above(s2, theta2f, hi * hi + soft2f)) {
-                        const TreeRec r = p.rec[v.y];
-                        const double dx = __dsub_rn(r.cx, px), dy = __dsub_rn(r.cy, py), dz = __dsub_rn(r.cz, pz);
+                        const double4_32a r = p.tree.d4[v.y];
+                        const double dx = __dsub_rn(r.x, px), dy = __dsub_rn(r.y, py), dz = __dsub_rn(r.z, pz);
                         const double r2 = __dadd_rn(
                             __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)), soft2);
-                        acc = (v.z < 0 || r.top <= kMaxDepth - 1) && sm.side2[v.x] < __dmul_rn(theta2, r2);
+                        acc = (v.z < 0 || v.w != 0) && sm.side2[v.x] < __dmul_rn(theta2, r2);
                     }
                 }
                 const unsigned res = __ballot_sync(0xffffffffu, acc);
@@ -457,7 +453,8 @@ int launch_exact_p(bh_context* ctx, const TravParams& p)
 
 }  // namespace
 
-int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int mode, double kick_h)
+int launch_exact_walk(bh_context* ctx, const ExactTree& tree, double theta, double soft2, double kick_h,
+                      int32_t* body_count, unsigned long long* inter_count, unsigned* err)
 {
     const int64_t n = ctx->n;
     if (n == 0) return BH_OK;
@@ -465,40 +462,42 @@ int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int m
     p.n = n;
     p.px = ctx->px; p.py = ctx->py; p.pz = ctx->pz;
     p.body_leaf = ctx->body_leaf;
-    p.rec = ctx->rec;
-    p.d4 = ctx->d4;
-    p.A = ctx->fA; p.B = ctx->fB; p.meta = ctx->fmeta;
+    p.tree = tree;
     p.bbox = ctx->bbox;
     p.theta2 = theta * theta;
-    p.G = G;
     p.soft2 = soft2;
     p.kick_h = kick_h;
     p.one = 1.0;
-    p.max_pops = 2 * n + 2;
+    p.max_passes = 2 * tree.nodes + 2;
     p.ax = ctx->ax; p.ay = ctx->ay; p.az = ctx->az;
     p.vx = ctx->vx; p.vy = ctx->vy; p.vz = ctx->vz;
-    p.inter_count = ctx->inter_count;
-    p.body_count = ctx->body_count;
-    p.err = ctx->err;
-    BH_CUDA_TRY(cudaMemsetAsync(ctx->inter_count, 0, sizeof(unsigned long long), ctx->stream));
-    // Lanes to a body in the exact walk: 4 (the evaluation's sums fill 24 lanes
-    // and the bodies share a walk) while that gives the chip 12 warps per SM,
-    // and more below, where a warp's own latency counts.  Forces in ms with
-    // 4 / 8 / 16 / 32 lanes: 300,149 bodies 2.96 / 3.67 / 5.36 / -, 19,054
-    // 1.21 / 1.26 / 1.39 / -, 8,000 0.69 / 0.46 / - / -, 4,000 0.44 / 0.29 /
-    // 0.23 / 0.25, 1,000 0.20 / 0.13 / 0.095 / 0.070.
+    p.inter_count = inter_count;
+    p.body_count = body_count;
+    p.err = err;
+    // Lanes to a body: 4 (the evaluation's sums fill 24 lanes and the bodies
+    // share a walk) while that gives the chip 12 warps per SM, and more below,
+    // where a warp's own latency counts.  Forces in ms with 4 / 8 / 16 / 32
+    // lanes: 300,149 bodies 2.96 / 3.67 / 5.36 / -, 19,054 1.21 / 1.26 / 1.39 /
+    // -, 8,000 0.69 / 0.46 / - / -, 4,000 0.44 / 0.29 / 0.23 / 0.25, 1,000
+    // 0.20 / 0.13 / 0.095 / 0.070.
     const int64_t want = 12 * (int64_t)num_sms() * 32;
-    const int lanes = n * 4 >= want ? 4 : n * 8 >= want ? 8 : n * 16 >= want ? 16 : 32;
+    if (n * 4 >= want) return launch_exact_p<4>(ctx, p);
+    if (n * 8 >= want) return launch_exact_p<8>(ctx, p);
+    if (n * 16 >= want) return launch_exact_p<16>(ctx, p);
+    return launch_exact_p<32>(ctx, p);
+}
+
+int launch_traverse(bh_context* ctx, double theta, double G, double soft2, int mode, double kick_h)
+{
+    const int64_t n = ctx->n;
+    if (n == 0) return BH_OK;
+    BH_CUDA_TRY(cudaMemsetAsync(ctx->inter_count, 0, sizeof(unsigned long long), ctx->stream));
     switch (mode) {
     case BH_MODE_PLAIN_FP64: {
         const int rc = launch_fp32_nodes(ctx, G, true);
         if (rc) return rc;
-        switch (lanes) {
-        case 4: return launch_exact_p<4>(ctx, p);
-        case 8: return launch_exact_p<8>(ctx, p);
-        case 16: return launch_exact_p<16>(ctx, p);
-        default: return launch_exact_p<32>(ctx, p);
-        }
+        return launch_exact_walk(ctx, ExactTree{2 * n, ctx->fA, ctx->fB, ctx->fmeta, ctx->d4}, theta, soft2, kick_h,
+                                 ctx->body_count, ctx->inter_count, ctx->err);
     }
     case BH_MODE_FP64_LIST:
         return launch_traverse_masked(ctx, theta, G, soft2, kick_h, true);

@@ -64,7 +64,8 @@ __global__ void fp32_nodes_kernel(const int32_t* __restrict__ counts, const Tree
         A[s] = make_float4(narrow_trunc(r.cx), narrow_trunc(r.cy), narrow_trunc(r.cz), narrow_trunc(G * r.m));
         B[s] = make_float4(low_part(r.cx), low_part(r.cy), low_part(r.cz), __int_as_float(leaf ? r.leaf : r.child));
         meta[s] = (uint32_t)r.nchild | ((uint32_t)r.depth << 8) | ((leaf ? 1u : 0u) << 16) |
-                  ((__double_as_longlong(r.m) << 1) == 0 ? 1u << 17 : 0u);
+                  ((__double_as_longlong(r.m) << 1) == 0 ? 1u << 17 : 0u) |
+                  (leaf && r.top <= kMaxDepth - 1 ? 1u << 18 : 0u);
     }
 }
 

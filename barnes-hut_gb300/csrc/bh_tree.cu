@@ -624,7 +624,7 @@ __device__ inline void far_com(double m, double wx, double wy, double wz, TreeRe
 struct FarOut {
     float4* A;       // {hi.x, hi.y, hi.z, G m}
     float4* B;       // {lo.x, lo.y, lo.z, bits of child or leaf id}
-    uint32_t* meta;  // nchild | depth << 8 | leaf << 16 | massless << 17
+    uint32_t* meta;  // nchild | depth << 8 | leaf << 16 | massless << 17 | chain above the leaf << 18
     double G;
 };
 
@@ -684,7 +684,8 @@ __global__ void finalize_kernel(const int32_t* __restrict__ counts, const int32_
             far.B[s] = make_float4(low_part(o.cx), low_part(o.cy), low_part(o.cz),
                                    __int_as_float(leaf ? o.leaf : o.child));
             far.meta[s] = (uint32_t)o.nchild | ((uint32_t)o.depth << 8) | ((leaf ? 1u : 0u) << 16) |
-                          ((__double_as_longlong(o.m) << 1) == 0 ? 1u << 17 : 0u);
+                          ((__double_as_longlong(o.m) << 1) == 0 ? 1u << 17 : 0u) |
+                          (leaf && o.top <= kMaxDepth - 1 ? 1u << 18 : 0u);
         }
         if (kMoments) {  // a feature: FP32 after narrowing on the bit patterns
             const double m = v.w;
