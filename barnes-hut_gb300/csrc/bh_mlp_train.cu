@@ -19,157 +19,343 @@
 namespace bh {
 namespace {
 
-constexpr int kFbThreads = 128;
+// A batch's samples are dealt to four row sets, sample b to row b / 4 of set
+// b % 4 (the four interleaved partial sums of dW2); `rows` rows are allotted to
+// each set, a multiple of kRowStep.
+constexpr int kFbSamples = 32;  // samples per block of the forward/backward kernel
+constexpr int kFbThreads = 256;
+constexpr int kRowStep = 64;
 
 struct Scratch {
-    float *xb, *h1b, *h2b, *dh1, *dh2, *dy, *loss_part;
+    int rows;
+    float* h1;    // [4][rows][64] layer-1 outputs
+    float* xb;    // [4][rows][8] inputs
+    float* dh1;   // [4][64][rows] layer deltas and layer-2 outputs, by unit
+    float* dh2;
+    float* h2;
+    float* dy;    // [4][rows]
+    float* loss_part;  // per 32 samples
+    float* p_w2;  // [4][64 * 64] partial sums of the gradient
+    float* p_w1;  // [32][64 * 8]
+    float* p_b;   // [64][193]: b1, b2, W3, b3
+};
+constexpr int kBiasParts = 3 * kHid + 1;
+
+struct FbSmem {
+    float W2[kHid * kHid];   // [i][j]
+    float W2t[kHid * kHid];  // [j][i]
+    float h1[kHid][kFbSamples];
+    float h2[kHid][kFbSamples];
+    float d2[kHid][kFbSamples];
+    float W1[kHid * kFeat], b1[kHid], b2[kHid], W3[kHid];
+    float b3;
 };
 
-// One thread per sample: forward, loss, backward to the layer deltas.
+// Forward, loss and backward to the layer deltas for 32 samples: lane = sample,
+// warp w computes units 8 w .. 8 w + 7 of each layer, so that eight independent
+// sums run beside one another and every weight is read by broadcast.  Each sum
+// keeps the order of its terms.  What bounds it is latency (a block's 32
+// samples are a chain of three small layers); one thread per sample, 32 blocks
+// of 128 on the whole chip, took 58 us for a batch of 4,096.
 __global__ void __launch_bounds__(kFbThreads) mlp_fwd_bwd_kernel(const float* __restrict__ X,
                                                                 const float* __restrict__ T,
                                                                 const int32_t* __restrict__ idx, int64_t off,
                                                                 int B, float inv_b, const float* __restrict__ P,
                                                                 Scratch s)
 {
-    __shared__ float W1[kHid * kFeat], b1[kHid], W2[kHid * kHid], b2[kHid], W3[kHid];
-    __shared__ float b3;
-    __shared__ float red[kFbThreads / 32];
-    for (int k = threadIdx.x; k < kHid * kHid; k += blockDim.x) W2[k] = bf16r(P[kOffW2 + k]);
-    for (int k = threadIdx.x; k < kHid * kFeat; k += blockDim.x) W1[k] = bf16r(P[kOffW1 + k]);
-    for (int k = threadIdx.x; k < kHid; k += blockDim.x) {
-        b1[k] = P[kOffB1 + k];
-        b2[k] = P[kOffB2 + k];
-        W3[k] = bf16r(P[kOffW3 + k]);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FbSmem& m = *reinterpret_cast<FbSmem*>(smem_raw);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, u0 = 8 * w;
+    for (int k = threadIdx.x; k < kHid * kHid; k += kFbThreads) {
+        const float v = bf16r(P[kOffW2 + k]);
+        m.W2[k] = v;
+        m.W2t[(k % kHid) * kHid + k / kHid] = v;
     }
-    if (threadIdx.x == 0) b3 = P[kOffB3];
+    for (int k = threadIdx.x; k < kHid * kFeat; k += kFbThreads) m.W1[k] = bf16r(P[kOffW1 + k]);
+    if (threadIdx.x < kHid) {
+        m.b1[threadIdx.x] = P[kOffB1 + threadIdx.x];
+        m.b2[threadIdx.x] = P[kOffB2 + threadIdx.x];
+        m.W3[threadIdx.x] = bf16r(P[kOffW3 + threadIdx.x]);
+    }
+    if (threadIdx.x == 0) m.b3 = P[kOffB3];
+    const int b = blockIdx.x * kFbSamples + lane;
+    const bool live = b < B;
+    const int64_t sidx = live ? (idx ? (int64_t)idx[off + b] : off + b) : 0;
+    float xb[kFeat];
+#pragma unroll
+    for (int k = 0; k < kFeat; ++k) xb[k] = live ? bf16r(X[sidx * kFeat + k]) : 0.0f;
+    const float target = live ? T[sidx] : 0.0f;
     __syncthreads();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    float l2 = 0.0f;
-    if (b < B) {
-        const int64_t sidx = idx ? (int64_t)idx[off + b] : off + b;
-        float xb[kFeat];
+    float h1[8];
 #pragma unroll
-        for (int k = 0; k < kFeat; ++k) xb[k] = bf16r(X[sidx * kFeat + k]);
-        float h1[kHid];
+    for (int u = 0; u < 8; ++u) {
+        float a = m.b1[u0 + u];
 #pragma unroll
-        for (int i = 0; i < kHid; ++i) {
-            float a = b1[i];
+        for (int k = 0; k < kFeat; ++k) a = fmaf(m.W1[(u0 + u) * kFeat + k], xb[k], a);
+        h1[u] = bf16r(fmaxf(a, 0.0f));
+        m.h1[u0 + u][lane] = h1[u];
+    }
+    __syncthreads();
+    float acc[8], h2[8];
 #pragma unroll
-            for (int k = 0; k < kFeat; ++k) a = fmaf(W1[i * kFeat + k], xb[k], a);
-            h1[i] = bf16r(fmaxf(a, 0.0f));
+    for (int u = 0; u < 8; ++u) acc[u] = m.b2[u0 + u];
+#pragma unroll 8
+    for (int j = 0; j < kHid; ++j) {
+        const float h = m.h1[j][lane];
+        const float4 v0 = *reinterpret_cast<const float4*>(&m.W2t[j * kHid + u0]);
+        const float4 v1 = *reinterpret_cast<const float4*>(&m.W2t[j * kHid + u0 + 4]);
+        acc[0] = fmaf(v0.x, h, acc[0]); acc[1] = fmaf(v0.y, h, acc[1]);
+        acc[2] = fmaf(v0.z, h, acc[2]); acc[3] = fmaf(v0.w, h, acc[3]);
+        acc[4] = fmaf(v1.x, h, acc[4]); acc[5] = fmaf(v1.y, h, acc[5]);
+        acc[6] = fmaf(v1.z, h, acc[6]); acc[7] = fmaf(v1.w, h, acc[7]);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        h2[u] = bf16r(fmaxf(acc[u], 0.0f));
+        m.h2[u0 + u][lane] = h2[u];
+    }
+    __syncthreads();
+    float y = m.b3;  // in every warp
+#pragma unroll 16
+    for (int i = 0; i < kHid; ++i) y = fmaf(m.W3[i], m.h2[i][lane], y);
+    const float diff = y - target;
+    const float dy = 2.0f * diff * inv_b;
+    float d2[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        d2[u] = h2[u] > 0.0f ? dy * m.W3[u0 + u] : 0.0f;
+        m.d2[u0 + u][lane] = d2[u];
+        acc[u] = 0.0f;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int i = 0; i < kHid; ++i) {
+        const float d = m.d2[i][lane];
+        const float4 v0 = *reinterpret_cast<const float4*>(&m.W2[i * kHid + u0]);
+        const float4 v1 = *reinterpret_cast<const float4*>(&m.W2[i * kHid + u0 + 4]);
+        acc[0] = fmaf(d, v0.x, acc[0]); acc[1] = fmaf(d, v0.y, acc[1]);
+        acc[2] = fmaf(d, v0.z, acc[2]); acc[3] = fmaf(d, v0.w, acc[3]);
+        acc[4] = fmaf(d, v1.x, acc[4]); acc[5] = fmaf(d, v1.y, acc[5]);
+        acc[6] = fmaf(d, v1.z, acc[6]); acc[7] = fmaf(d, v1.w, acc[7]);
+    }
+    if (live) {
+        const int q = b & 3, r = b >> 2;
+        float4* o = reinterpret_cast<float4*>(s.h1 + ((int64_t)q * s.rows + r) * kHid + u0);
+        o[0] = make_float4(h1[0], h1[1], h1[2], h1[3]);
+        o[1] = make_float4(h1[4], h1[5], h1[6], h1[7]);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int64_t k = ((int64_t)q * kHid + u0 + u) * s.rows + r;
+            s.dh1[k] = h1[u] > 0.0f ? acc[u] : 0.0f;
+            s.dh2[k] = d2[u];
+            s.h2[k] = h2[u];
         }
-        float h2[kHid];
-        float y = b3;
-#pragma unroll 4
-        for (int i = 0; i < kHid; ++i) {
-            float a = b2[i];
-#pragma unroll
-            for (int j = 0; j < kHid; ++j) a = fmaf(W2[i * kHid + j], h1[j], a);
-            h2[i] = bf16r(fmaxf(a, 0.0f));
-        }
-#pragma unroll
-        for (int i = 0; i < kHid; ++i) y = fmaf(W3[i], h2[i], y);
-        const float diff = y - T[sidx];
-        l2 = diff * diff;
-        const float dy = 2.0f * diff * inv_b;
-        s.dy[b] = dy;
-#pragma unroll
-        for (int k = 0; k < kFeat; ++k) s.xb[(int64_t)b * kFeat + k] = xb[k];
-#pragma unroll
-        for (int i = 0; i < kHid; ++i) {
-            s.h1b[(int64_t)b * kHid + i] = h1[i];
-            s.h2b[(int64_t)b * kHid + i] = h2[i];
-            h2[i] = h2[i] > 0.0f ? dy * W3[i] : 0.0f;  // now dh2
-            s.dh2[(int64_t)b * kHid + i] = h2[i];
-        }
-#pragma unroll 4
-        for (int j = 0; j < kHid; ++j) {
-            float a = 0.0f;
-#pragma unroll
-            for (int i = 0; i < kHid; ++i) a = fmaf(h2[i], W2[i * kHid + j], a);
-            s.dh1[(int64_t)b * kHid + j] = h1[j] > 0.0f ? a : 0.0f;
+        if (w == 0) {
+            float4* x = reinterpret_cast<float4*>(s.xb + ((int64_t)q * s.rows + r) * kFeat);
+            x[0] = make_float4(xb[0], xb[1], xb[2], xb[3]);
+            x[1] = make_float4(xb[4], xb[5], xb[6], xb[7]);
+            s.dy[(int64_t)q * s.rows + r] = dy;
         }
     }
-    // block partial of the squared error
+    if (w == 0) {
+        float l2 = live ? diff * diff : 0.0f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l2 += __shfl_down_sync(0xffffffffu, l2, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l2;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int k = 0; k < kFbThreads / 32; ++k) t += red[k];
-        s.loss_part[blockIdx.x] = t;
+        for (int o = 16; o > 0; o >>= 1) l2 += __shfl_down_sync(0xffffffffu, l2, o);
+        if (lane == 0) s.loss_part[blockIdx.x] = l2;
     }
 }
 
-// Block i reduces every gradient entry of hidden unit i over the batch.
-__global__ void __launch_bounds__(256) mlp_grad_reduce_kernel(int B, int nloss, Scratch s, float* __restrict__ g,
-                                                             float* __restrict__ loss_out, float inv_b)
+__device__ __forceinline__ void copy16(void* smem, const void* global)
 {
-    __shared__ float part[256];
-    const int i = blockIdx.x, t = threadIdx.x;
-    // dW2[i][j] = sum_b dh2[b][i] h1b[b][j]: 64 columns x 4 partial sums
-    {
-        const int j = t & 63, q = t >> 6;
-        float a = 0.0f;
-        for (int b = q; b < B; b += 4) a = fmaf(s.dh2[(int64_t)b * kHid + i], s.h1b[(int64_t)b * kHid + j], a);
-        part[t] = a;
-        __syncthreads();
-        if (t < 64) g[kOffW2 + i * kHid + t] = (part[t] + part[t + 64]) + (part[t + 128] + part[t + 192]);
-        __syncthreads();
-    }
-    // dW1[i][k] = sum_b dh1[b][i] xb[b][k]: 8 columns x 32 partial sums
-    {
-        const int k = t & 7, q = t >> 3;
-        float a = 0.0f;
-        for (int b = q; b < B; b += 32) a = fmaf(s.dh1[(int64_t)b * kHid + i], s.xb[(int64_t)b * kFeat + k], a);
-        part[t] = a;
-        __syncthreads();
-        if (t < 8) {
-            float r = 0.0f;
-            for (int u = 0; u < 32; ++u) r += part[u * 8 + t];
-            g[kOffW1 + i * kFeat + t] = r;
-        }
-        __syncthreads();
-    }
-    // db1[i], db2[i], dW3[i]: 3 sums x 64 partials (+ db3 and the loss in block 0)
-    {
-        const int which = t >> 6, q = t & 63;
-        float a = 0.0f;
-        if (which == 0)
-            for (int b = q; b < B; b += 64) a += s.dh1[(int64_t)b * kHid + i];
-        else if (which == 1)
-            for (int b = q; b < B; b += 64) a += s.dh2[(int64_t)b * kHid + i];
-        else if (which == 2)
-            for (int b = q; b < B; b += 64) a = fmaf(s.dy[b], s.h2b[(int64_t)b * kHid + i], a);
-        else if (i == 0)
-            for (int b = q; b < B; b += 64) a += s.dy[b];
-        part[t] = a;
-        __syncthreads();
-        if (t < 4) {
-            float r = 0.0f;
-            for (int u = 0; u < 64; ++u) r += part[t * 64 + u];
-            if (t == 0) g[kOffB1 + i] = r;
-            if (t == 1) g[kOffB2 + i] = r;
-            if (t == 2) g[kOffW3 + i] = r;
-            if (t == 3 && i == 0) g[kOffB3] = r;
-        }
-        if (i == 0 && t == 0 && loss_out) {
-            float l = 0.0f;
-            for (int u = 0; u < nloss; ++u) l += s.loss_part[u];
-            loss_out[0] = l * inv_b;
-            loss_out[1] += l * inv_b;  // running sum over the epoch
-        }
-    }
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+                 "l"(global));
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n"); }
+template <int N>
+__device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-__global__ void adam_kernel(float* __restrict__ P, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, float lr, float b1, float b2, float c1, float c2, float eps)
+// The gradient's sums over the batch, to partial sums (one term after the
+// other within each, in batch order).  Blocks 0..63: dW2[i][j] = sum dh2[i]
+// h1[j] for four units i and one row set, one sum per thread: a chain of B / 4
+// FMAs, four cycles each, which is what bounds it (a batch of 4,096: 4,096
+// cycles, 2.1 us), while the rows stream through shared memory four steps
+// ahead.  Blocks 64..95: the sums over 32 (dW1) and 64 (biases, W3) interleaved
+// parts for eight units and one row set.  Reading the rows from L2 as they were
+// needed, 64 blocks took 75 us for a batch of 4,096.
+constexpr int kReduceThreads = 256;
+constexpr int kW2Units = 4;                       // units per block
+constexpr int kW2Blocks = 4 * kHid / kW2Units;    // 64
+constexpr int kSmallUnits = 8;
+constexpr int kSmallBlocks = 4 * kHid / kSmallUnits;  // 32
+constexpr int kSteps = 4;  // copies in flight
+
+struct W2Step {
+    float h1[kRowStep][kHid];
+    float d2[kW2Units][kRowStep];
+};
+struct SmallTile {
+    float dh1[kSmallUnits][kRowStep], dh2[kSmallUnits][kRowStep], h2[kSmallUnits][kRowStep];
+    float xb[kRowStep][kFeat];
+    float dy[kRowStep];
+};
+constexpr size_t kReduceSmem =
+    kSteps * (sizeof(W2Step) > sizeof(SmallTile) ? sizeof(W2Step) : sizeof(SmallTile));
+
+__global__ void __launch_bounds__(kReduceThreads) mlp_grad_reduce_kernel(int B, Scratch s)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int t = threadIdx.x;
+    const bool small = blockIdx.x >= kW2Blocks;
+    const int q = blockIdx.x & 3;
+    const int g = (small ? blockIdx.x - kW2Blocks : blockIdx.x) >> 2;
+    const int n = (B - q + 3) / 4;  // rows of this set
+    const int steps = (n + kRowStep - 1) / kRowStep;
+    if (!small) {
+        W2Step* st = reinterpret_cast<W2Step*>(smem_raw);
+        const int j = t & 63, ii = t >> 6, i0 = g * kW2Units;
+        const float* h1 = s.h1 + (int64_t)q * s.rows * kHid;
+        const float* d2 = s.dh2 + ((int64_t)q * kHid + i0) * s.rows;
+        auto fetch = [&](int k) {
+            if (k < steps) {
+                W2Step& c = st[k % kSteps];
+                const float* src = h1 + (int64_t)k * kRowStep * kHid;
+#pragma unroll
+                for (int o = 0; o < kRowStep * kHid / 4; o += kReduceThreads)
+                    copy16(&c.h1[0][0] + 4 * (o + t), src + 4 * (o + t));
+                if (t < kW2Units * kRowStep / 4)
+                    copy16(&c.d2[t / 16][4 * (t % 16)], d2 + (int64_t)(t / 16) * s.rows + k * kRowStep + 4 * (t % 16));
+            }
+            copy_commit();
+        };
+        static_assert(kRowStep == 64 && kReduceThreads == kW2Units * kHid, "copy shape");
+        for (int k = 0; k < kSteps - 1; ++k) fetch(k);
+        float a = 0.0f;
+        for (int k = 0; k < steps; ++k) {
+            copy_wait<kSteps - 2>();
+            __syncthreads();  // step k is here for all, step k - 1 read by all
+            fetch(k + kSteps - 1);
+            const W2Step& c = st[k % kSteps];
+            const int rows = n - k * kRowStep < kRowStep ? n - k * kRowStep : kRowStep;
+            if (rows == kRowStep) {
+#pragma unroll 16
+                for (int r = 0; r < kRowStep; ++r) a = fmaf(c.d2[ii][r], c.h1[r][j], a);
+            } else {
+                for (int r = 0; r < rows; ++r) a = fmaf(c.d2[ii][r], c.h1[r][j], a);
+            }
+        }
+        s.p_w2[(int64_t)q * kHid * kHid + (i0 + ii) * kHid + j] = a;
+        return;
+    }
+    SmallTile* st = reinterpret_cast<SmallTile*>(smem_raw);
+    const int i0 = g * kSmallUnits;
+    const int64_t u0 = ((int64_t)q * kHid + i0) * s.rows;
+    auto fetch = [&](int k) {
+        if (k < steps) {
+            SmallTile& c = st[k % kSteps];
+            const int64_t r0 = (int64_t)k * kRowStep;
+            if (t < kSmallUnits * kRowStep / 4) {
+                const int u = t / 16, r = 4 * (t % 16);
+                copy16(&c.dh1[u][r], s.dh1 + u0 + (int64_t)u * s.rows + r0 + r);
+                copy16(&c.dh2[u][r], s.dh2 + u0 + (int64_t)u * s.rows + r0 + r);
+                copy16(&c.h2[u][r], s.h2 + u0 + (int64_t)u * s.rows + r0 + r);
+                copy16(&c.xb[0][0] + 4 * t, s.xb + ((int64_t)q * s.rows + r0) * kFeat + 4 * t);
+            }
+            if (t < kRowStep / 4) copy16(&c.dy[4 * t], s.dy + (int64_t)q * s.rows + r0 + 4 * t);
+        }
+        copy_commit();
+    };
+    static_assert(kRowStep * kFeat == kSmallUnits * kRowStep, "copy shape");
+    for (int k = 0; k < kSteps - 1; ++k) fetch(k);
+    // dW1: unit t / 32, part v = (t / 4) % 8 (rows v, v + 8, ...), features
+    // t % 4 and t % 4 + 4.  Biases and W3: 3 x 8 units x 16 parts, two per
+    // thread (t and t + 256); b3: 16 more parts, in unit group 0.
+    const int wu = t >> 5, wv = (t >> 2) & 7, wk = t & 3;
+    float a0 = 0.0f, a1 = 0.0f, c0 = 0.0f, c1 = 0.0f;
+    const int e1 = t + kReduceThreads;
+    const int kind0 = t / 128, unit0 = (t >> 4) & 7, v0 = t & 15;
+    const int kind1 = e1 / 128, unit1 = (e1 >> 4) & 7, v1 = e1 & 15;  // kind 2: dW3, 3: db3 (e1 >= 384)
+    for (int k = 0; k < steps; ++k) {
+        copy_wait<kSteps - 2>();
+        __syncthreads();
+        fetch(k + kSteps - 1);
+        const SmallTile& c = st[k % kSteps];
+        const int rows = n - k * kRowStep < kRowStep ? n - k * kRowStep : kRowStep;
+        for (int r = wv; r < rows; r += 8) {
+            const float d = c.dh1[wu][r];
+            a0 = fmaf(d, c.xb[r][wk], a0);
+            a1 = fmaf(d, c.xb[r][wk + 4], a1);
+        }
+        for (int r = v0; r < rows; r += 16) c0 += kind0 ? c.dh2[unit0][r] : c.dh1[unit0][r];
+        if (kind1 == 2) {
+            for (int r = v1; r < rows; r += 16) c1 = fmaf(c.dy[r], c.h2[unit1][r], c1);
+        } else if (g == 0 && e1 < 400) {
+            for (int r = v1; r < rows; r += 16) c1 += c.dy[r];
+        }
+    }
+    // part u = b mod 32 (or 64) is row set q, rows v modulo 8 (or 16)
+    float* pw = s.p_w1 + (int64_t)(q + 4 * wv) * kHid * kFeat + (i0 + wu) * kFeat;
+    pw[wk] = a0;
+    pw[wk + 4] = a1;
+    s.p_b[(q + 4 * v0) * kBiasParts + kind0 * kHid + i0 + unit0] = c0;
+    if (kind1 == 2) s.p_b[(q + 4 * v1) * kBiasParts + 2 * kHid + i0 + unit1] = c1;
+    else if (g == 0 && e1 < 400) s.p_b[(q + 4 * v1) * kBiasParts + 3 * kHid] = c1;
+}
+
+// Parameter k's gradient from the partial sums, added in part order.
+__device__ __forceinline__ float grad_of(const Scratch& s, int k)
+{
+    if (k >= kOffW2 && k < kOffB2) {
+        const float* p = s.p_w2 + (k - kOffW2);
+        constexpr int n = kHid * kHid;
+        return (p[0] + p[n]) + (p[2 * n] + p[3 * n]);
+    }
+    const float* p;
+    int parts, stride;
+    if (k < kOffB1) {
+        p = s.p_w1 + k; parts = 32; stride = kHid * kFeat;
+    } else {
+        const int e = k < kOffW2 ? k - kOffB1 : kHid + (k - kOffB2);
+        p = s.p_b + e; parts = 64; stride = kBiasParts;
+    }
+    float r = 0.0f;
+#pragma unroll 16
+    for (int u = 0; u < parts; ++u) r += p[u * stride];
+    return r;
+}
+
+// The batch's loss from the per-32-sample sums, in groups of four; the running
+// sum over an epoch in loss_out[1].
+__device__ __forceinline__ void sum_loss(const Scratch& s, int B, float inv_b, float* loss_out)
+{
+    const int np = (B + kFbSamples - 1) / kFbSamples;
+    float l = 0.0f;
+    for (int u = 0; u < np; u += 4) {
+        float t = 0.0f;
+        for (int k = u; k < u + 4 && k < np; ++k) t += s.loss_part[k];
+        l += t;
+    }
+    loss_out[0] = l * inv_b;
+    loss_out[1] += l * inv_b;
+}
+
+__global__ void grad_kernel(int B, float inv_b, Scratch s, float* __restrict__ g, float* __restrict__ loss_out)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < kParams) g[k] = grad_of(s, k);
+    if (k == kParams) sum_loss(s, B, inv_b, loss_out);
+}
+
+__global__ void adam_kernel(int B, float inv_b, Scratch s, float* __restrict__ P, float* __restrict__ m,
+                            float* __restrict__ v, float lr, float b1, float b2, float c1, float c2, float eps,
+                            float* __restrict__ loss_out)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == kParams) sum_loss(s, B, inv_b, loss_out);
     if (k >= kParams) return;
-    const float gk = g[k];
+    const float gk = grad_of(s, k);
     const float mk = b1 * m[k] + (1.0f - b1) * gk;
     const float vk = b2 * v[k] + (1.0f - b2) * gk * gk;
     m[k] = mk;
@@ -195,26 +381,40 @@ struct DevBuf {
 
 bool alloc_scratch(DevBuf& d, int B, Scratch& s)
 {
-    s.xb = d.alloc<float>((size_t)B * kFeat);
-    s.h1b = d.alloc<float>((size_t)B * kHid);
-    s.h2b = d.alloc<float>((size_t)B * kHid);
-    s.dh1 = d.alloc<float>((size_t)B * kHid);
-    s.dh2 = d.alloc<float>((size_t)B * kHid);
-    s.dy = d.alloc<float>(B);
-    s.loss_part = d.alloc<float>((B + kFbThreads - 1) / kFbThreads);
-    return s.xb && s.h1b && s.h2b && s.dh1 && s.dh2 && s.dy && s.loss_part;
+    s.rows = ((B + 3) / 4 + kRowStep - 1) / kRowStep * kRowStep;
+    const size_t r = 4 * (size_t)s.rows;
+    // One allocation: the arrays above, each a multiple of 64 floats.
+    const size_t len[] = {r * kHid, r * kFeat, r * kHid, r * kHid, r * kHid, r, (size_t)(B / kFbSamples + 64),
+                          (size_t)4 * kHid * kHid, (size_t)32 * kHid * kFeat, (size_t)64 * kBiasParts};
+    float** to[] = {&s.h1, &s.xb, &s.dh1, &s.dh2, &s.h2, &s.dy, &s.loss_part, &s.p_w2, &s.p_w1, &s.p_b};
+    size_t total = 0;
+    for (size_t n : len) total += (n + 63) / 64 * 64;
+    float* p = d.alloc<float>(total);
+    if (!p) return false;
+    for (int k = 0; k < 10; ++k) {
+        *to[k] = p;
+        p += (len[k] + 63) / 64 * 64;
+    }
+    return true;
 }
 
+// Forward, backward and the gradient's partial sums of one batch.
 int fwd_bwd(const float* X, const float* T, const int32_t* idx, int64_t off, int B, const float* P, Scratch& s,
-            float* g, float* loss, cudaStream_t st)
+            cudaStream_t st)
 {
-    const int blocks = (B + kFbThreads - 1) / kFbThreads;
-    mlp_fwd_bwd_kernel<<<blocks, kFbThreads, 0, st>>>(X, T, idx, off, B, 1.0f / (float)B, P, s);
+    BH_CUDA_TRY(cudaFuncSetAttribute(mlp_fwd_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(FbSmem)));
+    BH_CUDA_TRY(cudaFuncSetAttribute(mlp_grad_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kReduceSmem));
+    mlp_fwd_bwd_kernel<<<(B + kFbSamples - 1) / kFbSamples, kFbThreads, sizeof(FbSmem), st>>>(X, T, idx, off, B,
+                                                                                           1.0f / (float)B, P, s);
     BH_CUDA_TRY(cudaGetLastError());
-    mlp_grad_reduce_kernel<<<kHid, 256, 0, st>>>(B, blocks, s, g, loss, 1.0f / (float)B);
+    mlp_grad_reduce_kernel<<<kW2Blocks + kSmallBlocks, kReduceThreads, kReduceSmem, st>>>(B, s);
     BH_CUDA_TRY(cudaGetLastError());
     return BH_OK;
 }
+
+constexpr int kParamBlocks = kParams / 256 + 1;  // one thread past the parameters sums the loss
 
 }  // namespace
 }  // namespace bh
@@ -243,8 +443,10 @@ extern "C" int bh_mlp_gradient(const float* params, const float* X, const float*
     BH_CUDA_TRY(cudaMemcpy(dP, params, sizeof(float) * kParams, cudaMemcpyHostToDevice));
     BH_CUDA_TRY(cudaMemcpy(dX, X, sizeof(float) * n * kFeat, cudaMemcpyHostToDevice));
     BH_CUDA_TRY(cudaMemcpy(dT, T, sizeof(float) * n, cudaMemcpyHostToDevice));
-    int rc = fwd_bwd(dX, dT, nullptr, 0, (int)n, dP, s, dG, dL, 0);
+    int rc = fwd_bwd(dX, dT, nullptr, 0, (int)n, dP, s, 0);
     if (rc) return rc;
+    grad_kernel<<<kParamBlocks, 256>>>((int)n, 1.0f / (float)n, s, dG, dL);
+    BH_CUDA_TRY(cudaGetLastError());
     BH_CUDA_TRY(cudaMemcpy(grad_out, dG, sizeof(float) * kParams, cudaMemcpyDeviceToHost));
     if (loss_out) BH_CUDA_TRY(cudaMemcpy(loss_out, dL, sizeof(float), cudaMemcpyDeviceToHost));
     return BH_OK;
@@ -302,7 +504,6 @@ extern "C" int bh_mlp_train(const float* features, const float* labels, int64_t 
 
     DevBuf d;
     float* dP = d.alloc<float>(kParams);
-    float* dG = d.alloc<float>(kParams);
     float* dM = d.alloc<float>(kParams);
     float* dV = d.alloc<float>(kParams);
     float* dX = d.alloc<float>((size_t)n * kFeat);
@@ -311,7 +512,7 @@ extern "C" int bh_mlp_train(const float* features, const float* labels, int64_t 
     float* dL = d.alloc<float>(2);
     Scratch s;
     const int B = (int)std::min<int64_t>(batch, n);
-    if (!dP || !dG || !dM || !dV || !dX || !dT || !dI || !dL || !alloc_scratch(d, B, s))
+    if (!dP || !dM || !dV || !dX || !dT || !dI || !dL || !alloc_scratch(d, B, s))
         return bh_fail(BH_ERR_OUT_OF_MEMORY, "bh_mlp_train: device allocation failed");
     BH_CUDA_TRY(cudaMemcpy(dP, P.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice));
     BH_CUDA_TRY(cudaMemset(dM, 0, sizeof(float) * kParams));
@@ -328,12 +529,12 @@ extern "C" int bh_mlp_train(const float* features, const float* labels, int64_t 
         BH_CUDA_TRY(cudaMemcpy(dI, order.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
         BH_CUDA_TRY(cudaMemset(dL, 0, 2 * sizeof(float)));
         for (int64_t k = 0; k < nb; ++k) {
-            int rc = fwd_bwd(dX, dT, dI, k * B, B, dP, s, dG, dL, 0);
+            int rc = fwd_bwd(dX, dT, dI, k * B, B, dP, s, 0);
             if (rc) return rc;
             ++step;
             const float c1 = 1.0f / (1.0f - std::pow(b1, (float)step));
             const float c2 = 1.0f / (1.0f - std::pow(b2, (float)step));
-            adam_kernel<<<(kParams + 255) / 256, 256>>>(dP, dG, dM, dV, lr, b1, b2, c1, c2, eps);
+            adam_kernel<<<kParamBlocks, 256>>>(B, 1.0f / (float)B, s, dP, dM, dV, lr, b1, b2, c1, c2, eps, dL);
             BH_CUDA_TRY(cudaGetLastError());
         }
         float l[2] = {0.f, 0.f};
