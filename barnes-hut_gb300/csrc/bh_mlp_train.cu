@@ -41,9 +41,10 @@ struct Scratch {
 };
 constexpr int kBiasParts = 3 * kHid + 1;
 
+constexpr int kW2tRow = kHid + 4;
 struct FbSmem {
     float W2[kHid * kHid];   // [i][j]
-    float W2t[kHid * kHid];  // [j][i]
+    float W2t[kHid * kW2tRow];  // [j][i], rows padded against bank conflicts
     float h1[kHid][kFbSamples];
     float h2[kHid][kFbSamples];
     float d2[kHid][kFbSamples];
@@ -55,8 +56,9 @@ struct FbSmem {
 // warp w computes units 8 w .. 8 w + 7 of each layer, so that eight independent
 // sums run beside one another and every weight is read by broadcast.  Each sum
 // keeps the order of its terms.  What bounds it is latency (a block's 32
-// samples are a chain of three small layers); one thread per sample, 32 blocks
-// of 128 on the whole chip, took 58 us for a batch of 4,096.
+// samples are a chain of three small layers); with one thread per sample, 32
+// blocks of 128 on the whole chip, a batch of 4,096 took 135 us over its three
+// kernels, and takes 30 (in ncu 11 here, 12 in the sums, 6 in Adam).
 __global__ void __launch_bounds__(kFbThreads) mlp_fwd_bwd_kernel(const float* __restrict__ X,
                                                                 const float* __restrict__ T,
                                                                 const int32_t* __restrict__ idx, int64_t off,
@@ -66,10 +68,17 @@ __global__ void __launch_bounds__(kFbThreads) mlp_fwd_bwd_kernel(const float* __
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FbSmem& m = *reinterpret_cast<FbSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, u0 = 8 * w;
-    for (int k = threadIdx.x; k < kHid * kHid; k += kFbThreads) {
-        const float v = bf16r(P[kOffW2 + k]);
-        m.W2[k] = v;
-        m.W2t[(k % kHid) * kHid + k / kHid] = v;
+    static_assert(kOffW2 % 4 == 0, "rows of W2 are read as float4");
+#pragma unroll
+    for (int q = 0; q < kHid * kHid / 4 / kFbThreads; ++q) {
+        const int k = 4 * (threadIdx.x + q * kFbThreads), i = k / kHid, j = k % kHid;
+        float4 v = *reinterpret_cast<const float4*>(P + kOffW2 + k);
+        v.x = bf16r(v.x); v.y = bf16r(v.y); v.z = bf16r(v.z); v.w = bf16r(v.w);
+        *reinterpret_cast<float4*>(&m.W2[k]) = v;
+        m.W2t[j * kW2tRow + i] = v.x;
+        m.W2t[(j + 1) * kW2tRow + i] = v.y;
+        m.W2t[(j + 2) * kW2tRow + i] = v.z;
+        m.W2t[(j + 3) * kW2tRow + i] = v.w;
     }
     for (int k = threadIdx.x; k < kHid * kFeat; k += kFbThreads) m.W1[k] = bf16r(P[kOffW1 + k]);
     if (threadIdx.x < kHid) {
@@ -102,8 +111,8 @@ __global__ void __launch_bounds__(kFbThreads) mlp_fwd_bwd_kernel(const float* __
 #pragma unroll 8
     for (int j = 0; j < kHid; ++j) {
         const float h = m.h1[j][lane];
-        const float4 v0 = *reinterpret_cast<const float4*>(&m.W2t[j * kHid + u0]);
-        const float4 v1 = *reinterpret_cast<const float4*>(&m.W2t[j * kHid + u0 + 4]);
+        const float4 v0 = *reinterpret_cast<const float4*>(&m.W2t[j * kW2tRow + u0]);
+        const float4 v1 = *reinterpret_cast<const float4*>(&m.W2t[j * kW2tRow + u0 + 4]);
         acc[0] = fmaf(v0.x, h, acc[0]); acc[1] = fmaf(v0.y, h, acc[1]);
         acc[2] = fmaf(v0.z, h, acc[2]); acc[3] = fmaf(v0.w, h, acc[3]);
         acc[4] = fmaf(v1.x, h, acc[4]); acc[5] = fmaf(v1.y, h, acc[5]);
@@ -183,8 +192,7 @@ __device__ __forceinline__ void copy_wait()
 // FMAs, four cycles each, which is what bounds it (a batch of 4,096: 4,096
 // cycles, 2.1 us), while the rows stream through shared memory four steps
 // ahead.  Blocks 64..95: the sums over 32 (dW1) and 64 (biases, W3) interleaved
-// parts for eight units and one row set.  Reading the rows from L2 as they were
-// needed, 64 blocks took 75 us for a batch of 4,096.
+// parts for eight units and one row set.
 constexpr int kReduceThreads = 256;
 constexpr int kW2Units = 4;                       // units per block
 constexpr int kW2Blocks = 4 * kHid / kW2Units;    // 64
@@ -304,6 +312,10 @@ __global__ void __launch_bounds__(kReduceThreads) mlp_grad_reduce_kernel(int B, 
     else if (g == 0 && e1 < 400) s.p_b[(q + 4 * v1) * kBiasParts + 3 * kHid] = c1;
 }
 
+// One more block than these sums the loss.
+constexpr int kParamThreads = 128;
+constexpr int kParamBlocks = (kParams + kParamThreads - 1) / kParamThreads;
+
 // Parameter k's gradient from the partial sums, added in part order.
 __device__ __forceinline__ float grad_of(const Scratch& s, int k)
 {
@@ -326,34 +338,48 @@ __device__ __forceinline__ float grad_of(const Scratch& s, int k)
     return r;
 }
 
-// The batch's loss from the per-32-sample sums, in groups of four; the running
-// sum over an epoch in loss_out[1].
+// The batch's loss from the per-32-sample sums, by one warp: groups of four,
+// one per lane, added in order; the running sum over an epoch in loss_out[1].
 __device__ __forceinline__ void sum_loss(const Scratch& s, int B, float inv_b, float* loss_out)
 {
+    const int lane = threadIdx.x & 31;
     const int np = (B + kFbSamples - 1) / kFbSamples;
     float l = 0.0f;
-    for (int u = 0; u < np; u += 4) {
+    for (int u0 = 0; u0 < np; u0 += 128) {
         float t = 0.0f;
-        for (int k = u; k < u + 4 && k < np; ++k) t += s.loss_part[k];
-        l += t;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int u = u0 + 4 * lane + k;
+            t += u < np ? s.loss_part[u] : 0.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < 32; ++k) l += __shfl_sync(0xffffffffu, t, k);  // past the end: + 0
     }
-    loss_out[0] = l * inv_b;
-    loss_out[1] += l * inv_b;
+    if (lane == 0) {
+        loss_out[0] = l * inv_b;
+        loss_out[1] += l * inv_b;
+    }
 }
 
 __global__ void grad_kernel(int B, float inv_b, Scratch s, float* __restrict__ g, float* __restrict__ loss_out)
 {
+    if (blockIdx.x == kParamBlocks) {
+        if (threadIdx.x < 32) sum_loss(s, B, inv_b, loss_out);
+        return;
+    }
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < kParams) g[k] = grad_of(s, k);
-    if (k == kParams) sum_loss(s, B, inv_b, loss_out);
 }
 
 __global__ void adam_kernel(int B, float inv_b, Scratch s, float* __restrict__ P, float* __restrict__ m,
                             float* __restrict__ v, float lr, float b1, float b2, float c1, float c2, float eps,
                             float* __restrict__ loss_out)
 {
+    if (blockIdx.x == kParamBlocks) {
+        if (threadIdx.x < 32) sum_loss(s, B, inv_b, loss_out);
+        return;
+    }
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == kParams) sum_loss(s, B, inv_b, loss_out);
     if (k >= kParams) return;
     const float gk = grad_of(s, k);
     const float mk = b1 * m[k] + (1.0f - b1) * gk;
@@ -361,6 +387,117 @@ __global__ void adam_kernel(int B, float inv_b, Scratch s, float* __restrict__ P
     m[k] = mk;
     v[k] = vk;
     P[k] -= lr * (mk * c1) / (sqrtf(vk * c2) + eps);
+}
+
+// Standardisation of the features and labels (FP64 sums, as the scaling's
+// definition; one thread per feature and row class, columns 8 = the label).
+constexpr int kStdBlocks = 128, kStdThreads = 288;  // 32 rows x 9 columns
+struct StdScratch {
+    double sum[kStdBlocks][9], sq[kStdBlocks][9];
+    float lo[kStdBlocks][kFeat], hi[kStdBlocks][kFeat];
+    MlpScale sc;
+    float loss[2];
+};
+
+__global__ void __launch_bounds__(kStdThreads) std_sum_kernel(int64_t n, const float* __restrict__ X,
+                                                             const float* __restrict__ T, StdScratch* s)
+{
+    __shared__ double ps[kStdThreads], pq[kStdThreads];
+    const int c = threadIdx.x % 9, r = threadIdx.x / 9;
+    double a = 0.0, q = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * 32 + r; i < n; i += 32 * kStdBlocks) {
+        const double v = c < kFeat ? X[i * kFeat + c] : T[i];
+        a += v;
+        q += v * v;
+    }
+    ps[threadIdx.x] = a;
+    pq[threadIdx.x] = q;
+    __syncthreads();
+    if (threadIdx.x < 9) {
+        for (int k = 1; k < 32; ++k) {
+            a += ps[9 * k + c];
+            q += pq[9 * k + c];
+        }
+        s->sum[blockIdx.x][c] = a;
+        s->sq[blockIdx.x][c] = q;
+    }
+}
+
+// Warp c: column c.
+__global__ void __launch_bounds__(kStdThreads) std_scale_kernel(int64_t n, StdScratch* s)
+{
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double a = 0.0, q = 0.0;
+#pragma unroll
+    for (int k = lane; k < kStdBlocks; k += 32) {
+        a += s->sum[k][c];
+        q += s->sq[k][c];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, off);
+        q += __shfl_xor_sync(0xffffffffu, q, off);
+    }
+    if (lane > 0) return;
+    const double mu = a / n, v = q / n - mu * mu, var = v < 1e-12 ? 1e-12 : v;
+    if (c < kFeat) {
+        s->sc.mean[c] = (float)mu;
+        s->sc.inv_std[c] = (float)(1.0 / sqrt(var));
+    } else {
+        s->sc.lmean = (float)mu;
+        s->sc.lstd = (float)sqrt(var);
+    }
+}
+
+__global__ void __launch_bounds__(kStdThreads) std_apply_kernel(int64_t n, float* __restrict__ X, float* __restrict__ T,
+                                                               StdScratch* s)
+{
+    __shared__ float pl[kStdThreads], ph[kStdThreads];
+    const int c = threadIdx.x % 9, r = threadIdx.x / 9;
+    const float mean = c < kFeat ? s->sc.mean[c] : s->sc.lmean, inv = c < kFeat ? s->sc.inv_std[c] : 0.0f;
+    const float lstd = s->sc.lstd;
+    float lo = 1e30f, hi = -1e30f;
+    for (int64_t i = (int64_t)blockIdx.x * 32 + r; i < n; i += 32 * kStdBlocks) {
+        if (c < kFeat) {
+            const float z = (X[i * kFeat + c] - mean) * inv;
+            X[i * kFeat + c] = z;
+            lo = z < lo ? z : lo;
+            hi = hi < z ? z : hi;
+        } else {
+            T[i] = __fdiv_rn(T[i] - mean, lstd);
+        }
+    }
+    pl[threadIdx.x] = lo;
+    ph[threadIdx.x] = hi;
+    __syncthreads();
+    if (threadIdx.x < kFeat) {
+        for (int k = 1; k < 32; ++k) {
+            lo = fminf(lo, pl[9 * k + c]);
+            hi = fmaxf(hi, ph[9 * k + c]);
+        }
+        s->lo[blockIdx.x][c] = lo;
+        s->hi[blockIdx.x][c] = hi;
+    }
+}
+
+__global__ void __launch_bounds__(32 * kFeat) std_range_kernel(StdScratch* s)
+{
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float lo = 1e30f, hi = -1e30f;
+#pragma unroll
+    for (int k = lane; k < kStdBlocks; k += 32) {
+        lo = fminf(lo, s->lo[k][c]);
+        hi = fmaxf(hi, s->hi[k][c]);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+    }
+    if (lane == 0) {
+        s->sc.lo[c] = lo;
+        s->sc.hi[c] = hi;
+    }
 }
 
 struct DevBuf {
@@ -414,8 +551,6 @@ int fwd_bwd(const float* X, const float* T, const int32_t* idx, int64_t off, int
     return BH_OK;
 }
 
-constexpr int kParamBlocks = kParams / 256 + 1;  // one thread past the parameters sums the loss
-
 }  // namespace
 }  // namespace bh
 
@@ -445,7 +580,7 @@ extern "C" int bh_mlp_gradient(const float* params, const float* X, const float*
     BH_CUDA_TRY(cudaMemcpy(dT, T, sizeof(float) * n, cudaMemcpyHostToDevice));
     int rc = fwd_bwd(dX, dT, nullptr, 0, (int)n, dP, s, 0);
     if (rc) return rc;
-    grad_kernel<<<kParamBlocks, 256>>>((int)n, 1.0f / (float)n, s, dG, dL);
+    grad_kernel<<<kParamBlocks + 1, kParamThreads>>>((int)n, 1.0f / (float)n, s, dG, dL);
     BH_CUDA_TRY(cudaGetLastError());
     BH_CUDA_TRY(cudaMemcpy(grad_out, dG, sizeof(float) * kParams, cudaMemcpyDeviceToHost));
     if (loss_out) BH_CUDA_TRY(cudaMemcpy(loss_out, dL, sizeof(float), cudaMemcpyDeviceToHost));
@@ -463,37 +598,6 @@ extern "C" int bh_mlp_train(const float* features, const float* labels, int64_t 
         cudaGetLastError();
         return bh_fail(BH_ERR_NO_DEVICE, "bh_mlp_train: no CUDA device");
     }
-    // Standardisation from the data (host, FP64 sums).
-    MlpScale sc;
-    double mean[kFeat] = {0}, sq[kFeat] = {0}, lm = 0, ls = 0;
-    for (int64_t r = 0; r < n; ++r) {
-        for (int k = 0; k < kFeat; ++k) {
-            const double v = features[r * kFeat + k];
-            mean[k] += v;
-            sq[k] += v * v;
-        }
-        lm += labels[r];
-        ls += (double)labels[r] * labels[r];
-    }
-    for (int k = 0; k < kFeat; ++k) {
-        const double mu = mean[k] / n, var = std::max(sq[k] / n - mu * mu, 1e-12);
-        sc.mean[k] = (float)mu;
-        sc.inv_std[k] = (float)(1.0 / std::sqrt(var));
-        sc.lo[k] = 1e30f;
-        sc.hi[k] = -1e30f;
-    }
-    sc.lmean = (float)(lm / n);
-    sc.lstd = (float)std::sqrt(std::max(ls / n - (lm / n) * (lm / n), 1e-12));
-    std::vector<float> Z((size_t)n * kFeat), TL(n);
-    for (int64_t r = 0; r < n; ++r) {
-        for (int k = 0; k < kFeat; ++k) {
-            const float z = (features[r * kFeat + k] - sc.mean[k]) * sc.inv_std[k];
-            Z[r * kFeat + k] = z;
-            sc.lo[k] = std::min(sc.lo[k], z);
-            sc.hi[k] = std::max(sc.hi[k], z);
-        }
-        TL[r] = (labels[r] - sc.lmean) / sc.lstd;
-    }
     // He-normal initialisation, zero biases.
     std::mt19937_64 rng(seed);
     std::normal_distribution<double> nd(0.0, 1.0);
@@ -503,29 +607,38 @@ extern "C" int bh_mlp_train(const float* features, const float* labels, int64_t 
     for (int k = 0; k < kHid; ++k) P[kOffW3 + k] = (float)(nd(rng) * std::sqrt(1.0 / kHid));
 
     DevBuf d;
-    float* dP = d.alloc<float>(kParams);
-    float* dM = d.alloc<float>(kParams);
-    float* dV = d.alloc<float>(kParams);
-    float* dX = d.alloc<float>((size_t)n * kFeat);
-    float* dT = d.alloc<float>(n);
-    int32_t* dI = d.alloc<int32_t>(n);
-    float* dL = d.alloc<float>(2);
+    float* dP = d.alloc<float>(3 * kParams);  // parameters and the two moments
+    float* dM = dP + kParams;
+    float* dV = dM + kParams;
+    float* dX = d.alloc<float>((size_t)n * (kFeat + 2));  // features, labels, order
+    float* dT = dX + (size_t)n * kFeat;
+    int32_t* dI = reinterpret_cast<int32_t*>(dT + n);
+    StdScratch* dS = d.alloc<StdScratch>(1);
     Scratch s;
     const int B = (int)std::min<int64_t>(batch, n);
-    if (!dP || !dM || !dV || !dX || !dT || !dI || !dL || !alloc_scratch(d, B, s))
+    if (!dP || !dX || !dS || !alloc_scratch(d, B, s))
         return bh_fail(BH_ERR_OUT_OF_MEMORY, "bh_mlp_train: device allocation failed");
+    float* dL = dS->loss;
     BH_CUDA_TRY(cudaMemcpy(dP, P.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice));
-    BH_CUDA_TRY(cudaMemset(dM, 0, sizeof(float) * kParams));
-    BH_CUDA_TRY(cudaMemset(dV, 0, sizeof(float) * kParams));
-    BH_CUDA_TRY(cudaMemcpy(dX, Z.data(), sizeof(float) * n * kFeat, cudaMemcpyHostToDevice));
-    BH_CUDA_TRY(cudaMemcpy(dT, TL.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
+    BH_CUDA_TRY(cudaMemsetAsync(dM, 0, sizeof(float) * 2 * kParams));
+    BH_CUDA_TRY(cudaMemcpy(dX, features, sizeof(float) * n * kFeat, cudaMemcpyHostToDevice));
+    BH_CUDA_TRY(cudaMemcpy(dT, labels, sizeof(float) * n, cudaMemcpyHostToDevice));
+    // Standardisation in place.
+    std_sum_kernel<<<kStdBlocks, kStdThreads>>>(n, dX, dT, dS);
+    BH_CUDA_TRY(cudaGetLastError());
+    std_scale_kernel<<<1, kStdThreads>>>(n, dS);
+    BH_CUDA_TRY(cudaGetLastError());
+    std_apply_kernel<<<kStdBlocks, kStdThreads>>>(n, dX, dT, dS);
+    BH_CUDA_TRY(cudaGetLastError());
+    std_range_kernel<<<1, 32 * kFeat>>>(dS);
+    BH_CUDA_TRY(cudaGetLastError());
     std::vector<int32_t> order(n);
     std::iota(order.begin(), order.end(), 0);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     int64_t step = 0;
     const int64_t nb = n / B;  // full batches only
+    std::shuffle(order.begin(), order.end(), rng);
     for (int e = 0; e < epochs; ++e) {
-        std::shuffle(order.begin(), order.end(), rng);
         BH_CUDA_TRY(cudaMemcpy(dI, order.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
         BH_CUDA_TRY(cudaMemset(dL, 0, 2 * sizeof(float)));
         for (int64_t k = 0; k < nb; ++k) {
@@ -534,14 +647,16 @@ extern "C" int bh_mlp_train(const float* features, const float* labels, int64_t 
             ++step;
             const float c1 = 1.0f / (1.0f - std::pow(b1, (float)step));
             const float c2 = 1.0f / (1.0f - std::pow(b2, (float)step));
-            adam_kernel<<<kParamBlocks, 256>>>(B, 1.0f / (float)B, s, dP, dM, dV, lr, b1, b2, c1, c2, eps, dL);
+            adam_kernel<<<kParamBlocks + 1, kParamThreads>>>(B, 1.0f / (float)B, s, dP, dM, dV, lr, b1, b2, c1, c2, eps, dL);
             BH_CUDA_TRY(cudaGetLastError());
         }
+        // the next epoch's order, while the device works on this one
+        if (e + 1 < epochs) std::shuffle(order.begin(), order.end(), rng);
         float l[2] = {0.f, 0.f};
         BH_CUDA_TRY(cudaMemcpy(l, dL, 2 * sizeof(float), cudaMemcpyDeviceToHost));
         if (loss_out) loss_out[e] = l[1] / (float)std::max<int64_t>(nb, 1);  // mean batch loss of the epoch
     }
     BH_CUDA_TRY(cudaMemcpy(params_out, dP, sizeof(float) * kParams, cudaMemcpyDeviceToHost));
-    std::memcpy(scale_out, &sc, sizeof(MlpScale));
+    BH_CUDA_TRY(cudaMemcpy(scale_out, &dS->sc, sizeof(MlpScale), cudaMemcpyDeviceToHost));
     return BH_OK;
 }
