@@ -115,12 +115,10 @@ void layout(bh_context* ctx, Carver& c)
     ctx->node_s = c.take<double4_32a>(n);
     ctx->slot_ref = c.take<int32_t>(2 * n);
     ctx->slot_top = c.take<uint8_t>(2 * n);
-    ctx->depth_off = c.take<int32_t>(32);
-    ctx->depth_nodes = c.take<int32_t>(n);
+    ctx->mono_span = c.take<int32_t>(bh::monopole_ints(n));
     ctx->rec = c.take<bh::TreeRec>(2 * n);
     ctx->counts = c.take<int32_t>(16);
-    const int64_t nblk = (n + 1023) / 1024;
-    ctx->scan_tmp = c.take<int32_t>(std::max<int64_t>(bh::scan_tmp_ints(2 * n), 21 * nblk + 64));
+    ctx->scan_tmp = c.take<int32_t>(bh::scan_tmp_ints(2 * n));
     ctx->inter_count = c.take<unsigned long long>(1);
     ctx->body_count = c.take<int32_t>(n);
     ctx->fA = c.take<float4>(2 * n);

@@ -378,8 +378,7 @@ struct bh_context {
     double4_32a* node_s = nullptr;  // branching-node sums {m x, m y, m z, m}
     int32_t* slot_ref = nullptr;    // >= 0 leaf id, < 0 ~node id
     uint8_t* slot_top = nullptr;
-    int32_t* depth_off = nullptr;   // 23 offsets into depth_nodes (by depth)
-    int32_t* depth_nodes = nullptr; // node ids bucketed by depth
+    int32_t* mono_span = nullptr;   // nodes the stages of the monopole pass leave over
     bh::TreeRec* rec = nullptr;     // traversal records, slot 0 = root
     int32_t* counts = nullptr;      // device scalars: [0]=L, [1]=B, [2]=slots
     int32_t* scan_tmp = nullptr;    // block sums of the device scans
@@ -464,6 +463,8 @@ int64_t scan_tmp_ints(int64_t n_max);
 // Ints of the per-block summaries of the tree build's boundary pass for up
 // to n bodies.
 int64_t boundary_pass_ints(int64_t n);
+// Ints of the monopole pass's lists of nodes left over.
+int64_t monopole_ints(int64_t n);
 int launch_sort(bh_context* ctx);
 int launch_permute(bh_context* ctx);
 // The permutation gathers into the second body set; the two sets then trade

@@ -29,6 +29,7 @@
 // double intrinsics (no contraction), so masses and centres of mass are bit
 // for bit the reference's.
 #include <climits>
+#include <utility>
 
 #include "bh_internal.cuh"
 
@@ -408,10 +409,29 @@ __global__ void node_place_kernel(const int32_t* __restrict__ counts, const int8
     }
 }
 
-// One node's sums from its children, in slot (= octant) order from 0.0
-// (linear_octree.cpp:69-87), and with kMoments the second moment by the
-// parallel-axis rule (see below).  The children's sums were written by the
-// previous level's launch; loads bypass L1.
+// ---- Monopole pass ------------------------------------------------------
+// Every branching node's sums from its children's, in slot (= octant) order
+// from 0.0 (linear_octree.cpp:69-87), deepest level first.  A block takes
+// kChunk consecutive leaves and all the nodes inside them: it sorts those by
+// depth and works up level by level in shared memory, with a block barrier
+// between levels.  The nodes that reach past the chunk (at most 21 around each
+// end) are left for the next stage, whose blocks take kFan chunks each, and so
+// on until one block holds the rest.  No atomics on global memory, and two
+// launches up to 32,768 bodies or three up to two million, where one launch
+// per depth took 21, and three more to sort the nodes by depth.  Bound: the
+// FP64 additions (a node has 3.3 children on average) and, in the later
+// stages, their latency.  The whole build, ms: 4,000,000 bodies 0.81 -> 0.73,
+// 1,000,000 with second moments 0.51 -> 0.41, 300,149 0.28 -> 0.18, 19,054
+// 0.20 -> 0.10, 1,000 0.17 -> 0.09.  512 leaves per block: 256 and 1,024 gave
+// the same within 3 %.
+constexpr int kChunk = 512;          // leaves per block of the first stage
+constexpr int kChunkThreads = 256;
+constexpr int kFan = 64;             // groups per block of a later stage
+constexpr int kRestThreads = 512;
+constexpr int kRestItems = 384;      // nodes of a later stage's block with their sums in shared memory
+constexpr int kMaxSpan = 2 * kMaxDepth;  // nodes left over per group
+constexpr int kDepths = kMaxDepth;       // branching depths 0..20
+
 __device__ __forceinline__ double4_32a load_sums(const double4_32a* p)
 {
     const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
@@ -419,158 +439,416 @@ __device__ __forceinline__ double4_32a load_sums(const double4_32a* p)
     return double4_32a{a.x, a.y, b.x, b.y};
 }
 
-// A node has at most 8 children: their slot entries are loaded together,
-// then their sums four at a time, before the additions (independent loads
-// in flight instead of a chain of dependent ones), which still run in slot
-// order.
-template <bool kMoments>
-__device__ void node_sums(int b, const int32_t* __restrict__ node_cs, const int32_t* __restrict__ node_nchild,
-                          const int32_t* __restrict__ slot_ref, const double4_32a* ls, double4_32a* ns,
-                          const double* lq, double* nq)
+// acc + child, the first child's 0.0 + v decided on the bit patterns.
+__device__ __forceinline__ double add_sum(double acc, double v, bool first)
 {
-    const int s0 = node_cs[b] + 1, nc = node_nchild[b];
-    int rr[8];
+    return first ? plus_zero(v) : __dadd_rn(acc, v);
+}
+__device__ __forceinline__ void add_sums(double4_32a& acc, const double4_32a& v, bool first)
+{
+    acc.x = add_sum(acc.x, v.x, first);
+    acc.y = add_sum(acc.y, v.y, first);
+    acc.z = add_sum(acc.z, v.z, first);
+    acc.w = add_sum(acc.w, v.w, first);
+}
+
+// Four consecutive lanes work on a node: one sum each (a dependent FP64
+// addition takes about 100 cycles here, so a level's time is its longest chain;
+// one lane with the four sums takes up to four times as long).  The second
+// moment's terms are formed four children at a time and added by each lane.
+__device__ __forceinline__ double quad_get(double v, int j)  // lane j's of the four
+{
+    const int lane = threadIdx.x & 31;
+    return __shfl_sync(0xFu << (lane & 28), v, (lane & 28) + j);
+}
+
+// A node's second moment by the parallel-axis rule, one child's share:
+// m_c |c_c - c|^2 = |w_c - m_c c|^2 / m_c: u = w_c - m_c c by FMA keeps the
+// cancellation in FP64; the division by m_c needs only the feature's precision
+// (an FP32 reciprocal, 2^-22).  Masses are >= 0, so "> 0" is a test on the bit
+// pattern.
+__device__ __forceinline__ double moment_uu(const double4_32a& v, double gx, double gy, double gz)  // |u|^2
+{
+    const double ux = fma(-v.w, gx, v.x), uy = fma(-v.w, gy, v.y), uz = fma(-v.w, gz, v.z);
+    return fma(ux, ux, fma(uy, uy, uz * uz));
+}
+__device__ __forceinline__ double moment_add(double uu, double mass, double cq)
+{
+    if (__double_as_longlong(mass) <= 0) return 0.0;
+    return fma(uu, widen(__frcp_rn(narrow_trunc(mass))), cq);
+}
+__device__ __forceinline__ double moment_share(const double4_32a& v, double cq, double gx, double gy, double gz)
+{
+    return moment_add(moment_uu(v, gx, gy, gz), v.w, cq);
+}
+
+// The order a block takes its nodes in: deepest first, and within a depth by
+// child count, so that the lanes of a warp add equally many children (the FP64
+// pipe takes an addition for one lane as long as for 32).
+constexpr int kBins = 8 * kDepths;
+__device__ __forceinline__ int bin_of(int depth, int nchild) { return 8 * (kDepths - 1 - depth) + (8 - nchild); }
+
+// Exclusive prefix of the bin counts (and the total behind it), by warp 0.
+__device__ __forceinline__ void bin_offsets(const int* cnt, int* off)
+{
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int carry = 0;
+        for (int base = 0; base < kBins; base += 32) {
+            const int v = base + lane < kBins ? cnt[base + lane] : 0;
+            int x = v;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) rr[c] = c < nc ? slot_ref[s0 + c] : 0;
-    double sm = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (base + lane < kBins) off[base + lane] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) off[kBins] = carry;
+    }
+}
+
+template <bool kMoments>
+struct ChunkSmem {
+    double4_32a leaf[kChunk];
+    double4_32a node[kChunk];
+    double uu[kMoments ? 2 * kChunk + 8 * kMaxSpan : 1];  // per child slot
+    int child[2 * kChunk + 8 * kMaxSpan];  // child slots' refs of the chunk's nodes
+    int cs[kChunk + 1];                    // first child of each node in `child`
+    uint16_t order[kChunk];                // local nodes, deepest first
+    int cnt[kBins], pos[kBins], off[kBins + 1];
+    int span;
+};
+
+template <bool kMoments>
+__global__ void __launch_bounds__(kChunkThreads) monopole_chunk_kernel(
+    const int32_t* __restrict__ counts, const int32_t* __restrict__ rep_node, const int32_t* __restrict__ node_a,
+    const int32_t* __restrict__ node_e, const uint8_t* __restrict__ node_depth, const int32_t* __restrict__ node_cs,
+    const int32_t* __restrict__ node_nchild, const int32_t* __restrict__ slot_ref, const double4_32a* __restrict__ ls,
+    double4_32a* __restrict__ ns, const double* __restrict__ lq, double* __restrict__ nq,
+    int32_t* __restrict__ span_cnt, int32_t* __restrict__ span)
+{
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    ChunkSmem<kMoments>& m = *reinterpret_cast<ChunkSmem<kMoments>*>(smem_raw);
+    const int L = counts[0], B = counts[1];
+    const int c0 = blockIdx.x * kChunk, c1 = min(c0 + kChunk, L);
+    if (c0 >= L) {
+        if (threadIdx.x == 0) span_cnt[blockIdx.x] = 0;
+        return;
+    }
+    // The nodes whose first split lies in the chunk (numbered in that order).
+    const int n0 = rep_node[c0], n1 = c1 < L ? rep_node[c1] : B;
+    const int nn = n1 - n0;
+    for (int k = threadIdx.x; k < c1 - c0; k += kChunkThreads) {
+        m.leaf[k] = ls[c0 + k];
+    }
+    for (int k = threadIdx.x; k < kBins; k += kChunkThreads) m.cnt[k] = m.pos[k] = 0;
+    if (threadIdx.x == 0) m.span = 0;
+    __syncthreads();
+    const int s0 = nn > 0 ? node_cs[n0] : 0;
+    int bin[kChunk / kChunkThreads];  // -1: not a node inside the chunk
 #pragma unroll
-    for (int h = 0; h < 8; h += 4) {
-        if (h >= nc) break;
-        double4_32a vv[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            if (h + c < nc) vv[c] = load_sums(rr[h + c] >= 0 ? ls + rr[h + c] : ns + ~rr[h + c]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (h + c < nc) {
-                sm = __dadd_rn(sm, vv[c].w);
-                sx = __dadd_rn(sx, vv[c].x);
-                sy = __dadd_rn(sy, vv[c].y);
-                sz = __dadd_rn(sz, vv[c].z);
+    for (int q = 0; q < kChunk / kChunkThreads; ++q) {
+        const int k = threadIdx.x + q * kChunkThreads;
+        bin[q] = -1;
+        if (k < nn) {
+            const int b = n0 + k, f = node_cs[b], nc = node_nchild[b];
+            m.cs[k] = f - s0;
+            if (k == nn - 1) m.cs[nn] = f - s0 + nc;
+            if (node_a[b] >= c0 && node_e[b] <= c1) {
+                bin[q] = bin_of(node_depth[b], nc);
+                atomicAdd(&m.cnt[bin[q]], 1);
+            } else {
+                const int at = atomicAdd(&m.span, 1);
+                if (at < kMaxSpan) span[(int64_t)blockIdx.x * kMaxSpan + at] = b;
             }
         }
     }
-    ns[b] = double4_32a{sx, sy, sz, sm};
+    __syncthreads();
+    bin_offsets(m.cnt, m.off);
+    if (threadIdx.x == 0) span_cnt[blockIdx.x] = min(m.span, kMaxSpan);
+    const int children = nn > 0 ? m.cs[nn] : 0;
+    for (int k = threadIdx.x; k < children; k += kChunkThreads) m.child[k] = slot_ref[s0 + 1 + k];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kChunk / kChunkThreads; ++q)
+        if (bin[q] >= 0)
+            m.order[m.off[bin[q]] + atomicAdd(&m.pos[bin[q]], 1)] = (uint16_t)(threadIdx.x + q * kChunkThreads);
+    __syncthreads();
+    for (int level = 0; level < kDepths; ++level) {
+        const int lo = m.off[8 * level], hi = m.off[8 * level + 8];
+        if (lo == hi) continue;
+        for (int t = 4 * lo + threadIdx.x; t < 4 * hi; t += kChunkThreads) {
+            const int k = m.order[t >> 2];
+            const int f = m.cs[k], e = m.cs[k + 1];
+            double sum = 0.0;
+            for (int c = f; c < e; ++c) {
+                const int r = m.child[c];
+                sum = add_sum(sum, (r >= 0 ? &m.leaf[r - c0].x : &m.node[~r - n0].x)[t & 3], c == f);
+            }
+            (&m.node[k].x)[t & 3] = sum;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < kChunk / kChunkThreads; ++q) {
+        const int k = threadIdx.x + q * kChunkThreads;
+        if (bin[q] >= 0) ns[n0 + k] = m.node[k];
+    }
     if (kMoments) {
-        // m_c |c_c - c|^2 = |w_c - m_c c|^2 / m_c: u = w_c - m_c c by FMA
-        // keeps the cancellation in FP64; the division by m_c needs only
-        // the feature's precision (an FP32 reciprocal, 2^-22).  Masses are
-        // >= 0, so "> 0" is a test on the bit pattern.
+        // The distances of the children from the centres need only the sums:
+        // all nodes at once, with full warps.  Then the moments themselves,
+        // level by level, in place of the sums' x.
+        for (int t = threadIdx.x; t < m.off[kBins]; t += kChunkThreads) {
+            const int k = m.order[t];
+            const double4_32a sum = m.node[k];
+            if (__double_as_longlong(sum.w) <= 0) continue;
+            const double is = rcp_nr(sum.w);
+            const double gx = sum.x * is, gy = sum.y * is, gz = sum.z * is;
+            for (int c = m.cs[k]; c < m.cs[k + 1]; ++c) {
+                const int r = m.child[c];
+                m.uu[c] = moment_uu(r >= 0 ? m.leaf[r - c0] : m.node[~r - n0], gx, gy, gz);
+            }
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < c1 - c0; k += kChunkThreads) m.leaf[k].x = lq[c0 + k];
+        __syncthreads();
+        for (int level = 0; level < kDepths; ++level) {
+            const int lo = m.off[8 * level], hi = m.off[8 * level + 8];
+            if (lo == hi) continue;
+            for (int t = 4 * lo + threadIdx.x; t < 4 * hi; t += kChunkThreads) {
+                const int k = m.order[t >> 2], j = t & 3;
+                double q = 0.0;
+                if (__double_as_longlong(m.node[k].w) > 0) {
+                    const int f = m.cs[k], e = m.cs[k + 1];
+                    for (int c = f; c < e; c += 4) {
+                        double share = 0.0;
+                        if (c + j < e) {
+                            const int r = m.child[c + j];
+                            const double4_32a& v = r >= 0 ? m.leaf[r - c0] : m.node[~r - n0];
+                            share = moment_add(m.uu[c + j], v.w, v.x);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const double x = quad_get(share, i);
+                            if (c + i < e) q += x;
+                        }
+                    }
+                }
+                if (j == 0) {
+                    m.node[k].x = q;
+                    nq[n0 + k] = q;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// A node's sums (and second moment) from its children's in memory, for the
+// nodes of a later stage that do not fit its table.
+template <bool kMoments>
+__device__ __noinline__ void node_sums(int b, const int32_t* __restrict__ node_cs,
+                                       const int32_t* __restrict__ node_nchild, const int32_t* __restrict__ slot_ref,
+                                       const double4_32a* ls, double4_32a* ns, const double* lq, double* nq)
+{
+    const int s0 = node_cs[b] + 1, nc = node_nchild[b];
+    double4_32a sum;
+    for (int c = 0; c < nc; ++c) {
+        const int r = slot_ref[s0 + c];
+        add_sums(sum, load_sums(r >= 0 ? ls + r : ns + ~r), c == 0);
+    }
+    ns[b] = sum;
+    if (kMoments) {
         double q = 0.0;
-        if (__double_as_longlong(sm) > 0) {
-            const double is = rcp_nr(sm);
-            const double gx = sx * is, gy = sy * is, gz = sz * is;
+        if (__double_as_longlong(sum.w) > 0) {
+            const double is = rcp_nr(sum.w);
+            const double gx = sum.x * is, gy = sum.y * is, gz = sum.z * is;
             for (int c = 0; c < nc; ++c) {
                 const int r = slot_ref[s0 + c];
-                const double4_32a v = load_sums(r >= 0 ? ls + r : ns + ~r);
-                const double cq = __ldcg(r >= 0 ? lq + r : nq + ~r);
-                if (__double_as_longlong(v.w) > 0) {
-                    const double ux = fma(-v.w, gx, v.x), uy = fma(-v.w, gy, v.y), uz = fma(-v.w, gz, v.z);
-                    const double uu = fma(ux, ux, fma(uy, uy, uz * uz));
-                    q += cq + uu * widen(__frcp_rn(narrow_trunc(v.w)));
-                }
+                q += moment_share(load_sums(r >= 0 ? ls + r : ns + ~r), __ldcg(r >= 0 ? lq + r : nq + ~r), gx, gy, gz);
             }
         }
         nq[b] = q;
     }
 }
 
-// Depth buckets of the branching nodes (depths 0..20), three kernels:
-// per-block counts, a scan of each depth's block counts, per-block placement.
-constexpr int kBucketThreads = 1024;
-constexpr int kDepths = kMaxDepth;  // branching depths 0..20
-
-__global__ void bucket_count_kernel(const int32_t* __restrict__ counts, const uint8_t* __restrict__ node_depth,
-                                    int32_t* __restrict__ blk_cnt, int nblk)
-{
-    __shared__ int32_t c[kDepths];
-    if (threadIdx.x < kDepths) c[threadIdx.x] = 0;
-    __syncthreads();
-    const int B = counts[1];
-    const int b = blockIdx.x * kBucketThreads + threadIdx.x;
-    if (b < B) atomicAdd(&c[node_depth[b]], 1);
-    __syncthreads();
-    if (threadIdx.x < kDepths) blk_cnt[threadIdx.x * nblk + blockIdx.x] = c[threadIdx.x];
-}
-
-// One block per depth: the exclusive scan of that depth's per-block counts
-// (offsets within the depth's bucket) and the depth's total.
-__global__ void __launch_bounds__(kBucketThreads) bucket_scan_kernel(int32_t* __restrict__ blk_cnt, int nblk,
-                                                                      int32_t* __restrict__ depth_tot)
-{
-    __shared__ int32_t warp_tot[32];
-    const int d = blockIdx.x;
-    int32_t* c = blk_cnt + (int64_t)d * nblk;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int carry = 0;
-    for (int base = 0; base < nblk; base += kBucketThreads) {
-        const int i = base + threadIdx.x;
-        const int v = i < nblk ? c[i] : 0;
-        int x = v;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        if (lane == 31) warp_tot[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            int t = warp_tot[lane];
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, t, off);
-                if (lane >= off) t += y;
-            }
-            warp_tot[lane] = t;
-        }
-        __syncthreads();
-        if (i < nblk) c[i] = carry + (w > 0 ? warp_tot[w - 1] : 0) + x - v;
-        carry += warp_tot[31];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) depth_tot[d] = carry;
-}
-
-// Each block: the depth offsets from the totals (block 0 also stores them
-// for the level launches), then its nodes into their depth buckets.
-__global__ void bucket_place_kernel(const int32_t* __restrict__ counts, const uint8_t* __restrict__ node_depth,
-                                    const int32_t* __restrict__ blk_off, int nblk,
-                                    const int32_t* __restrict__ depth_tot, int32_t* __restrict__ depth_off,
-                                    int32_t* __restrict__ depth_nodes)
-{
-    __shared__ int32_t c[kDepths];
-    __shared__ int32_t off[kDepths + 1];
-    if (threadIdx.x < kDepths) c[threadIdx.x] = 0;
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int d = 0; d < kDepths; ++d) {
-            off[d] = run;
-            run += depth_tot[d];
-        }
-        off[kDepths] = run;
-    }
-    __syncthreads();
-    if (blockIdx.x == 0 && threadIdx.x <= kDepths) depth_off[threadIdx.x] = off[threadIdx.x];
-    const int B = counts[1];
-    const int b = blockIdx.x * kBucketThreads + threadIdx.x;
-    if (b < B) {
-        const int d = node_depth[b];
-        const int r = atomicAdd(&c[d], 1);  // order inside a bucket is irrelevant
-        depth_nodes[off[d] + blk_off[d * nblk + blockIdx.x] + r] = b;
-    }
-}
-
-// Monopole (and second moment) of the branching nodes at one depth, from
-// the sums of the level below (node_sums).
+// A later stage: the nodes left over by kFan groups of `leaves` leaves each.
+// Children whose sums are known already (leaves, nodes of earlier stages) are
+// loaded before the levels begin, the others' come through shared memory, so
+// that a level waits for no memory.  node_item: scratch, the place of a node in the order.
 template <bool kMoments>
-__global__ void monopole_level_kernel(int depth, const int32_t* __restrict__ depth_off,
-                                      const int32_t* __restrict__ depth_nodes, const int32_t* __restrict__ node_cs,
-                                      const int32_t* __restrict__ node_nchild, const int32_t* __restrict__ slot_ref,
-                                      const double4_32a* ls, double4_32a* ns, const double* lq, double* nq)
+struct RestSmem {
+    double4_32a sum[kRestItems];  // (kMoments: then the second moment in x)
+    int32_t order[kFan * kMaxSpan];  // local nodes, in bin order
+    int cnt[kBins], pos[kBins], off[kBins + 1], spans;
+};
+
+template <bool kMoments>
+__global__ void __launch_bounds__(kRestThreads) monopole_rest_kernel(
+    const int32_t* __restrict__ counts, int groups, int64_t leaves, const int32_t* __restrict__ in_cnt,
+    const int32_t* __restrict__ in, const int32_t* __restrict__ node_a, const int32_t* __restrict__ node_e,
+    const uint8_t* __restrict__ node_depth, const int32_t* __restrict__ node_cs,
+    const int32_t* __restrict__ node_nchild, const int32_t* __restrict__ slot_ref, const double4_32a* ls,
+    double4_32a* ns, const double* lq, double* nq, int32_t* node_item, int32_t* __restrict__ span_cnt,
+    int32_t* __restrict__ span)
 {
-    const int lo = depth_off[depth], hi = depth_off[depth + 1];
-    for (int k = lo + blockIdx.x * blockDim.x + threadIdx.x; k < hi; k += gridDim.x * blockDim.x)
-        node_sums<kMoments>(depth_nodes[k], node_cs, node_nchild, slot_ref, ls, ns, lq, nq);
+    static_assert(kRestThreads % kFan == 0, "equal shares of a list");
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    RestSmem<kMoments>& m = *reinterpret_cast<RestSmem<kMoments>*>(smem_raw);
+    const int L = counts[0];
+    const int64_t c0 = (int64_t)blockIdx.x * kFan * leaves;
+    const int64_t c1 = min((int64_t)L, c0 + kFan * leaves);
+    for (int k = threadIdx.x; k < kBins; k += kRestThreads) m.cnt[k] = m.pos[k] = 0;
+    if (threadIdx.x == 0) m.spans = 0;
+    __syncthreads();
+    // Thread t reads every (kRestThreads / kFan)th entry of list t % kFan.
+    const int g = blockIdx.x * kFan + threadIdx.x % kFan;
+    const int entries = g < groups ? in_cnt[g] : 0;
+    const int32_t* list = in + (int64_t)g * kMaxSpan;
+    auto place = [&](int b) { return node_a[b] >= c0 && node_e[b] <= c1 ? bin_of(node_depth[b], node_nchild[b]) : -1; };
+    for (int e = threadIdx.x / kFan; e < entries; e += kRestThreads / kFan) {
+        const int b = list[e], bin = place(b);
+        if (bin >= 0) {
+            atomicAdd(&m.cnt[bin], 1);
+        } else {
+            const int at = atomicAdd(&m.spans, 1);
+            if (at < kMaxSpan) span[(int64_t)blockIdx.x * kMaxSpan + at] = b;
+        }
+    }
+    __syncthreads();
+    bin_offsets(m.cnt, m.off);
+    if (threadIdx.x == 0) span_cnt[blockIdx.x] = min(m.spans, kMaxSpan);
+    __syncthreads();
+    for (int e = threadIdx.x / kFan; e < entries; e += kRestThreads / kFan) {
+        const int b = list[e], bin = place(b);
+        if (bin >= 0) {
+            const int k = m.off[bin] + atomicAdd(&m.pos[bin], 1);
+            m.order[k] = b;
+            node_item[b] = k;
+        }
+    }
+    __syncthreads();
+    // Lane j of four takes component j of the items (thread / 4) + i kQuads.
+    constexpr int kQuads = kRestThreads / 4, kItems = kRestItems / kQuads;
+    const int j = threadIdx.x & 3, quad = threadIdx.x >> 2, total = m.off[kBins];
+    const bool fits = total <= kRestItems;
+    int node[kItems], nc[kItems];
+    double v[kItems][8] = {};        // the children's component j
+    int16_t src[kItems][8];          // child c: its place in the order, or -1 with v[c] loaded
+    double cq[kMoments ? kItems : 1][2];  // second moments of children j and j + 4
+    if (fits) {
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const int k = quad + i * kQuads;
+            node[i] = nc[i] = 0;
+            if (k >= total) continue;
+            node[i] = m.order[k];
+            nc[i] = node_nchild[node[i]];
+            const int s0 = node_cs[node[i]] + 1;
+            int ref[8], at[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) ref[c] = c < nc[i] ? slot_ref[s0 + c] : 0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) at[c] = c < nc[i] && ref[c] < 0 ? __ldcg(node_item + ~ref[c]) : -1;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                // (node_item of a node of another stage or block is stale)
+                if ((unsigned)at[c] >= (unsigned)total || m.order[at[c]] != ~ref[c]) at[c] = -1;
+                src[i][c] = (int16_t)at[c];
+                if (c < nc[i] && at[c] < 0)
+                    v[i][c] = __ldcg(&(ref[c] >= 0 ? ls + ref[c] : ns + ~ref[c])->x + j);
+                if (kMoments && c < nc[i] && at[c] < 0 && (c & 3) == j)
+                    cq[i][c >> 2] = __ldcg(ref[c] >= 0 ? lq + ref[c] : nq + ~ref[c]);
+            }
+        }
+    }
+    for (int level = 0; level < kDepths; ++level) {
+        const int lo = m.off[8 * level], hi = m.off[8 * level + 8];
+        if (lo == hi) continue;
+        if (fits) {
+#pragma unroll
+            for (int i = 0; i < kItems; ++i) {
+                const int k = quad + i * kQuads;
+                if (k < lo || k >= hi) continue;
+                double sum = 0.0;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    if (c >= nc[i]) break;
+                    if (src[i][c] >= 0) v[i][c] = (&m.sum[src[i][c]].x)[j];
+                    sum = add_sum(sum, v[i][c], c == 0);
+                }
+                (&m.sum[k].x)[j] = sum;
+                (&ns[node[i]].x)[j] = sum;
+            }
+        } else {
+            for (int k = lo + threadIdx.x; k < hi; k += kRestThreads)
+                node_sums<kMoments>(m.order[k], node_cs, node_nchild, slot_ref, ls, ns, lq, nq);
+        }
+        __syncthreads();  // also orders the block's global writes
+    }
+    if (kMoments && fits) {
+        // As in the first stage: the distances for all nodes at once (kept by
+        // the lane that takes the child's term), then the moments level by
+        // level, in the place of the sums' x.
+        double uu[kItems][2], mass[kItems][2];
+        bool some[kItems];
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const int k = quad + i * kQuads;
+            some[i] = k < total && __double_as_longlong(m.sum[k < total ? k : 0].w) > 0;
+            if (!some[i]) continue;
+            const double4_32a sum = m.sum[k];
+            const double is = rcp_nr(sum.w);
+            const double gx = sum.x * is, gy = sum.y * is, gz = sum.z * is;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (4 * h >= nc[i]) break;
+                double4_32a w{0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const double x = quad_get(v[i][4 * h + c], 0), y = quad_get(v[i][4 * h + c], 1);
+                    const double z = quad_get(v[i][4 * h + c], 2), u = quad_get(v[i][4 * h + c], 3);
+                    if (c == j) w = double4_32a{x, y, z, u};
+                }
+                uu[i][h] = moment_uu(w, gx, gy, gz);
+                mass[i][h] = w.w;
+            }
+        }
+        __syncthreads();
+        for (int level = 0; level < kDepths; ++level) {
+            const int lo = m.off[8 * level], hi = m.off[8 * level + 8];
+            if (lo == hi) continue;
+#pragma unroll
+            for (int i = 0; i < kItems; ++i) {
+                const int k = quad + i * kQuads;
+                if (k < lo || k >= hi) continue;
+                double q = 0.0;
+                if (some[i]) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (4 * h >= nc[i]) break;
+                        const int at = j == 0 ? src[i][4 * h] : j == 1 ? src[i][4 * h + 1]
+                                     : j == 2 ? src[i][4 * h + 2] : src[i][4 * h + 3];
+                        double share = 0.0;
+                        if (4 * h + j < nc[i])
+                            share = moment_add(uu[i][h], mass[i][h], at >= 0 ? m.sum[at].x : cq[i][h]);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const double x = quad_get(share, c);
+                            if (4 * h + c < nc[i]) q += x;
+                        }
+                    }
+                }
+                if (j == 0) {
+                    m.sum[k].x = q;
+                    nq[node[i]] = q;
+                }
+            }
+            __syncthreads();
+        }
+    }
 }
 
 // com = w/m when m > 0 (linear_octree.cpp:95-104), then the merge of
@@ -703,6 +981,45 @@ __global__ void slot_count_kernel(int32_t* counts, const int32_t* __restrict__ c
 
 }  // namespace
 
+namespace {
+
+template <bool kMoments>
+int launch_monopoles(bh_context* ctx)
+{
+    cudaStream_t st = ctx->stream;
+    const size_t smem = sizeof(ChunkSmem<kMoments>);
+    BH_CUDA_TRY(cudaFuncSetAttribute(monopole_chunk_kernel<kMoments>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem));
+    static_assert(sizeof(RestSmem<true>) <= 48 * 1024, "no opt-in needed");
+    int64_t groups = (ctx->n + kChunk - 1) / kChunk;
+    // Two stages' lists in turn: counts, then kMaxSpan nodes per group.
+    const int64_t half = monopole_ints(ctx->cap) / 2;
+    int32_t* in = ctx->mono_span;
+    int32_t* out = ctx->mono_span + half;
+    monopole_chunk_kernel<kMoments><<<(unsigned)groups, kChunkThreads, smem, st>>>(
+        ctx->counts, ctx->rep_node, ctx->node_a, ctx->node_e, ctx->node_depth, ctx->node_cs, ctx->node_nchild,
+        ctx->slot_ref, ctx->leaf_s, ctx->node_s, ctx->leaf_q, ctx->node_q, in, in + groups);
+    BH_LAUNCH_CHECK(ctx);
+    for (int64_t leaves = kChunk; groups > 1; leaves *= kFan) {
+        const int64_t next = (groups + kFan - 1) / kFan;
+        monopole_rest_kernel<kMoments><<<(unsigned)next, kRestThreads, sizeof(RestSmem<kMoments>), st>>>(
+            ctx->counts, (int)groups, leaves, in, in + groups, ctx->node_a, ctx->node_e, ctx->node_depth, ctx->node_cs,
+            ctx->node_nchild, ctx->slot_ref, ctx->leaf_s, ctx->node_s, ctx->leaf_q, ctx->node_q, ctx->head, out,
+            out + next);
+        BH_LAUNCH_CHECK(ctx);
+        std::swap(in, out);
+        groups = next;
+    }
+    return BH_OK;
+}
+
+}  // namespace
+
+int64_t monopole_ints(int64_t n)
+{
+    return 2 * ((n + kChunk - 1) / kChunk) * (kMaxSpan + 1);
+}
+
 int64_t boundary_pass_ints(int64_t n)
 {
     const int64_t nb = (n + 1 + kBT - 1) / kBT;
@@ -766,33 +1083,9 @@ int launch_build(bh_context* ctx, const double* mass, bool moments, bool far_fus
         ctx->split_rank, ctx->slot_ref, ctx->slot_top, ctx->err);
     BH_LAUNCH_CHECK(ctx);
 
-    // 3./4. monopoles (and second moments), level by level, deepest first:
-    // depth buckets of the branching nodes, then one launch per depth; each
-    // node sums its children in slot order from 0.0.  No atomics.
-    {
-        const int nblk = (int)((n + kBucketThreads - 1) / kBucketThreads);
-        bucket_count_kernel<<<nblk, kBucketThreads, 0, st>>>(ctx->counts, ctx->node_depth, ctx->scan_tmp, nblk);
-        BH_LAUNCH_CHECK(ctx);
-        int32_t* depth_tot = ctx->scan_tmp + (int64_t)kDepths * nblk;
-        bucket_scan_kernel<<<kDepths, kBucketThreads, 0, st>>>(ctx->scan_tmp, nblk, depth_tot);
-        BH_LAUNCH_CHECK(ctx);
-        bucket_place_kernel<<<nblk, kBucketThreads, 0, st>>>(ctx->counts, ctx->node_depth, ctx->scan_tmp, nblk,
-                                                             depth_tot, ctx->depth_off, ctx->depth_nodes);
-        BH_LAUNCH_CHECK(ctx);
-        for (int d = kMaxDepth - 1; d >= 0; --d) {
-            if (moments)
-                monopole_level_kernel<true><<<g, kThreads, 0, st>>>(d, ctx->depth_off, ctx->depth_nodes,
-                                                                    ctx->node_cs, ctx->node_nchild, ctx->slot_ref,
-                                                                    ctx->leaf_s, ctx->node_s, ctx->leaf_q,
-                                                                    ctx->node_q);
-            else
-                monopole_level_kernel<false><<<g, kThreads, 0, st>>>(d, ctx->depth_off, ctx->depth_nodes,
-                                                                     ctx->node_cs, ctx->node_nchild, ctx->slot_ref,
-                                                                     ctx->leaf_s, ctx->node_s, ctx->leaf_q,
-                                                                     ctx->node_q);
-            BH_LAUNCH_CHECK(ctx);
-        }
-    }
+    // 3./4. monopoles (and second moments): chunks of leaves, then what reaches
+    // past them
+    if ((rc = moments ? launch_monopoles<true>(ctx) : launch_monopoles<false>(ctx))) return rc;
 
     // 5. traversal records
     const int gs = grid_for(2 * n, kThreads, maxb);
