@@ -57,6 +57,23 @@ __device__ inline int common_depth(uint64_t a, uint64_t b)
     return (62 - hb) / 3;
 }
 
+// The hardware's FP32 estimates of 1/sqrt(x) and sqrt(x) (within 2^-22) with
+// subnormal arguments taken as zero: rsqrtf and sqrtf put a scaling for those,
+// and sqrtf a correctly rounded result, around them.  (An r^-3 formed from
+// r^2 below 2^-126 overflows in FP32 either way.)
+__device__ __forceinline__ float rsqrt_est(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float sqrt_est(float x)
+{
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // 1/sqrt(x) in FP64 from the FP32 hardware estimate y0 (relative error below
 // 2^-21 with the truncation below) and one third-order Householder step for
 // f(y) = 1/y^2 - x:

@@ -90,9 +90,10 @@ constexpr int kStk = 384;
 // stays below this; the first one always may, which adds at most 8 items per
 // level of one root path (21 levels), so the stack never passes kStk.
 constexpr int kSoftStk = kStk - 21 * 8 - 8;
-// FP32 tests: a relative margin on the squares (eight roundings of 2^-24
-// each are below 5e-7) with an absolute one against underflow, and the error
-// of a group-relative distance relative to the coordinates' magnitudes: each
+// FP32 tests: a relative margin on the squares (eight roundings of 2^-24 each
+// and a square root's 2^-22 are below 1e-6) with an absolute one against
+// underflow (of squares below 2^-126, which sqrt_est takes as zero, too), and
+// the error of a group-relative distance relative to the coordinates' magnitudes: each
 // component of a difference is off by at most 2^-24 (3 |c| + 2 |r|), so the
 // distance by sqrt(3) times that, below 3.2e-7 (|c| + |r|); the hi + lo
 // split of an absolute coordinate adds 2^-46 of it, so sqrt(3) 2^-46, below
@@ -295,8 +296,8 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
                     const float fx = fmaxf(fabsf(cx - bminx), fabsf(cx - bmaxx));
                     const float fy = fmaxf(fabsf(cy - bminy), fabsf(cy - bmaxy));
                     const float fz = fmaxf(fabsf(cz - bminz), fabsf(cz - bmaxz));
-                    const float dlo = fmaxf(sqrtf(ex * ex + ey * ey + ez * ez) - nerr, 0.0f);
-                    const float dhi = sqrtf(fx * fx + fy * fy + fz * fz) + nerr;
+                    const float dlo = fmaxf(sqrt_est(ex * ex + ey * ey + ez * ez) - nerr, 0.0f);
+                    const float dhi = sqrt_est(fx * fx + fy * fy + fz * fz) + nerr;
                     const float s2 = sm.side2f[depth];
                     if (sure_below(s2, theta2f, dlo * dlo + soft2f)) A = M;
                     else mixed = !sure_above(s2, theta2f, dhi * dhi + soft2f);
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
                     const float4 u = sm.und[w][kk];
                     const int4 v = sm.und2[w][kk];
                     const float dxf = u.x - rx, dyf = u.y - ry, dzf = u.z - rz;
-                    const float df = sqrtf(dxf * dxf + dyf * dyf + dzf * dzf);
+                    const float df = sqrt_est(dxf * dxf + dyf * dyf + dzf * dzf);
                     const float lo = fmaxf(df - u.w, 0.0f), hi = df + u.w;
                     const float s2 = sm.side2f[v.x];
                     if (v.z >= 0 ? v.z != my_leaf : sure_below(s2, theta2f, lo * lo + soft2f)) {

@@ -26,7 +26,7 @@
 //   displacement's bits on the integer pipes, to within an ulp
 //   (soft::scale); six FP64 instructions per 32 pairs are left of 13 (the
 //   differences and the accumulating FMAs).  300,149 bodies, theta 1.05:
-//   3.27 -> 1.90 ms of forces.
+//   3.27 -> 1.88 ms of forces.
 // BH_MODE_FP32_FAR: precision form.  The bodies with id < num_direct (Sun and
 //   planets) are taken out of the tree (masses zeroed before the build) and
 //   summed directly in FP64.  Far-field interactions run in FP32 on
@@ -36,9 +36,13 @@
 //   one FP64 instruction per visit (the FP64 pipe is 1/60 of the FP32 one
 //   here, and three FP64 subtractions per visit would cost more than the
 //   interaction).  FP32 partials of each staged list are added into FP64
-//   accumulators.
+//   accumulators.  Instruction issue bounds it: with the plain hardware
+//   estimates (rsqrt_est, sqrt_est) and the popped ranges counted by ballots
+//   instead of a shuffle scan, 1M bodies (theta 0.8) went from 1.61 to
+//   1.49 ms of forces, the group form at 4M (theta 1.05) from 3.37 to 3.14.
 // Collection (bh_learned_collect): the FP32 walk with the theta test only,
 //   recording every candidate's group, slot, lane mask and raw features.
+#include <cfloat>
 #include <climits>
 
 #include "bh_soft64.cuh"
@@ -273,37 +277,29 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                 }
             } else {
                 // Pop whole ranges from the top while they fit in 32 lanes.
+                // (The running counts come from ballots of the counts' bits.)
                 const int avail = sp < 32 ? sp : 32;
-                int rfirst = 0, rcnt = 0;
-                unsigned rmask = 0;
-                if (lane < avail) {
-                    const int2 ent = stk[sp - 1 - lane];
-                    rfirst = ent.x & ((1 << kSlotBits) - 1);
-                    rcnt = (int)((unsigned)ent.x >> kSlotBits) + 1;
-                    rmask = (unsigned)ent.y;
-                }
-                int incl = rcnt;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, off);
-                    if (lane >= off) incl += t;
-                }
+                int2 ent = make_int2(0, 0);
+                if (lane < avail) ent = stk[sp - 1 - lane];
+                const int cm1 = (int)((unsigned)ent.x >> kSlotBits);  // count - 1
+                const unsigned le = lt | me;
+                const int incl = min(lane + 1, avail) + __popc(__ballot_sync(0xffffffffu, cm1 & 1) & le) +
+                                 2 * __popc(__ballot_sync(0xffffffffu, cm1 & 2) & le) +
+                                 4 * __popc(__ballot_sync(0xffffffffu, cm1 & 4) & le);
                 const bool take = lane < avail && incl <= 32;
                 R = __popc(__ballot_sync(0xffffffffu, take));
                 const int T = __shfl_sync(0xffffffffu, incl, R - 1);
-                const int rstart = incl - rcnt;
+                const int rstart = incl - cm1 - 1;
                 const unsigned starts = __reduce_or_sync(0xffffffffu, take ? (1u << rstart) : 0u);
-                const int rj = __popc(starts & ((2u << lane) - 1u)) - 1;
-                const int f_r = __shfl_sync(0xffffffffu, rfirst, rj);
-                const int s_r = __shfl_sync(0xffffffffu, rstart, rj);
-                m_r = __shfl_sync(0xffffffffu, rmask, rj);
+                const int rj = __popc(starts & le) - 1;
+                node = __shfl_sync(0xffffffffu, (ent.x & ((1 << kSlotBits) - 1)) - rstart, rj) + lane;
+                m_r = kGroup ? full : __shfl_sync(0xffffffffu, (unsigned)ent.y, rj);
                 pops += T;
                 if (sp - R + T > Smem::kStk || pops > p.max_pops) {
                     overflow = true;
                     break;
                 }
                 has = lane < T;
-                node = f_r + (lane - s_r);
             }
             unsigned M = 0, A = 0;
             int nc = 0, ref = 0, depth = 0;
@@ -339,7 +335,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                     nerr = err;
                     if (kFP64) {
                         s2 = sm.side2f[depth];
-                        const float dlo = fmaxf(sqrtf(dmin2) - err, 0.0f), dhi = sqrtf(dmax2) + err;
+                        const float dlo = fmaxf(sqrt_est(dmin2) - err, 0.0f), dhi = sqrt_est(dmax2 + FLT_MIN) + err;
                         if (s2 * (1.0f + kMargin) < theta2f * dlo * dlo) A = M;
                         else if (s2 * (1.0f - kMargin) > theta2f * dhi * dhi) A = 0;
                         else mixed = true;
@@ -424,7 +420,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                     const float cz = __shfl_sync(0xffffffffu, e.z, j);
                     const float ej = 2.0f * __shfl_sync(0xffffffffu, nerr, j);
                     const float dxf = cx - rx, dyf = cy - ry, dzf = cz - rz;
-                    const float df = sqrtf(dxf * dxf + dyf * dyf + dzf * dzf);
+                    const float df = sqrt_est(dxf * dxf + dyf * dyf + dzf * dzf + FLT_MIN);
                     const float lo = fmaxf(df - ej, 0.0f), hi = df + ej;
                     const float s2j = sm.side2f[dj], sf = (float)soft2;
                     const bool sure_acc = s2j * (1.0f + kMargin) < theta2f * (lo * lo + sf);
@@ -518,7 +514,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                         const float gm = __shfl_sync(0xffffffffu, e.w, j);
                         if (Aj & me) {
                             const float dx = cx - rx, dy = cy - ry, dz = cz - rz;
-                            const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, (float)soft2))));
+                            const float inv = rsqrt_est(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, (float)soft2))));
                             const float sc = gm * (inv * inv * inv);
                             ox = fmaf(sc, dx, ox);
                             oy = fmaf(sc, dy, oy);
@@ -543,7 +539,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                 }
                 if (kFP64) LN[pos] = node;
                 if (Smem::kLL) LL[pos] = leaf ? ref : -1;  // for the own-leaf test
-                LM[pos] = A;
+                if (!kGroup) LM[pos] = A;
             }
             nlist += __popc(am);
             // Push one sibling range per opened node, with the lanes that
@@ -686,7 +682,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                         float* P = reinterpret_cast<float*>(L + (nlist - 1)) + 1;
                         P[0] = P[2] = P[4] = kGroup ? 1e18f : 0.0f;
                         P[6] = 0.0f;
-                        LM[nlist] = 0u;
+                        if (!kGroup) LM[nlist] = 0u;
                     }
                     __syncwarp();
                 }
@@ -702,7 +698,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                         const f32x2 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, sf2)));
                         float r0, r1;
                         upk(r2, r0, r1);
-                        const f32x2 inv = pk(rsqrtf(r0), rsqrtf(r1));
+                        const f32x2 inv = pk(rsqrt_est(r0), rsqrt_est(r1));
                         const f32x2 sc = mul2(zw.y, mul2(mul2(inv, inv), inv));
                         fx = fma2(sc, dx, fx);
                         fy = fma2(sc, dy, fy);
@@ -718,7 +714,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                     const f32x2 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, sf2)));
                     float r0, r1;
                     upk(r2, r0, r1);
-                    const f32x2 inv = pk(rsqrtf(r0), rsqrtf(r1));
+                    const f32x2 inv = pk(rsqrt_est(r0), rsqrt_est(r1));
                     float s0, s1;
                     upk(mul2(zw.y, mul2(mul2(inv, inv), inv)), s0, s1);
                     const bool t0 = (mj.x & me) != 0u, t1 = (mj.y & me) != 0u;

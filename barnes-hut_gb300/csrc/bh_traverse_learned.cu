@@ -18,6 +18,7 @@
 // each lane of its mask decides for itself, as in the plain walk.
 // Candidates whose features fall outside the training range go the same way
 // and are counted.
+#include <cfloat>
 #include <climits>
 
 #include "bh_walk.cuh"
@@ -33,6 +34,8 @@ constexpr int kPendCap = 32;    // deferred candidates per warp
 struct LearnSmem : WalkSmem<false, kLearnInfer> {
     int pend_node[kWarps][kPendCap];
     unsigned pend_mask[kWarps][kPendCap];
+    float spread_min[kMaxDepth + 1];  // the spread's floor, 1e-8 of the side, per depth
+    float l2side2[kMaxDepth + 1];     // log2 side^2
 };
 
 // Five blocks per SM: the network's fragments and the deferral state take
@@ -50,7 +53,10 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
         if (L < dz) L = dz;
         const double side = __ddiv_rn(L, (double)(1ull << threadIdx.x));
         sm.side2d[threadIdx.x] = __dmul_rn(side, side);
-        sm.side2f[threadIdx.x] = (float)sm.side2d[threadIdx.x];
+        const float s2f = (float)sm.side2d[threadIdx.x];
+        sm.side2f[threadIdx.x] = s2f;
+        sm.spread_min[threadIdx.x] = 1e-8f * sqrtf(s2f);
+        sm.l2side2[threadIdx.x] = __log2f(s2f);
     }
     __syncthreads();
 
@@ -148,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
         // stack's when enough wait (or nothing else is left).
         const bool from_pend = npend > 0 && (npend >= kPendFlush || sp == 0);
         if (sp > 0 || from_pend) {
-            int R = 0, T = 0, f_r = 0, s_r = 0;
+            int R = 0, T = 0, first = 0;
             unsigned m_r = 0;
             float plerr = 0.0f;  // network's predicted log10 error of deferred row `lane`
             if (from_pend) {
@@ -161,30 +167,23 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
                 }
             } else {
                 // Pop whole ranges from the top while they fit in 32 lanes.
+                // (The running counts come from ballots of the counts' bits.)
                 const int avail = sp < 32 ? sp : 32;
-                int rfirst = 0, rcnt = 0;
-                unsigned rmask = 0;
-                if (lane < avail) {
-                    const int2 ent = stk[sp - 1 - lane];
-                    rfirst = ent.x & ((1 << kSlotBits) - 1);
-                    rcnt = (int)((unsigned)ent.x >> kSlotBits) + 1;
-                    rmask = (unsigned)ent.y;
-                }
-                int incl = rcnt;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, off);
-                    if (lane >= off) incl += t;
-                }
+                int2 ent = make_int2(0, 0);
+                if (lane < avail) ent = stk[sp - 1 - lane];
+                const int cm1 = (int)((unsigned)ent.x >> kSlotBits);  // count - 1
+                const unsigned le = lt | me;
+                const int incl = min(lane + 1, avail) + __popc(__ballot_sync(0xffffffffu, cm1 & 1) & le) +
+                                 2 * __popc(__ballot_sync(0xffffffffu, cm1 & 2) & le) +
+                                 4 * __popc(__ballot_sync(0xffffffffu, cm1 & 4) & le);
                 const bool take = lane < avail && incl <= 32;
                 R = __popc(__ballot_sync(0xffffffffu, take));
                 T = __shfl_sync(0xffffffffu, incl, R - 1);
-                const int rstart = incl - rcnt;
+                const int rstart = incl - cm1 - 1;
                 const unsigned starts = __reduce_or_sync(0xffffffffu, take ? (1u << rstart) : 0u);
-                const int rj = __popc(starts & ((2u << lane) - 1u)) - 1;
-                f_r = __shfl_sync(0xffffffffu, rfirst, rj);
-                s_r = __shfl_sync(0xffffffffu, rstart, rj);
-                m_r = __shfl_sync(0xffffffffu, rmask, rj);
+                const int rj = __popc(starts & le) - 1;
+                first = __shfl_sync(0xffffffffu, (ent.x & ((1 << kSlotBits) - 1)) - rstart, rj);
+                m_r = __shfl_sync(0xffffffffu, (unsigned)ent.y, rj);
                 pops += T;
                 if (sp - R + T > kStack || pops > p.max_pops) {
                     overflow = true;
@@ -203,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
                     node = sm.pend_node[w][lane];
                     M = sm.pend_mask[w][lane];
                 } else {
-                    node = f_r + (lane - s_r);
+                    node = first + lane;
                     M = m_r;
                 }
                 const float4 a = __ldg(p.A + node);
@@ -231,7 +230,7 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
                     nc = (int)(mt & 0xFF);
                     // Absolute error of the FP32 group-relative distances.
                     const float err = kAbsErr * (fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + bmag);
-                    const float dlo = fmaxf(sqrtf(dmin2) - err, 0.0f), dhi = sqrtf(dmax2) + err;
+                    const float dlo = fmaxf(sqrt_est(dmin2) - err, 0.0f), dhi = sqrt_est(dmax2 + FLT_MIN) + err;
                     if (s2 * (1.0f + kMargin) < theta2f * dlo * dlo) {
                         A = M;
                     } else {
@@ -262,11 +261,12 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
                     lerr = plerr;
                 } else if (__ballot_sync(0xffffffffu, cand)) {
                     constexpr float kL = 0.30102999566f;  // log10(2)
-                    float l2dmin = 0.0f, lspr = 0.0f, lest = 0.0f;
+                    float l2dmin = 0.0f, lspr = 0.0f, lgm = 0.0f, lest = 0.0f;
                     if (cand) {
                         l2dmin = __log2f(dmin2);
-                        lspr = __log2f(fmaxf(__ldg(p.spread + node), 1e-8f * sqrtf(s2)));
-                        lest = kL * (__log2f(e.w) - l2dmin - lascale) + 2.0f * kL * (lspr - 0.5f * l2dmin);
+                        lspr = __log2f(fmaxf(__ldg(p.spread + node), sm.spread_min[depth]));
+                        lgm = kL * (__log2f(e.w) - l2dmin - lascale);
+                        lest = lgm + 2.0f * kL * (lspr - 0.5f * l2dmin);
                     }
                     const bool sure = cand && lest + p.l_band < lallow;
                     const bool band = cand && !sure && lest - p.l_band <= lallow;
@@ -274,14 +274,14 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
                     float zq[kFeat];
                     if (band) {
                         // the features, as the collection computes them
-                        const float l2s = __log2f(s2);
+                        const float l2s = sm.l2side2[depth];
                         const float dcx = e.x - bcx, dcy = e.y - bcy, dcz = e.z - bcz;
                         const float ldmin = 0.5f * l2dmin;
                         float f[kFeat];
                         f[0] = kL * (0.5f * l2s - ldmin);
                         f[1] = kL * (lspr - ldmin);
                         f[2] = kL * (lext - ldmin);
-                        f[3] = kL * (__log2f(e.w) - l2dmin - lascale);
+                        f[3] = lgm;
                         f[4] = kL * 0.5f * (__log2f(dmax2) - l2dmin);
                         f[5] = (float)depth * (1.0f / kMaxDepth);
                         f[6] = kL * (lspr - 0.5f * l2s);
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kThreads, 5) traverse_learned_kernel(FParams p
                 const f32x2 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, sf2)));
                 float r0, r1;
                 upk(r2, r0, r1);
-                const f32x2 inv = pk(rsqrtf(r0), rsqrtf(r1));
+                const f32x2 inv = pk(rsqrt_est(r0), rsqrt_est(r1));
                 float s0, s1;
                 upk(mul2(zw.y, mul2(mul2(inv, inv), inv)), s0, s1);
                 const bool t0 = (mj.x & me) != 0u, t1 = (mj.y & me) != 0u;
