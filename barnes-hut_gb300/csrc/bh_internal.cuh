@@ -30,6 +30,9 @@ constexpr int kRadix = 256;
 constexpr int kSortThreads = 512;      // onesweep tile: 512 threads x 8 keys
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kClusterSortMax = 65536;  // keys one cluster sorts (8 blocks x 8192; 16-bit payloads)
+// Whether launch_sort reads the digit histograms of launch_keys / launch_hist.
+inline bool sort_uses_hist(int64_t n) { return n > kClusterSortMax; }
 
 // SM count of the current device (cudaDevAttrMultiProcessorCount), read once
 // per device and cached; grids are sized in multiples of it.  1 when the
@@ -487,9 +490,10 @@ int launch_permute(bh_context* ctx);
 // The permutation gathers into the second body set; the two sets then trade
 // places (host pointers only).
 void swap_body_sets(bh_context* ctx);
-// Digit counts for sort_passes_raw (hist zeroed by the caller).
-int launch_digit_hist(int64_t n, const uint64_t* keys, uint32_t* hist, cudaStream_t st);
-// The onesweep passes over raw buffers (the allocation-free sort entry).
+// Digit counts and zeroed counters for sort_passes_raw.
+int prepare_sort_raw(int64_t n, const uint64_t* keys, uint32_t* hist, uint32_t* lookback, uint32_t* tile_ctr,
+                     cudaStream_t st);
+// The sort over raw buffers (the allocation-free sort entry, the LET codes).
 int sort_passes_raw(int64_t n, const uint64_t* keys_in, uint64_t* keys_out, uint32_t* vals_out, uint64_t* key_alt,
                     uint32_t* val_alt, uint32_t* hist, uint32_t* lookback, uint32_t* tile_ctr, unsigned* err,
                     cudaStream_t stream);

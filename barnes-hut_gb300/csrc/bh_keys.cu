@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kKeyThreads) hist_kernel(int64_t n, const uint
 
 int launch_hist(bh_context* ctx)
 {
-    if (ctx->n == 0) return BH_OK;
+    if (ctx->n == 0 || !sort_uses_hist(ctx->n)) return BH_OK;
     BH_CUDA_TRY(cudaMemsetAsync(ctx->hist, 0, sizeof(uint32_t) * kSortPasses * kRadix, ctx->stream));
     int64_t want = (ctx->n + kKeyThreads * 4 - 1) / (kKeyThreads * 4);
     const int blocks = (int)(want < 1 ? 1 : (want > 4 * bh::num_sms() ? 4 * bh::num_sms() : want));
@@ -234,6 +234,7 @@ int bbox_partial_bytes(int blocks) { return blocks * 6 * (int)sizeof(Ext); }
 int launch_keys(bh_context* ctx, bool with_hist)
 {
     if (ctx->n == 0) return BH_OK;
+    with_hist = with_hist && sort_uses_hist(ctx->n);
     if (with_hist) BH_CUDA_TRY(cudaMemsetAsync(ctx->hist, 0, sizeof(uint32_t) * kSortPasses * kRadix, ctx->stream));
     int64_t want = (ctx->n + kKeyThreads * 4 - 1) / (kKeyThreads * 4);
     const int blocks = (int)(want < 1 ? 1 : (want > 4 * bh::num_sms() ? 4 * bh::num_sms() : want));

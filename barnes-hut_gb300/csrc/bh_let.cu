@@ -670,11 +670,8 @@ int pseudo_tree_device(bh_context* ctx, const uint64_t* prefix, const uint8_t* d
         BH_CUDA_TRY(cudaMemsetAsync(perm, 0, sizeof(uint32_t), st));
         BH_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
     } else {
-        BH_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * bh::kSortPasses * bh::kRadix, st));
-        BH_CUDA_TRY(cudaMemsetAsync(lookback, 0, sizeof(uint32_t) * bh::kSortPasses * tiles * bh::kRadix, st));
-        BH_CUDA_TRY(cudaMemsetAsync(tile_ctr, 0, sizeof(uint32_t) * bh::kSortPasses, st));
         BH_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
-        if ((rc = bh::launch_digit_hist(t, code, hist, st))) return rc;
+        if ((rc = bh::prepare_sort_raw(t, code, hist, lookback, tile_ctr, st))) return rc;
         if ((rc = bh::sort_passes_raw(t, code, code_s, perm, key_alt, val_alt, hist, lookback, tile_ctr, err, st)))
             return rc;
     }
@@ -1035,10 +1032,7 @@ extern "C" int bh_let_accelerations(bh_context* ctx, const uint64_t* prefix, con
         BH_CUDA_TRY(cudaMemcpyAsync(code_s, code, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
         BH_CUDA_TRY(cudaMemsetAsync(perm, 0, sizeof(uint32_t), st));
     } else {
-        BH_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * bh::kSortPasses * bh::kRadix, st));
-        BH_CUDA_TRY(cudaMemsetAsync(lookback, 0, sizeof(uint32_t) * bh::kSortPasses * tiles * bh::kRadix, st));
-        BH_CUDA_TRY(cudaMemsetAsync(tile_ctr, 0, sizeof(uint32_t) * bh::kSortPasses, st));
-        if ((rc = bh::launch_digit_hist(t, code, hist, st))) return rc;
+        if ((rc = bh::prepare_sort_raw(t, code, hist, lookback, tile_ctr, st))) return rc;
         if ((rc = bh::sort_passes_raw(t, code, code_s, perm, key_alt, val_alt, hist, lookback, tile_ctr, err, st)))
             return rc;
     }

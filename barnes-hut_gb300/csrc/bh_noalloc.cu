@@ -84,10 +84,16 @@ __global__ void __launch_bounds__(kHistThreads) noalloc_hist_kernel(int64_t n, c
 
 namespace bh {
 
-// Digit counts of the eight passes (hist: kSortPasses x kRadix, zeroed by
-// the caller) for sort_passes_raw.
-int launch_digit_hist(int64_t n, const uint64_t* keys, uint32_t* hist, cudaStream_t st)
+// What sort_passes_raw reads: the digit counts of the eight passes (hist),
+// and zeroed look-back words of the tiles this call uses and tile counters.
+int prepare_sort_raw(int64_t n, const uint64_t* keys, uint32_t* hist, uint32_t* lookback, uint32_t* tile_ctr,
+                     cudaStream_t st)
 {
+    if (!sort_uses_hist(n)) return BH_OK;
+    const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+    BH_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kSortPasses * kRadix, st));
+    BH_CUDA_TRY(cudaMemsetAsync(lookback, 0, sizeof(uint32_t) * kSortPasses * tiles * kRadix, st));
+    BH_CUDA_TRY(cudaMemsetAsync(tile_ctr, 0, sizeof(uint32_t) * kSortPasses, st));
     int64_t blocks = (n + kHistThreads * 4 - 1) / (kHistThreads * 4);
     if (blocks > 4 * bh::num_sms()) blocks = 4 * bh::num_sms();
     if (blocks < 1) blocks = 1;
@@ -128,14 +134,8 @@ extern "C" int bh_sort_keys_noalloc(const uint64_t* keys_in, uint64_t* keys_out,
         BH_CUDA_TRY(cudaStreamSynchronize(st));
         return BH_OK;
     }
-    // Clear what must start at zero: histograms, the look-back words of the
-    // tiles this call uses, tile counters, the error word.
-    const int64_t tiles = (n + bh::kSortTile - 1) / bh::kSortTile;
-    BH_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * bh::kSortPasses * bh::kRadix, st));
-    BH_CUDA_TRY(cudaMemsetAsync(lookback, 0, sizeof(uint32_t) * bh::kSortPasses * tiles * bh::kRadix, st));
-    BH_CUDA_TRY(cudaMemsetAsync(tile_ctr, 0, sizeof(uint32_t) * bh::kSortPasses, st));
     BH_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
-    if ((rc = bh::launch_digit_hist(n, keys_in, hist, st))) return rc;
+    if ((rc = bh::prepare_sort_raw(n, keys_in, hist, lookback, tile_ctr, st))) return rc;
     if ((rc = bh::sort_passes_raw(n, keys_in, keys_out, perm_out, key_alt, val_alt, hist, lookback, tile_ctr, err,
                                   st)))
         return rc;

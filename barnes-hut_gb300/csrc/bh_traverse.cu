@@ -31,7 +31,7 @@
 //
 // Measured (theta 1.05, ms of forces; before: one node per pass, 32 bodies
 // per warp, IEEE operations on the FP64 pipe):
-//   300,149 bodies 12.66 -> 2.96, 19,054 7.71 -> 1.21, 1,000 1.23 -> 0.071.
+//   300,149 bodies 12.66 -> 2.90, 19,054 7.71 -> 1.21, 1,000 1.23 -> 0.071.
 #include <climits>
 
 #include "bh_internal.cuh"
