@@ -279,7 +279,7 @@ int step_once(bh_context* ctx, double dt, double theta, double G, int mode)
 // A step with the kick (every step of a run after its first) through a CUDA
 // graph: captured from step_once on first use for this (bodies, mode, dt,
 // theta, G, merge, direct-body count) configuration, then replayed, which
-// enqueues the step's ~50 kernels with one call.  The step reads one body set
+// enqueues the step's 15 to 40 kernels with one call.  The step reads one body set
 // and leaves the state in the other, so there is one graph per starting set;
 // after a replay the host pointers trade places as step_once's permutation
 // would make them.  The kernels read no host state that the key leaves out:

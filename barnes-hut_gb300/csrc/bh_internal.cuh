@@ -363,7 +363,7 @@ struct bh_context {
     // Radix sort scratch.
     uint64_t* key_alt = nullptr;
     uint32_t* perm = nullptr;      // after the sort: previous position per slot
-    uint32_t* perm_alt = nullptr;
+    uint32_t* perm_alt = nullptr;  // the sort's second payload; the build's block-local child numbers
     uint32_t* hist = nullptr;      // kSortPasses x 256 digit counts, then starts
     uint32_t* lookback = nullptr;  // kSortPasses x tiles x 256 status words
     uint32_t* tile_ctr = nullptr;  // kSortPasses tile counters
@@ -387,7 +387,7 @@ struct bh_context {
     int32_t* bnd_next = nullptr;    // boundary j: next boundary no deeper than j, n + 1
     int32_t* split_node = nullptr;  // boundary j: the branching node it splits, n + 1
     int8_t* split_rank = nullptr;   // boundary j: its rank among that node's splits, n + 1
-    int32_t* ansv_blk = nullptr;    // per-block summaries of the boundary pass
+    int32_t* ansv_blk = nullptr;    // per-block summaries of the boundary pass, then child counts
     int32_t* rep_node = nullptr;    // branching-node id of a representative boundary
     int32_t* node_rep = nullptr;    // representative boundary of each node
     int32_t* node_a = nullptr;      // first leaf of each node

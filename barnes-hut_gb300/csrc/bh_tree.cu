@@ -28,6 +28,13 @@
 // step mass' = 0 + mass, com' = (0*0 + mass*com) / mass'.  All with IEEE
 // double intrinsics (no contraction), so masses and centres of mass are bit
 // for bit the reference's.
+//
+// Below some 100,000 bodies the launches bound the build (3 to 5 us each, and
+// every stage needs the one before), so a stage carries what the next needs
+// from it in its blocks' sums: the representatives' and children's numbers
+// come from the resolve and split passes themselves, with no scans of their
+// own.  Build per step, before -> after: 1,000 bodies 89 -> 60 us, 19,054
+// 97 -> 72, 300,149 182 -> 123, 1M 257 -> 234, 4M 728 -> 707.
 #include <climits>
 #include <utility>
 
@@ -52,58 +59,6 @@ inline int grid_for(int64_t n, int threads, int max_blocks)
     return (int)(b > max_blocks ? max_blocks : b);
 }
 
-// Leaf sums in body order (linear_octree.cpp:28-38) and boundary depths.
-// kMoments: also the leaf's second moment about its centre of mass (the
-// learned criterion's spread feature), sum_b m_b |x_b - c|^2.
-// nzero > 0: the bodies with id < nzero count as massless (the FP32 forms'
-// far-field tree, which leaves the Sun and planets to the direct terms).
-template <bool kMoments>
-__global__ void leaf_sum_kernel(const int32_t* __restrict__ counts, const int32_t* __restrict__ leaf_first,
-                                const uint64_t* __restrict__ leaf_key, const double* __restrict__ px,
-                                const double* __restrict__ py, const double* __restrict__ pz,
-                                const double* __restrict__ m, const uint64_t* __restrict__ id, int nzero,
-                                double4_32a* __restrict__ ls, int8_t* __restrict__ cdep, double* __restrict__ lq)
-{
-    auto mass = [&](int b) { return nzero > 0 && id[b] < (uint64_t)nzero ? 0.0 : m[b]; };
-    const int L = counts[0];
-    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < L; l += gridDim.x * blockDim.x) {
-        double sm = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
-        const int b0 = leaf_first[l], b1 = leaf_first[l + 1];
-        if (b1 == b0 + 1) {
-            // One body: each sum is 0.0 + v, which is v except that -0.0
-            // becomes +0.0; decided on the bit patterns (no FP64 addition).
-            const double mb = mass(b0);
-            sm = plus_zero(mb);
-            sx = plus_zero(__dmul_rn(px[b0], mb));
-            sy = plus_zero(__dmul_rn(py[b0], mb));
-            sz = plus_zero(__dmul_rn(pz[b0], mb));
-        } else {
-            for (int b = b0; b < b1; ++b) {
-                const double mb = mass(b);
-                sm = __dadd_rn(sm, mb);
-                sx = __dadd_rn(sx, __dmul_rn(px[b], mb));
-                sy = __dadd_rn(sy, __dmul_rn(py[b], mb));
-                sz = __dadd_rn(sz, __dmul_rn(pz[b], mb));
-            }
-        }
-        ls[l] = double4_32a{sx, sy, sz, sm};
-        cdep[l] = l == 0 ? (int8_t)-1 : (int8_t)common_depth(leaf_key[l - 1], leaf_key[l]);
-        if (l == L - 1) cdep[L] = -1;  // right sentinel of the boundary pass
-        if (kMoments) {
-            double q = 0.0;
-            if (b1 - b0 > 1 && sm > 0) {
-                const double is = rcp_nr(sm);
-                const double cx = sx * is, cy = sy * is, cz = sz * is;
-                for (int b = b0; b < b1; ++b) {
-                    const double dx = px[b] - cx, dy = py[b] - cy, dz = pz[b] - cz;
-                    q += mass(b) * (dx * dx + dy * dy + dz * dz);
-                }
-            }
-            lq[l] = q;
-        }
-    }
-}
-
 // ---- Tree structure from the boundary depths ---------------------------
 // With d(j) = cdep[j] for the boundaries 1 <= j < L and d(0) = d(L) = -1,
 // the branching node that boundary j splits (the cell of depth d(j) holding
@@ -123,6 +78,10 @@ __global__ void leaf_sum_kernel(const int32_t* __restrict__ counts, const int32_
 constexpr int kNT = kMaxDepth + 1;  // thresholds t: d <= t - 1
 constexpr int kBT = 1024;           // boundary positions per block
 constexpr int kBW = kBT / 32;
+// Up to this many blocks the resolve pass scans the blocks' summaries itself
+// instead of reading bnd_scan_kernel's result (a launch, about 3 us, against
+// four loads a lane).
+constexpr int kDirectBlocks = 128;
 
 __device__ __forceinline__ int bnd_depth(const int8_t* __restrict__ cdep, int L, int64_t j)
 {
@@ -159,16 +118,69 @@ __device__ __forceinline__ void warp_threshold_ends(int v, int lane, int wbase, 
     for (int t = lo; t <= min(p_prev, kNT - 1); ++t) wf[t] = wbase + lane;
 }
 
-// Per block: for every threshold the last and the first position at or below it.
-__global__ void __launch_bounds__(kBT) bnd_summary_kernel(const int32_t* __restrict__ counts,
-                                                          const int8_t* __restrict__ cdep,
-                                                          int32_t* __restrict__ blast, int32_t* __restrict__ bfirst)
+// Leaf sums in body order (linear_octree.cpp:28-38), boundary depths, and per
+// block, for every threshold, the last and the first position at or below it.
+// A thread per boundary position; two blocks to an SM (32 registers) for the
+// loads in flight: 107 us at 4M with one, 70 with two.
+// kMoments: also the leaf's second moment about its centre of mass (the
+// learned criterion's spread feature), sum_b m_b |x_b - c|^2.
+// nzero > 0: the bodies with id < nzero count as massless (the FP32 forms'
+// far-field tree, which leaves the Sun and planets to the direct terms).
+template <bool kMoments>
+__global__ void __launch_bounds__(kBT, 2) leaf_bnd_kernel(
+    const int32_t* __restrict__ counts, const int32_t* __restrict__ leaf_first, const uint64_t* __restrict__ leaf_key,
+    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
+    const double* __restrict__ m, const uint64_t* __restrict__ id, int nzero, double4_32a* __restrict__ ls,
+    int8_t* __restrict__ cdep, double* __restrict__ lq, int32_t* __restrict__ blast, int32_t* __restrict__ bfirst)
 {
     static_assert(kNT <= 32, "one lane per threshold");
     __shared__ int wl[kBW][kNT], wf[kBW][kNT];
+    auto mass = [&](int b) { return nzero > 0 && id[b] < (uint64_t)nzero ? 0.0 : m[b]; };
     const int L = counts[0];
     const int64_t j = (int64_t)blockIdx.x * kBT + threadIdx.x;
-    const int v = bnd_depth(cdep, L, j);
+    int v = 127;  // past the sentinel: no threshold
+    if (j < L) {
+        const int l = (int)j;
+        double sm = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+        const int b0 = leaf_first[l], b1 = leaf_first[l + 1];
+        v = l == 0 ? -1 : common_depth(leaf_key[l - 1], leaf_key[l]);
+        cdep[l] = (int8_t)v;
+        if (b1 == b0 + 1) {
+            // One body: each sum is 0.0 + v, which is v except that -0.0
+            // becomes +0.0; decided on the bit patterns (no FP64 addition).
+            const double mb = mass(b0);
+            sm = plus_zero(mb);
+            sx = plus_zero(__dmul_rn(px[b0], mb));
+            sy = plus_zero(__dmul_rn(py[b0], mb));
+            sz = plus_zero(__dmul_rn(pz[b0], mb));
+        } else {
+#pragma unroll 1
+            for (int b = b0; b < b1; ++b) {
+                const double mb = mass(b);
+                sm = __dadd_rn(sm, mb);
+                sx = __dadd_rn(sx, __dmul_rn(px[b], mb));
+                sy = __dadd_rn(sy, __dmul_rn(py[b], mb));
+                sz = __dadd_rn(sz, __dmul_rn(pz[b], mb));
+            }
+        }
+        ls[l] = double4_32a{sx, sy, sz, sm};
+        if (kMoments) {
+            double q = 0.0;
+            if (b1 - b0 > 1 && sm > 0) {
+                const double is = rcp_nr(sm);
+                const double cx = sx * is, cy = sy * is, cz = sz * is;
+#pragma unroll 1
+                for (int b = b0; b < b1; ++b) {
+                    const double dx = px[b] - cx, dy = py[b] - cy, dz = pz[b] - cz;
+                    q += mass(b) * (dx * dx + dy * dy + dz * dz);
+                }
+            }
+            lq[l] = q;
+        }
+    } else if (j == L) {
+        v = -1;  // right sentinel of the boundary pass
+        cdep[L] = -1;
+    }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wbase = (int)(j - lane);
     warp_threshold_ends(v, lane, wbase, wl[w], wf[w]);
@@ -254,13 +266,16 @@ __global__ void __launch_bounds__(1024) bnd_scan_kernel(int nblk, const int32_t*
 }
 
 // Per boundary: the representative flag (flag[j], 0 for j = 0 and j >= L up
-// to cap), pl, pr and next.
+// to cap), pl, pr and next; per block the number of representatives.
+// scanned: blast / bfirst hold bnd_scan_kernel's prefixes and suffixes; else
+// the blocks' own positions, which the block scans for itself.
 __global__ void __launch_bounds__(kBT) bnd_resolve_kernel(const int32_t* __restrict__ counts,
                                                           const int8_t* __restrict__ cdep,
-                                                          const int32_t* __restrict__ bpre,
-                                                          const int32_t* __restrict__ bsuf, int32_t* __restrict__ flag,
-                                                          int32_t* __restrict__ pl, int32_t* __restrict__ pr,
-                                                          int32_t* __restrict__ nxt, int64_t cap)
+                                                          const int32_t* __restrict__ blast,
+                                                          const int32_t* __restrict__ bfirst, int scanned,
+                                                          int32_t* __restrict__ flag, int32_t* __restrict__ pl,
+                                                          int32_t* __restrict__ pr, int32_t* __restrict__ nxt,
+                                                          int32_t* __restrict__ bsum, int64_t cap)
 {
     __shared__ int wl[kBW][kNT], wf[kBW][kNT];
     const int L = counts[0];
@@ -300,7 +315,19 @@ __global__ void __launch_bounds__(kBT) bnd_resolve_kernel(const int32_t* __restr
         }
         int ex = __shfl_up_sync(0xffffffffu, inc, 1);
         if (lane == 0) ex = -1;
-        wl[lane][t] = max(bpre[(int64_t)blockIdx.x * kNT + t], ex);
+        int before = -1, after = INT_MAX;
+        if (scanned) {
+            before = blast[(int64_t)blockIdx.x * kNT + t];
+            after = bfirst[(int64_t)blockIdx.x * kNT + t];
+        } else {
+            for (int b = lane; b < (int)gridDim.x; b += 32) {
+                if (b < (int)blockIdx.x) before = max(before, blast[b * kNT + t]);
+                if (b > (int)blockIdx.x) after = min(after, bfirst[b * kNT + t]);
+            }
+            before = __reduce_max_sync(0xffffffffu, before);
+            after = __reduce_min_sync(0xffffffffu, after);
+        }
+        wl[lane][t] = max(before, ex);
         int sinc = wf[lane][t];
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
@@ -309,10 +336,9 @@ __global__ void __launch_bounds__(kBT) bnd_resolve_kernel(const int32_t* __restr
         }
         int sex = __shfl_down_sync(0xffffffffu, sinc, 1);
         if (lane == 31) sex = INT_MAX;
-        wf[lane][t] = min(bsuf[(int64_t)blockIdx.x * kNT + t], sex);
+        wf[lane][t] = min(after, sex);
     }
     __syncthreads();
-    if (j >= cap) return;
     int f = 0;
     if (j >= 1 && j < L) {
         const unsigned below = (1u << lane) - 1u, above = ~below & ~(1u << lane);
@@ -330,54 +356,159 @@ __global__ void __launch_bounds__(kBT) bnd_resolve_kernel(const int32_t* __restr
         pr[j] = next(lt_m, v);
         nxt[j] = next(le_m, v + 1);
     }
-    flag[j] = f;
+    if (j < cap) flag[j] = f;
+    const int reps = __syncthreads_count(f);
+    if (threadIdx.x == 0) bsum[blockIdx.x] = reps;
 }
 
-// Each branching node from its representative: depth, leaf range and its
-// splits (at most 7) with their ranks; child count = splits + 1.
-__global__ void node_split_kernel(const int32_t* __restrict__ counts, const int8_t* __restrict__ cdep,
-                                  const int32_t* __restrict__ flag, const int32_t* __restrict__ excl,
-                                  const int32_t* __restrict__ pl, const int32_t* __restrict__ pr,
-                                  const int32_t* __restrict__ nxt, int32_t* __restrict__ node_rep,
-                                  int32_t* __restrict__ node_a, int32_t* __restrict__ node_e,
-                                  uint8_t* __restrict__ node_depth, int32_t* __restrict__ node_nchild,
-                                  int32_t* __restrict__ split_node, int8_t* __restrict__ split_rank,
-                                  unsigned* __restrict__ err)
+// Each branching node from its representative (a thread per boundary; node
+// ids count the representatives, so the blocks' numbers before come from
+// bnd_resolve_kernel's sums): depth, leaf range and its splits (at most 7)
+// with their ranks; child count = splits + 1, its first child's place among
+// the children of the block's nodes (cs), and the block's child count (csum).
+__global__ void __launch_bounds__(kBT) node_split_kernel(
+    int32_t* counts, const int8_t* __restrict__ cdep, const int32_t* __restrict__ flag,
+    const int32_t* __restrict__ bsum, const int32_t* __restrict__ pl, const int32_t* __restrict__ pr,
+    const int32_t* __restrict__ nxt, int32_t* __restrict__ rep_node, int32_t* __restrict__ node_rep,
+    int32_t* __restrict__ node_a, int32_t* __restrict__ node_e, uint8_t* __restrict__ node_depth,
+    int32_t* __restrict__ node_nchild, int32_t* __restrict__ split_node, int8_t* __restrict__ split_rank,
+    int32_t* __restrict__ cs, int32_t* __restrict__ csum, unsigned* __restrict__ err)
 {
+    static_assert(kBW == 32, "one lane per warp");
+    __shared__ int w_before[kBW], w_reps[kBW], w_children[kBW];
     const int L = counts[0];
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < L; j += gridDim.x * blockDim.x) {
-        if (j == 0 || !flag[j]) continue;
-        const int b = excl[j];
-        const int c = cdep[j];
-        node_rep[b] = j;
-        node_a[b] = pl[j];
-        node_e[b] = pr[j];
-        node_depth[b] = (uint8_t)c;
-        int k = j, r = 0;
-        for (;;) {
-            split_node[k] = b;
-            split_rank[k] = (int8_t)r;
-            ++r;
-            k = nxt[k];
-            if (k >= L || cdep[k] != c || r >= 7) break;
-        }
-        if (k < L && cdep[k] == c) atomicOr(err, kErrOverflow);  // an eighth split: impossible for an octree
-        node_nchild[b] = r + 1;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t jj = (int64_t)blockIdx.x * kBT + threadIdx.x;
+    const bool rep = jj >= 1 && jj < L && flag[jj];
+    const unsigned reps = __ballot_sync(0xffffffffu, rep);
+    int before = 0;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += kBT) before += bsum[k];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) {
+        w_before[w] = before;
+        w_reps[w] = __popc(reps);
     }
+    __syncthreads();
+    before = __reduce_add_sync(0xffffffffu, w_before[lane] + (lane < w ? w_reps[lane] : 0));
+    const int b = before + __popc(reps & ((1u << lane) - 1u));
+    int children = 0;
+    if (jj < L) {
+        const int j = (int)jj;
+        rep_node[j] = b;
+        if (rep) {
+            const int c = cdep[j];
+            node_rep[b] = j;
+            node_a[b] = pl[j];
+            node_e[b] = pr[j];
+            node_depth[b] = (uint8_t)c;
+            int k = j, r = 0;
+            for (;;) {
+                split_node[k] = b;
+                split_rank[k] = (int8_t)r;
+                ++r;
+                k = nxt[k];
+                if (k >= L || cdep[k] != c || r >= 7) break;
+            }
+            if (k < L && cdep[k] == c) atomicOr(err, kErrOverflow);  // an eighth split: impossible for an octree
+            children = r + 1;
+            node_nchild[b] = children;
+        }
+    }
+    int inc = children;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += y;
+    }
+    if (lane == 31) w_children[w] = inc;
+    __syncthreads();
+    const int ahead = __reduce_add_sync(0xffffffffu, lane < w ? w_children[lane] : 0);
+    if (rep) cs[b] = ahead + inc - children;
+    if (threadIdx.x == kBT - 1) {
+        csum[blockIdx.x] = ahead + inc;
+        if (blockIdx.x == gridDim.x - 1) counts[1] = b + (rep ? 1 : 0);
+    }
+}
+
+// The sum of the blocks' child counts before each block, for node_place_kernel
+// where its blocks don't form it for themselves; one block.
+__global__ void __launch_bounds__(1024) child_offset_kernel(int nb, int32_t* __restrict__ csum)
+{
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < nb; base += 1024) {
+        const int k = base + (int)threadIdx.x;
+        const int x = k < nb ? csum[k] : 0;
+        int inc = x;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += y;
+        }
+        if (lane == 31) wsum[w] = inc;
+        __syncthreads();
+        const int ahead = __reduce_add_sync(0xffffffffu, lane < w ? wsum[lane] : 0);
+        const int total = __reduce_add_sync(0xffffffffu, wsum[lane]);
+        if (k < nb) csum[k] = carry + ahead + inc - x;
+        carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) csum[nb] = carry;
 }
 
 // Child slots: every leaf and branching node finds its parent from the
 // boundaries at its two ends (the deeper one splits the parent; both
 // sentinels: the root) and its place among the parent's children from that
-// split's rank.  Slot 0 is the root.
-__global__ void node_place_kernel(const int32_t* __restrict__ counts, const int8_t* __restrict__ cdep,
-                                  const int32_t* __restrict__ node_a, const int32_t* __restrict__ node_e,
-                                  const uint8_t* __restrict__ node_depth, const int32_t* __restrict__ node_cs,
-                                  const int32_t* __restrict__ split_node, const int8_t* __restrict__ split_rank,
-                                  int32_t* __restrict__ slot_ref, uint8_t* __restrict__ slot_top,
-                                  unsigned* __restrict__ err)
+// split's rank.  Slot 0 is the root.  A node's first child slot (node_cs) is
+// its place in its block (cs) behind the children of the blocks before, which
+// every block here sums from csum first (kOffBlocks of them at most; beyond,
+// child_offset_kernel has).
+constexpr int kOffBlocks = 4096;
+
+__global__ void __launch_bounds__(kThreads) node_place_kernel(
+    int32_t* counts, const int8_t* __restrict__ cdep, const int32_t* __restrict__ node_a,
+    const int32_t* __restrict__ node_e, const uint8_t* __restrict__ node_depth, const int32_t* __restrict__ node_rep,
+    const int32_t* __restrict__ cs, const int32_t* __restrict__ csum, int nb, int32_t* __restrict__ node_cs,
+    const int32_t* __restrict__ split_node, const int8_t* __restrict__ split_rank, int32_t* __restrict__ slot_ref,
+    uint8_t* __restrict__ slot_top, unsigned* __restrict__ err)
 {
-    const int L = counts[0], B = counts[1], S = counts[2];
+    __shared__ int off_s[kOffBlocks];
+    __shared__ int wsum[kThreads / 32];
+    const bool own = nb <= kOffBlocks;
+    int total;
+    if (own) {
+        // Thread t takes the blocks [t q, t q + q).
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        const int q = (nb + kThreads - 1) / kThreads, k0 = (int)threadIdx.x * q, k1 = min(k0 + q, nb);
+        int sum = 0;
+        for (int k = k0; k < k1; ++k) sum += csum[k];
+        int inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (lane == 31) wsum[w] = inc;
+        __syncthreads();
+        int run = inc - sum;
+        total = 0;
+        for (int k = 0; k < kThreads / 32; ++k) {
+            if (k < w) run += wsum[k];
+            total += wsum[k];
+        }
+        for (int k = k0; k < k1; ++k) {
+            off_s[k] = run;
+            run += csum[k];
+        }
+        __syncthreads();
+    } else {
+        total = csum[nb];
+    }
+    const int* off = own ? off_s : csum;
+    const auto first_child = [&](int b) { return cs[b] + off[node_rep[b] / kBT]; };
+    const int L = counts[0], B = counts[1], S = total + 1;  // the root and every child
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[2] = S;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L + B; i += gridDim.x * blockDim.x) {
         int a, e, ref;
         if (i < L) {
@@ -385,6 +516,7 @@ __global__ void node_place_kernel(const int32_t* __restrict__ counts, const int8
         } else {
             const int b = i - L;
             a = node_a[b]; e = node_e[b]; ref = ~b;
+            node_cs[b] = first_child(b);
         }
         const int ca = a == 0 ? -1 : cdep[a];
         const int ce = e >= L ? -1 : cdep[e];
@@ -397,7 +529,7 @@ __global__ void node_place_kernel(const int32_t* __restrict__ counts, const int8
                 atomicOr(err, kErrOverflow);
                 continue;
             }
-            s = node_cs[P] + 1 + split_rank[k] + (left ? 1 : 0);
+            s = first_child(P) + 1 + split_rank[k] + (left ? 1 : 0);
             top = node_depth[P] + 1;
             if (s < 1 || s >= S) {
                 atomicOr(err, kErrOverflow);
@@ -973,16 +1105,6 @@ __global__ void finalize_kernel(const int32_t* __restrict__ counts, const int32_
     }
 }
 
-__global__ void slot_count_kernel(int32_t* counts, const int32_t* __restrict__ child_total)
-{
-    // S = 1 (root) + every child slot.
-    counts[2] = 1 + *child_total;
-}
-
-}  // namespace
-
-namespace {
-
 template <bool kMoments>
 int launch_monopoles(bh_context* ctx)
 {
@@ -1034,53 +1156,51 @@ int launch_build(bh_context* ctx, const double* mass, bool moments, bool far_fus
     if (n == 0) return BH_OK;
     cudaStream_t st = ctx->stream;
     const int maxb = 8 * bh::num_sms();
-    const int g = grid_for(n, kThreads, maxb);
 
     // 1. leaves: ids, first bodies and keys from a scan of the keys' head flags
     int rc = device_number_leaves(ctx, ctx->key, n, ctx->counts + 0, ctx->body_leaf, ctx->leaf_first, ctx->leaf_key);
     if (rc) return rc;
-    if (moments)
-        leaf_sum_kernel<true><<<g, kThreads, 0, st>>>(ctx->counts, ctx->leaf_first, ctx->leaf_key, ctx->px, ctx->py,
-                                                      ctx->pz, mass, ctx->id, nzero, ctx->leaf_s, ctx->cdep,
-                                                      ctx->leaf_q);
-    else
-        leaf_sum_kernel<false><<<g, kThreads, 0, st>>>(ctx->counts, ctx->leaf_first, ctx->leaf_key, ctx->px, ctx->py,
-                                                       ctx->pz, mass, ctx->id, nzero, ctx->leaf_s, ctx->cdep,
-                                                       ctx->leaf_q);
-    BH_LAUNCH_CHECK(ctx);
 
-    // 2. branching nodes: the boundary pass (representative flags, node
-    // ranges, split chains) -> node ids -> child counts -> child slots
-    {
-        const int nb = (int)((n + 1 + kBT - 1) / kBT);
-        int32_t* blast = ctx->ansv_blk;
-        int32_t* bfirst = blast + (int64_t)nb * kNT;
-        int32_t* bpre = bfirst + (int64_t)nb * kNT;
-        int32_t* bsuf = bpre + (int64_t)nb * kNT;
-        bnd_summary_kernel<<<nb, kBT, 0, st>>>(ctx->counts, ctx->cdep, blast, bfirst);
-        BH_LAUNCH_CHECK(ctx);
+    // 2. leaf sums and branching nodes: the boundary pass (representative
+    // flags, node ranges, split chains) -> node ids and child counts -> slots
+    const int nb = (int)((n + 1 + kBT - 1) / kBT);
+    int32_t* blast = ctx->ansv_blk;
+    int32_t* bfirst = blast + (int64_t)nb * kNT;
+    int32_t* bpre = bfirst + (int64_t)nb * kNT;
+    int32_t* bsuf = bpre + (int64_t)nb * kNT;
+    int32_t* bsum = ctx->scan_tmp;
+    int32_t* csum = blast;  // free after the boundary pass; nb + 1
+    int32_t* cs = reinterpret_cast<int32_t*>(ctx->perm_alt);  // free after the sort
+    if (moments)
+        leaf_bnd_kernel<true><<<nb, kBT, 0, st>>>(ctx->counts, ctx->leaf_first, ctx->leaf_key, ctx->px, ctx->py, ctx->pz,
+                                                  mass, ctx->id, nzero, ctx->leaf_s, ctx->cdep, ctx->leaf_q, blast,
+                                                  bfirst);
+    else
+        leaf_bnd_kernel<false><<<nb, kBT, 0, st>>>(ctx->counts, ctx->leaf_first, ctx->leaf_key, ctx->px, ctx->py, ctx->pz,
+                                                   mass, ctx->id, nzero, ctx->leaf_s, ctx->cdep, ctx->leaf_q, blast,
+                                                   bfirst);
+    BH_LAUNCH_CHECK(ctx);
+    const bool scanned = nb > kDirectBlocks;
+    if (scanned) {
         bnd_scan_kernel<<<2 * kNT, 1024, 0, st>>>(nb, blast, bfirst, bpre, bsuf);
         BH_LAUNCH_CHECK(ctx);
-        bnd_resolve_kernel<<<nb, kBT, 0, st>>>(ctx->counts, ctx->cdep, bpre, bsuf, ctx->head, ctx->bnd_pl, ctx->bnd_pr,
-                                                ctx->bnd_next, n);
+    }
+    bnd_resolve_kernel<<<nb, kBT, 0, st>>>(ctx->counts, ctx->cdep, scanned ? bpre : blast, scanned ? bsuf : bfirst,
+                                           scanned ? 1 : 0, ctx->head, ctx->bnd_pl, ctx->bnd_pr, ctx->bnd_next, bsum,
+                                           n);
+    BH_LAUNCH_CHECK(ctx);
+    node_split_kernel<<<nb, kBT, 0, st>>>(ctx->counts, ctx->cdep, ctx->head, bsum, ctx->bnd_pl, ctx->bnd_pr,
+                                          ctx->bnd_next, ctx->rep_node, ctx->node_rep, ctx->node_a, ctx->node_e,
+                                          ctx->node_depth, ctx->node_nchild, ctx->split_node, ctx->split_rank, cs,
+                                          csum, ctx->err);
+    BH_LAUNCH_CHECK(ctx);
+    if (nb > kOffBlocks) {
+        child_offset_kernel<<<1, 1024, 0, st>>>(nb, csum);
         BH_LAUNCH_CHECK(ctx);
     }
-    // rep_node[j] = exclusive count of representatives before j, i.e. the
-    // node id of boundary j when it is a representative.
-    rc = device_exclusive_scan(ctx, ctx->head, ctx->rep_node, n, nullptr, ctx->counts + 1);
-    if (rc) return rc;
-    node_split_kernel<<<g, kThreads, 0, st>>>(ctx->counts, ctx->cdep, ctx->head, ctx->rep_node, ctx->bnd_pl,
-                                              ctx->bnd_pr, ctx->bnd_next, ctx->node_rep, ctx->node_a, ctx->node_e,
-                                              ctx->node_depth, ctx->node_nchild, ctx->split_node, ctx->split_rank,
-                                              ctx->err);
-    BH_LAUNCH_CHECK(ctx);
-    rc = device_exclusive_scan(ctx, ctx->node_nchild, ctx->node_cs, n, ctx->counts + 1, ctx->counts + 3);
-    if (rc) return rc;
-    slot_count_kernel<<<1, 1, 0, st>>>(ctx->counts, ctx->counts + 3);
-    BH_LAUNCH_CHECK(ctx);
     node_place_kernel<<<grid_for(2 * n, kThreads, maxb), kThreads, 0, st>>>(
-        ctx->counts, ctx->cdep, ctx->node_a, ctx->node_e, ctx->node_depth, ctx->node_cs, ctx->split_node,
-        ctx->split_rank, ctx->slot_ref, ctx->slot_top, ctx->err);
+        ctx->counts, ctx->cdep, ctx->node_a, ctx->node_e, ctx->node_depth, ctx->node_rep, cs, csum, nb, ctx->node_cs,
+        ctx->split_node, ctx->split_rank, ctx->slot_ref, ctx->slot_top, ctx->err);
     BH_LAUNCH_CHECK(ctx);
 
     // 3./4. monopoles (and second moments): chunks of leaves, then what reaches
