@@ -5,9 +5,9 @@
 // index-sorts with std::sort and gathers pos/mass/vel/ids/keys; here the
 // sort is a stable 8-pass LSD radix sort (8-bit digits) whose digit
 // histograms for all passes come from the key kernel, and each pass is one
-// kernel: tiles claim an id in launch order, rank their keys with warp
-// ballots (one per digit bit), publish per-digit tile counts, and obtain their
-// global offsets by a decoupled look-back over earlier tiles.  Every wait
+// kernel: tiles claim an id in launch order, rank their keys warp by warp,
+// publish per-digit tile counts, and obtain their global offsets by a decoupled
+// look-back over earlier tiles.  Every wait
 // in the look-back is bounded; on expiry the kernel raises kErrTimeout
 // and still publishes, so no tile can wait forever.
 //
@@ -27,10 +27,12 @@ constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagIncl = 2u << 30;
 constexpr uint32_t kCountMask = (1u << 30) - 1;
 constexpr int kSpinLimit = 1 << 22;
-constexpr int kBatch = 8;  // look-back: predecessors read per round
+constexpr int kBatch = 4;  // look-back: predecessors read per round
 
 struct SortSmem {
     uint32_t warp_hist[kWarps][kRadix];  // per-warp digit counts, then warp prefixes
+    uint32_t warp_mask[kWarps][kRadix];  // lanes per digit, for rank_item
+    uint32_t tile_hist[kRadix];          // the tile's digit counts
     uint32_t digit_excl[kRadix];         // tile-local start of each digit
     uint32_t global_base[kRadix];        // global start minus tile-local start
     uint32_t scan[kRadix / 32];
@@ -39,10 +41,37 @@ struct SortSmem {
     uint32_t vals[kSortTile];
 };
 
-// Exclusive scan over 256 values held one per thread by threads 0..255.
+// One item of a warp's ranking: the lane's rank among the warp's keys of its
+// digit so far, and its digit's count moved on.  Every lane sets its bit in the
+// digit's word of `mask` (zero before and after) and reads there which lanes
+// hold the same digit.  (A ballot per digit bit does without the words, but a
+// vote takes the SM about four cycles: 64 of them a thread bounded the ranking,
+// 4,400 cycles a tile.)
+template <typename Count>
+__device__ __forceinline__ uint32_t rank_item(uint32_t d, bool valid, unsigned lt, int lane, uint32_t* mask,
+                                              Count* hist)
+{
+    if (valid) atomicOr(&mask[d], 1u << lane);
+    __syncwarp();
+    uint32_t peers = 0, old = 0;
+    if (valid) {
+        peers = mask[d];
+        old = hist[d];
+    }
+    __syncwarp();
+    if (valid && (peers & lt) == 0u) {  // the lowest peer
+        mask[d] = 0;
+        hist[d] = (Count)(old + __popc(peers));
+    }
+    __syncwarp();
+    return old + __popc(peers & lt);
+}
+
+// Exclusive scan over 256 values held one per thread by 8 consecutive warps,
+// the first 256 threads of a block or those from a multiple of 256 on.
 __device__ uint32_t scan256(uint32_t v, uint32_t* tmp)
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 7;
     uint32_t x = v;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -67,8 +96,18 @@ __global__ void hist_scan_kernel(uint32_t* __restrict__ hist)
     h[threadIdx.x] = e;
 }
 
+// 16 warps rank the tile's keys and put them in order in shared memory; 8 more
+// publish its digit counts and look back while they do.  Latency bounds a tile:
+// what its successors wait for is kept short (no fence, since a flag and its
+// count are one word; four predecessors a round, where 8 read more that is not
+// there yet: 135 and 128 us at 1M).  Sort phase per step with one set of warps,
+// ballots for the ranking and a fence, and now: 100,000 keys 96 -> 84 us,
+// 300,149 110 -> 93, 1M 173 -> 128, 4M 420 -> 332.
+constexpr int kLookThreads = kRadix;  // a thread per digit
+constexpr int kTileThreads = kSortThreads + kLookThreads;
+
 template <bool kFirst>
-__global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
+__global__ void __launch_bounds__(kTileThreads, 2) onesweep_kernel(
     int64_t n, int shift, const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, const uint32_t* __restrict__ bucket_start,
     uint32_t* lookback, uint32_t* tile_ctr, unsigned* err)
@@ -76,87 +115,82 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SortSmem& s = *reinterpret_cast<SortSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool ranks = threadIdx.x < kSortThreads;
 
     if (threadIdx.x == 0) s.tile = atomicAdd(tile_ctr, 1u);
-    for (int k = threadIdx.x; k < kWarps * kRadix; k += kSortThreads) (&s.warp_hist[0][0])[k] = 0;
+    for (int k = threadIdx.x; k < (2 * kWarps + 1) * kRadix; k += kTileThreads) (&s.warp_hist[0][0])[k] = 0;
     __syncthreads();
     const uint32_t tile = s.tile;
     const int64_t base = (int64_t)tile * kSortTile;
+    const int64_t rem = n - base;
+    const int cnt = rem < kSortTile ? (int)rem : kSortTile;
 
-    // Load: warp w owns keys [w*256, w*256+256) of the tile, item k at lane l
-    // is key w*256 + k*32 + l, so (w, k, l) is the input order.
+    // Warp w owns keys [w*256, w*256+256) of the tile, item k at lane l is
+    // key w*256 + k*32 + l, so (w, k, l) is the input order.
     uint64_t key[kSortItems];
-    uint32_t val[kSortItems];
-    uint32_t rank[kSortItems];
-#pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const int64_t i = base + w * (32 * kSortItems) + k * 32 + lane;
-        if (i < n) {
-            key[k] = keys_in[i];
-            val[k] = kFirst ? (uint32_t)i : vals_in[i];
-        } else {
-            key[k] = ~0ull;
-            val[k] = 0;
-        }
-    }
-
-    // Rank within the warp: peers holding the same digit are found with one
-    // ballot per digit bit (a fixed cost; match.any takes longer the more
-    // distinct digits a warp holds, as in the low passes); the lowest peer
-    // bumps the warp's digit counter once.
+    uint32_t val[kSortItems], rank[kSortItems / 2] = {};  // rank: 16 bits an item
     const unsigned lt = (1u << lane) - 1u;
+    const int first = w * (32 * kSortItems) + lane;
+    if (ranks) {
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const int64_t i = base + w * (32 * kSortItems) + k * 32 + lane;
-        const bool valid = i < n;
-        const uint32_t d = valid ? (uint32_t)((key[k] >> shift) & 0xFF) : 0u;
-        // lanes past the end form their own peer set, apart from every digit
-        const unsigned vb = __ballot_sync(0xffffffffu, valid);
-        unsigned peers = valid ? vb : ~vb;
+        for (int k = 0; k < kSortItems; ++k) key[k] = first + k * 32 < cnt ? keys_in[base + first + k * 32] : ~0ull;
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const bool bit = (d >> b) & 1u;
-            const unsigned v = __ballot_sync(0xffffffffu, bit);
-            peers &= bit ? v : ~v;
-        }
-        const int leader = __ffs(peers) - 1;
-        uint32_t old = 0;
-        if (valid && lane == leader) {
-            old = s.warp_hist[w][d];
-            s.warp_hist[w][d] = old + __popc(peers);
-        }
-        old = __shfl_sync(0xffffffffu, old, leader);
-        rank[k] = old + __popc(peers & lt);
-        __syncwarp();
-    }
-    __syncthreads();
-
-    // Per digit: exclusive prefix over warps and the tile's total count.
-    uint32_t tile_count = 0;
-    if (threadIdx.x < kRadix) {
-        const int d = threadIdx.x;
-        uint32_t run = 0;
-        for (int ww = 0; ww < kWarps; ++ww) {
-            const uint32_t c = s.warp_hist[ww][d];
-            s.warp_hist[ww][d] = run;
+        for (int k = 0; k < kSortItems; ++k)
+            rank[k / 2] |= rank_item((uint32_t)(key[k] >> shift) & 0xFFu, first + k * 32 < cnt, lt, lane,
+                                     s.warp_mask[w], s.warp_hist[w])
+                           << 16 * (k & 1);
+#pragma unroll
+        for (int k = 0; k < kSortItems; ++k)
+            val[k] = kFirst ? (uint32_t)base + first + k * 32 : first + k * 32 < cnt ? vals_in[base + first + k * 32] : 0;
+        asm volatile("bar.sync 2, %0;" ::"n"(kSortThreads));
+        // Two threads per digit: exclusive prefix over the warps.
+        const int d = threadIdx.x >> 1, h = threadIdx.x & 1;
+        uint32_t sum = 0;
+#pragma unroll
+        for (int k = 0; k < kWarps / 2; ++k) sum += s.warp_hist[h * (kWarps / 2) + k][d];
+        uint32_t run = __shfl_up_sync(0xffffffffu, sum, 1);
+        if (h == 0) run = 0;
+#pragma unroll
+        for (int k = 0; k < kWarps / 2; ++k) {
+            const uint32_t c = s.warp_hist[h * (kWarps / 2) + k][d];
+            s.warp_hist[h * (kWarps / 2) + k][d] = run;
             run += c;
         }
-        tile_count = run;
+        if (h == 1) s.tile_hist[d] = run;
+    }
+    __syncthreads();
+    if (ranks) {
+        // ... and the digits' starts from the other warps.
+        asm volatile("bar.sync 3, %0;" ::"n"(kTileThreads));
+        // Into shared memory in tile-sorted order.
+#pragma unroll
+        for (int k = 0; k < kSortItems; ++k) {
+            if (first + k * 32 < cnt) {
+                const uint32_t d = (uint32_t)(key[k] >> shift) & 0xFFu;
+                const uint32_t p = s.digit_excl[d] + s.warp_hist[w][d] + (rank[k / 2] >> 16 * (k & 1) & 0xFFFFu);
+                if (p < (uint32_t)kSortTile) {
+                    s.keys[p] = key[k];
+                    s.vals[p] = val[k];
+                }
+            }
+        }
+    } else {
+        // Decoupled look-back: thread d sums earlier tiles' counts of digit d,
+        // reading kBatch predecessors per round (independent loads in flight)
+        // and stopping at the nearest inclusive prefix.  A predecessor that
+        // has not published yet is read again (bounded).
+        const int d = threadIdx.x - kSortThreads;
+        const uint32_t tile_count = s.tile_hist[d];
         volatile uint32_t* lb = lookback + (size_t)tile * kRadix;
         lb[d] = (tile == 0 ? kFlagIncl : kFlagAgg) | tile_count;
-        s.digit_excl[d] = scan256(tile_count, s.scan);
-    }
-
-    // Decoupled look-back: thread d sums earlier tiles' counts of digit d,
-    // reading kBatch predecessors per round (independent loads in flight)
-    // and stopping at the nearest inclusive prefix.  A predecessor that has
-    // not published yet is read again (bounded).
-    if (threadIdx.x < kRadix) {
-        const int d = threadIdx.x;
+        const uint32_t bucket = bucket_start[d];
+        const uint32_t start = scan256(tile_count, s.scan);
+        s.digit_excl[d] = start;
+        asm volatile("bar.arrive 3, %0;" ::"n"(kTileThreads) : "memory");
         uint32_t excl = 0;
         if (tile > 0) {
             const volatile uint32_t* lbv = lookback;
-            int64_t k = (int64_t)tile - 1;
+            int k = (int)tile - 1;
             int spins = 0;
             while (k >= 0) {
                 uint32_t v[kBatch];
@@ -183,34 +217,16 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
                         atomicOr(err, kErrTimeout);
                         break;
                     }
-                    __nanosleep(32);
                 }
                 k -= used;
             }
-            __threadfence();
-            ((volatile uint32_t*)lookback)[(size_t)tile * kRadix + d] = kFlagIncl | ((excl + tile_count) & kCountMask);
+            // (flag and count are one word: nothing to order it with)
+            lb[d] = kFlagIncl | ((excl + tile_count) & kCountMask);
         }
-        s.global_base[d] = bucket_start[d] + excl - s.digit_excl[d];
+        s.global_base[d] = bucket + excl - start;
     }
     __syncthreads();
-
-    // Scatter into shared memory in tile-sorted order, then write out.
-#pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const int64_t i = base + w * (32 * kSortItems) + k * 32 + lane;
-        if (i < n) {
-            const uint32_t d = (uint32_t)((key[k] >> shift) & 0xFF);
-            const uint32_t p = s.digit_excl[d] + s.warp_hist[w][d] + rank[k];
-            if (p < (uint32_t)kSortTile) {
-                s.keys[p] = key[k];
-                s.vals[p] = val[k];
-            }
-        }
-    }
-    __syncthreads();
-    const int64_t rem = n - base;
-    const int cnt = rem < kSortTile ? (int)rem : kSortTile;
-    for (int j = threadIdx.x; j < cnt; j += kSortThreads) {
+    for (int j = threadIdx.x; j < cnt; j += kTileThreads) {
         const uint64_t kk = s.keys[j];
         const uint32_t d = (uint32_t)((kk >> shift) & 0xFF);
         const uint32_t g = s.global_base[d] + (uint32_t)j;
@@ -233,11 +249,11 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
 // equal there share a cell of the tenth level, so in most sets few are left to
 // order: runs of equal high bits up to kTieRun long are ordered by insertion (stable, as the passes
 // are), and a set with a longer run is sorted again by all eight digits.
-// Sort phase per step, before -> after: 1,000 keys 71 -> 15 us, 19,054 92 -> 31,
-// 65,536 95 -> 49 (68 with 8 blocks, 79 with key and payload as two words).
-// At the large end the remote stores (a block's 4,096 words in 2.3 us a pass)
-// and the ranking (1.9) bound it; staging a pass's words in digit order before
-// they leave the block gained nothing.
+// Sort phase per step, before -> after: 1,000 keys 71 -> 15 us, 19,054 92 -> 29,
+// 65,536 95 -> 47 (68 with 8 blocks, 79 with key and payload as two words).
+// At the large end the remote stores bound it (a block's 4,096 words in 2.3 us
+// a pass); staging a pass's words in digit order before they leave the block
+// gained nothing.
 constexpr int kCThreads = 1024;
 constexpr int kCWarps = kCThreads / 32;
 constexpr int kCMax = 16;      // blocks, where the device takes clusters beyond the portable 8
@@ -248,6 +264,7 @@ constexpr int kHistRow = kRadix + 2;  // 129 words: the four quarters of a digit
 struct ClusterSmem {
     uint64_t words[kClusterSortMax / kCPortable];  // 32 bits of the key over the key's index
     uint16_t warp_hist[kCWarps][kHistRow];
+    uint32_t warp_mask[kCWarps][kRadix];
     uint32_t totals[kCMax][kRadix];  // every block's digit counts
     uint32_t base[kRadix];           // where the block's keys of a digit go
     uint32_t scan[kRadix / 32];
@@ -289,6 +306,7 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
         return e - g;
     };
 
+    for (int k = threadIdx.x; k < kCWarps * kRadix; k += kCThreads) (&s.warp_mask[0][0])[k] = 0;
     // Round 0 sorts by the high halves; rounds 1 and 2, where needed, by the
     // low and then by the high halves.
     for (int round = 0; round < 3; ++round) {
@@ -314,24 +332,10 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
             for (int k = lane; k < kHistRow / 2; k += 32) reinterpret_cast<uint32_t*>(s.warp_hist[w])[k] = 0;
             __syncwarp();
 #pragma unroll
-            for (int k = 0; k < I; ++k) {
-                const bool valid = w * (32 * I) + k * 32 + lane < cnt;
-                const uint32_t d = (uint32_t)(word[k] >> shift) & 0xFFu;
-                const unsigned vb = __ballot_sync(0xffffffffu, valid);
-                unsigned peers = valid ? vb : ~vb;
-#pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    const bool bit = (d >> b) & 1u;
-                    const unsigned v = __ballot_sync(0xffffffffu, bit);
-                    peers &= bit ? v : ~v;
-                }
-                // every peer reads the count before the lowest one bumps it
-                const uint32_t old = s.warp_hist[w][d];
-                __syncwarp();
-                if (valid && (peers & lt) == 0u) s.warp_hist[w][d] = (uint16_t)(old + __popc(peers));
-                rank[k] = (uint16_t)(old + __popc(peers & lt));
-                __syncwarp();
-            }
+            for (int k = 0; k < I; ++k)
+                rank[k] = (uint16_t)rank_item((uint32_t)(word[k] >> shift) & 0xFFu,
+                                              w * (32 * I) + k * 32 + lane < cnt, lt, lane, s.warp_mask[w],
+                                              s.warp_hist[w]);
             __syncthreads();
             {
                 // Four threads per digit: exclusive prefix over the warps,
@@ -539,10 +543,10 @@ int launch_sort(bh_context* ctx)
     for (int p = 0; p < kSortPasses; ++p) {
         uint32_t* lb = ctx->lookback + (size_t)p * tiles * kRadix;
         if (p == 0)
-            onesweep_kernel<true><<<(unsigned)tiles, kSortThreads, smem, ctx->stream>>>(
+            onesweep_kernel<true><<<(unsigned)tiles, kTileThreads, smem, ctx->stream>>>(
                 n, 8 * p, kin, vin, kout, vout, ctx->hist + p * kRadix, lb, ctx->tile_ctr + p, ctx->err);
         else
-            onesweep_kernel<false><<<(unsigned)tiles, kSortThreads, smem, ctx->stream>>>(
+            onesweep_kernel<false><<<(unsigned)tiles, kTileThreads, smem, ctx->stream>>>(
                 n, 8 * p, kin, vin, kout, vout, ctx->hist + p * kRadix, lb, ctx->tile_ctr + p, ctx->err);
         BH_LAUNCH_CHECK(ctx);
         uint64_t* tk = kin; kin = kout; kout = tk;
@@ -575,10 +579,10 @@ int sort_passes_raw(int64_t n, const uint64_t* keys_in, uint64_t* keys_out, uint
         uint32_t* vout = to_out ? vals_out : val_alt;
         uint32_t* lb = lookback + (size_t)p * tiles * kRadix;
         if (p == 0)
-            onesweep_kernel<true><<<(unsigned)tiles, kSortThreads, smem, stream>>>(
+            onesweep_kernel<true><<<(unsigned)tiles, kTileThreads, smem, stream>>>(
                 n, 8 * p, kin, vin, kout, vout, hist + p * kRadix, lb, tile_ctr + p, err);
         else
-            onesweep_kernel<false><<<(unsigned)tiles, kSortThreads, smem, stream>>>(
+            onesweep_kernel<false><<<(unsigned)tiles, kTileThreads, smem, stream>>>(
                 n, 8 * p, kin, vin, kout, vout, hist + p * kRadix, lb, tile_ctr + p, err);
         BH_CUDA_TRY(cudaGetLastError());
         kin = kout;
