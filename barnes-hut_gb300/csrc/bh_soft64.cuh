@@ -108,9 +108,18 @@ BH_SOFT float small_float_s(int v) { return float_of(0x4B400000u + (uint32_t)v) 
 BH_SOFT int small_round_s(float f) { return (int)(bits_of(f + 12582912.0f) - 0x4B400000u); }      // |f| < 2^22
 
 // The estimate of 1/sqrt(f) everything below starts from: within 2^-22.
+// (f is far from subnormal; rsqrtf puts a scaling for those around it.)
+#ifdef __CUDACC__
+__device__ __forceinline__ float rsqrt_hw(float f)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
+    return y;
+}
+#endif
 #ifndef BH_SOFT_RSQRT
 #ifdef __CUDA_ARCH__
-#define BH_SOFT_RSQRT(f) rsqrtf(f)
+#define BH_SOFT_RSQRT(f) rsqrt_hw(f)
 #else
 #define BH_SOFT_RSQRT(f) (1.0f / std::sqrt(f))
 #endif

@@ -31,7 +31,7 @@
 //
 // Measured (theta 1.05, ms of forces; before: one node per pass, 32 bodies
 // per warp, IEEE operations on the FP64 pipe):
-//   300,149 bodies 12.66 -> 2.90, 19,054 7.71 -> 1.21, 1,000 1.23 -> 0.071.
+//   300,149 bodies 12.66 -> 2.86, 19,054 7.71 -> 1.15, 1,000 1.23 -> 0.071.
 #include <climits>
 
 #include "bh_internal.cuh"
@@ -141,9 +141,10 @@ __device__ __noinline__ double ieee_scale(double dx, double dy, double dz, doubl
 
 // One interaction term with the reference's rounding (src/traversal.cpp:
 // 80-88): displacement, r^2 and the three products sc d.
-template <bool kSoft>
+// `beside`: work that does not depend on it, done in its waits.
+template <bool kSoft, typename F>
 __device__ __forceinline__ void exact_term(const double4_32a& r, double px, double py, double pz, double soft2,
-                                           bool on, double one, double& tx, double& ty, double& tz)
+                                           bool on, double one, double& tx, double& ty, double& tz, F beside)
 {
     const double dx = fma(r.x, one, -px), dy = fma(r.y, one, -py), dz = fma(r.z, one, -pz);
     // One of the three squares on the integer pipes balances them with the
@@ -151,6 +152,7 @@ __device__ __forceinline__ void exact_term(const double4_32a& r, double px, doub
     const double zz = soft::square(soft::bits_of(dz));
     double r2 = fma(fma(__dmul_rn(dx, dx), one, __dmul_rn(dy, dy)), one, zz);
     if (kSoft) r2 = fma(r2, one, soft2);
+    beside();
     if (!soft::term(dx, dy, dz, r2, r.w, tx, ty, tz) && on) {
         const double sc = ieee_scale(dx, dy, dz, soft2, r.w);
         tx = __dmul_rn(sc, dx);
@@ -223,34 +225,36 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
     int64_t passes = 0;
 
     // Evaluates the bodies' lists in order until none holds more than `left`
-    // entries.  P lanes evaluate P consecutive terms of a body; the sums run
-    // over them one after the other.
+    // entries.  P lanes evaluate P consecutive terms of a body.  The sums run
+    // over them one after the other, each waiting for the one before (about
+    // 100 cycles), so they take the terms of the step before while the next
+    // ones are evaluated (19,054 bodies 1.18 -> 1.15 ms, 8,000 0.46 -> 0.42).
+    auto T = sm.term[w];
+    const double* const sums = &T[lane < 3 * kBodies ? lane / kBodies : 2][lane % kBodies * P];
+    T[0][lane] = T[1][lane] = T[2][lane] = 0.0;
+    __syncwarp();
+    auto add = [&] {
+#pragma unroll
+        for (int k = 0; k < P; ++k) sum = fma(sum, one, sums[k]);
+    };
     auto flush = [&](int left) {
         int most = cnt - done;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
-        const int sum_body = lane % kBodies;
         for (; most > left; most -= P) {
             const int q = done + phase;
             const bool on = q < cnt;
             const double4_32a r = p.tree.d4[on ? PL[q & (Smem::kCap - 1)][body] : 0];
             double tx, ty, tz;
-            exact_term<kSoft>(r, px, py, pz, soft2, on, one, tx, ty, tz);
-            auto T = sm.term[w];
-            T[0][lane] = tx;
-            T[1][lane] = ty;
-            T[2][lane] = tz;
-            const int terms = __shfl_sync(0xffffffffu, cnt - done, sum_body * P);
-            if (lane < 3 * kBodies) {
-                const double* t = &T[lane / kBodies][sum_body * P];
-#pragma unroll
-                for (int k = 0; k < P; ++k)
-                    if (k < terms) sum = fma(sum, one, t[k]);
-            }
+            exact_term<kSoft>(r, px, py, pz, soft2, on, one, tx, ty, tz, add);
+            __syncwarp();
+            // (a sum is never -0, so adding +0 leaves it as it is)
+            T[0][lane] = on ? tx : 0.0;
+            T[1][lane] = on ? ty : 0.0;
+            T[2][lane] = on ? tz : 0.0;
             __syncwarp();
             done = min(done + P, cnt);
         }
-        __syncwarp();
     };
 
     while (sp > 0) {
@@ -409,6 +413,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
         __syncwarp();
     }
     flush(0);
+    add();
     if (overflow && lane == 0) atomicOr(p.err, kErrOverflow);
     if (lane < 3 * kBodies) {
         const int c = lane / kBodies;
@@ -478,9 +483,9 @@ int launch_exact_walk(bh_context* ctx, const ExactTree& tree, double theta, doub
     // Lanes to a body: 4 (the evaluation's sums fill 24 lanes and the bodies
     // share a walk) while that gives the chip 12 warps per SM, and more below,
     // where a warp's own latency counts.  Forces in ms with 4 / 8 / 16 / 32
-    // lanes: 300,149 bodies 2.96 / 3.67 / 5.36 / -, 19,054 1.21 / 1.26 / 1.39 /
-    // -, 8,000 0.69 / 0.46 / - / -, 4,000 0.44 / 0.29 / 0.23 / 0.25, 1,000
-    // 0.20 / 0.13 / 0.095 / 0.070.
+    // lanes: 300,149 bodies 2.86 / 3.67 / 5.36 / -, 19,054 1.15 / 1.18 / 1.30 /
+    // 2.19, 8,000 0.65 / 0.42 / 0.42 / 0.72, 4,000 0.41 / 0.27 / 0.21 / 0.28,
+    // 1,000 0.19 / 0.12 / 0.086 / 0.071.
     const int64_t want = 12 * (int64_t)num_sms() * 32;
     if (n * 4 >= want) return launch_exact_p<4>(ctx, p);
     if (n * 8 >= want) return launch_exact_p<8>(ctx, p);
