@@ -31,7 +31,7 @@
 //
 // Measured (theta 1.05, ms of forces; before: one node per pass, 32 bodies
 // per warp, IEEE operations on the FP64 pipe):
-//   300,149 bodies 12.66 -> 2.86, 19,054 7.71 -> 1.15, 1,000 1.23 -> 0.071.
+//   300,149 bodies 12.66 -> 2.86, 19,054 7.71 -> 1.12, 1,000 1.23 -> 0.071.
 #include <climits>
 
 #include "bh_internal.cuh"
@@ -161,7 +161,7 @@ __device__ __forceinline__ void exact_term(const double4_32a& r, double px, doub
     }
 }
 
-template <int P, bool kSoft>
+template <int P, bool kSoft, bool kAhead>
 __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams p)
 {
     using Smem = ExactSmem<P>;
@@ -241,10 +241,14 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
         int most = cnt - done;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
+        auto record = [&](int q) { return p.tree.d4[q < cnt ? PL[q & (Smem::kCap - 1)][body] : 0]; };
+        double4_32a next;
+        if (kAhead) next = record(done + phase);
         for (; most > left; most -= P) {
             const int q = done + phase;
             const bool on = q < cnt;
-            const double4_32a r = p.tree.d4[on ? PL[q & (Smem::kCap - 1)][body] : 0];
+            const double4_32a r = kAhead ? next : record(q);
+            if (kAhead) next = record(q + P);
             double tx, ty, tz;
             exact_term<kSoft>(r, px, py, pz, soft2, on, one, tx, ty, tz, add);
             __syncwarp();
@@ -435,10 +439,10 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
     }
 }
 
-template <int P, bool kSoft>
+template <int P, bool kSoft, bool kAhead>
 int launch_exact(bh_context* ctx, const TravParams& p)
 {
-    auto kernel = traverse_exact_kernel<P, kSoft>;
+    auto kernel = traverse_exact_kernel<P, kSoft, kAhead>;
     const size_t smem = sizeof(ExactSmem<P>);
     BH_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     BH_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -451,10 +455,10 @@ int launch_exact(bh_context* ctx, const TravParams& p)
 }
 
 // soft2 = 0 leaves r^2 as it is (r^2 + 0 = r^2): one FP64 addition less.
-template <int P>
+template <int P, bool kAhead = false>
 int launch_exact_p(bh_context* ctx, const TravParams& p)
 {
-    return p.soft2 == 0.0 ? launch_exact<P, false>(ctx, p) : launch_exact<P, true>(ctx, p);
+    return p.soft2 == 0.0 ? launch_exact<P, false, kAhead>(ctx, p) : launch_exact<P, true, kAhead>(ctx, p);
 }
 
 }  // namespace
@@ -485,9 +489,14 @@ int launch_exact_walk(bh_context* ctx, const ExactTree& tree, double theta, doub
     // where a warp's own latency counts.  Forces in ms with 4 / 8 / 16 / 32
     // lanes: 300,149 bodies 2.86 / 3.67 / 5.36 / -, 19,054 1.15 / 1.18 / 1.30 /
     // 2.19, 8,000 0.65 / 0.42 / 0.42 / 0.72, 4,000 0.41 / 0.27 / 0.21 / 0.28,
-    // 1,000 0.19 / 0.12 / 0.086 / 0.071.
+    // 1,000 0.19 / 0.12 / 0.086 / 0.071.  With 4 lanes and less than two rounds
+    // of warps (24 to an SM) the next step's records are loaded ahead: 19,054
+    // bodies 1.15 -> 1.12, 50,000 0.516 -> 0.510, but 100,000 0.931 -> 0.940
+    // (registers); with more lanes it is slower from the start (4,000 0.21 ->
+    // 0.22).
     const int64_t want = 12 * (int64_t)num_sms() * 32;
-    if (n * 4 >= want) return launch_exact_p<4>(ctx, p);
+    if (n * 4 >= 4 * want) return launch_exact_p<4>(ctx, p);
+    if (n * 4 >= want) return launch_exact_p<4, true>(ctx, p);
     if (n * 8 >= want) return launch_exact_p<8>(ctx, p);
     if (n * 16 >= want) return launch_exact_p<16>(ctx, p);
     return launch_exact_p<32>(ctx, p);

@@ -39,6 +39,13 @@ def test_sizes(bh, port, n):
     compare(bh, port, pos[:n], vel[:n], mass[:n], ids[:n], 1.05)
 
 
+@pytest.mark.parametrize("n", [58367, 58369])
+def test_records_loaded_ahead(bh, port, n):
+    """Below 58,368 bodies the evaluation loads the next step's records ahead."""
+    pos, vel, mass, ids = bh.generate_system(n, n, 0.1, 0.05)
+    compare(bh, port, pos[:n], vel[:n], mass[:n], ids[:n], 1.05)
+
+
 @pytest.mark.parametrize("n", [700, 5000, 9000, 16000])
 @pytest.mark.parametrize("theta,soft2", [(0.4, 0.0), (1.05, 1e-6), (0.8, 1e-2), (2.0, 0.0)])
 def test_angles_and_softening(bh, port, n, theta, soft2):
