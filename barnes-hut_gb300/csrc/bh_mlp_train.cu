@@ -52,41 +52,51 @@ struct FbSmem {
     float b3;
 };
 
+// A batch is a chain of three short kernels, each waiting for the one before.
+// They are launched so that a kernel's blocks are set up, and what does not
+// depend on the chain is loaded, while its predecessor runs; wait_for_chain()
+// returns when that one has completed, and lets the next be set up.  A kernel
+// waits before it writes anything or reads what the chain writes (past L1, whose
+// lines may be older than the wait), so it also knows all earlier ones complete.
+__device__ __forceinline__ void wait_for_chain()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_in_chain(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Forward, loss and backward to the layer deltas for 32 samples: lane = sample,
 // warp w computes units 8 w .. 8 w + 7 of each layer, so that eight independent
 // sums run beside one another and every weight is read by broadcast.  Each sum
 // keeps the order of its terms.  What bounds it is latency (a block's 32
 // samples are a chain of three small layers); with one thread per sample, 32
 // blocks of 128 on the whole chip, a batch of 4,096 took 135 us over its three
-// kernels, and takes 30 (in ncu 11 here, 12 in the sums, 6 in Adam).
+// kernels, and takes 22 (30 before they were chained; in ncu 11 here, 12 in
+// the sums, 6 in Adam).
 __global__ void __launch_bounds__(kFbThreads) mlp_fwd_bwd_kernel(const float* __restrict__ X,
                                                                 const float* __restrict__ T,
                                                                 const int32_t* __restrict__ idx, int64_t off,
-                                                                int B, float inv_b, const float* __restrict__ P,
+                                                                int B, float inv_b, const float* P,
                                                                 Scratch s)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FbSmem& m = *reinterpret_cast<FbSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, u0 = 8 * w;
-    static_assert(kOffW2 % 4 == 0, "rows of W2 are read as float4");
-#pragma unroll
-    for (int q = 0; q < kHid * kHid / 4 / kFbThreads; ++q) {
-        const int k = 4 * (threadIdx.x + q * kFbThreads), i = k / kHid, j = k % kHid;
-        float4 v = *reinterpret_cast<const float4*>(P + kOffW2 + k);
-        v.x = bf16r(v.x); v.y = bf16r(v.y); v.z = bf16r(v.z); v.w = bf16r(v.w);
-        *reinterpret_cast<float4*>(&m.W2[k]) = v;
-        m.W2t[j * kW2tRow + i] = v.x;
-        m.W2t[(j + 1) * kW2tRow + i] = v.y;
-        m.W2t[(j + 2) * kW2tRow + i] = v.z;
-        m.W2t[(j + 3) * kW2tRow + i] = v.w;
-    }
-    for (int k = threadIdx.x; k < kHid * kFeat; k += kFbThreads) m.W1[k] = bf16r(P[kOffW1 + k]);
-    if (threadIdx.x < kHid) {
-        m.b1[threadIdx.x] = P[kOffB1 + threadIdx.x];
-        m.b2[threadIdx.x] = P[kOffB2 + threadIdx.x];
-        m.W3[threadIdx.x] = bf16r(P[kOffW3 + threadIdx.x]);
-    }
-    if (threadIdx.x == 0) m.b3 = P[kOffB3];
     const int b = blockIdx.x * kFbSamples + lane;
     const bool live = b < B;
     const int64_t sidx = live ? (idx ? (int64_t)idx[off + b] : off + b) : 0;
@@ -94,6 +104,26 @@ __global__ void __launch_bounds__(kFbThreads) mlp_fwd_bwd_kernel(const float* __
 #pragma unroll
     for (int k = 0; k < kFeat; ++k) xb[k] = live ? bf16r(X[sidx * kFeat + k]) : 0.0f;
     const float target = live ? T[sidx] : 0.0f;
+    wait_for_chain();
+    static_assert(kOffW2 % 4 == 0, "rows of W2 are read as float4");
+#pragma unroll
+    for (int q = 0; q < kHid * kHid / 4 / kFbThreads; ++q) {
+        const int k = 4 * (threadIdx.x + q * kFbThreads), i = k / kHid, j = k % kHid;
+        float4 v = __ldcg(reinterpret_cast<const float4*>(P + kOffW2 + k));
+        v.x = bf16r(v.x); v.y = bf16r(v.y); v.z = bf16r(v.z); v.w = bf16r(v.w);
+        *reinterpret_cast<float4*>(&m.W2[k]) = v;
+        m.W2t[j * kW2tRow + i] = v.x;
+        m.W2t[(j + 1) * kW2tRow + i] = v.y;
+        m.W2t[(j + 2) * kW2tRow + i] = v.z;
+        m.W2t[(j + 3) * kW2tRow + i] = v.w;
+    }
+    for (int k = threadIdx.x; k < kHid * kFeat; k += kFbThreads) m.W1[k] = bf16r(__ldcg(P + kOffW1 + k));
+    if (threadIdx.x < kHid) {
+        m.b1[threadIdx.x] = __ldcg(P + kOffB1 + threadIdx.x);
+        m.b2[threadIdx.x] = __ldcg(P + kOffB2 + threadIdx.x);
+        m.W3[threadIdx.x] = bf16r(__ldcg(P + kOffW3 + threadIdx.x));
+    }
+    if (threadIdx.x == 0) m.b3 = __ldcg(P + kOffB3);
     __syncthreads();
     float h1[8];
 #pragma unroll
@@ -209,11 +239,17 @@ struct SmallTile {
     float xb[kRowStep][kFeat];
     float dy[kRowStep];
 };
-constexpr size_t kReduceSmem =
-    kSteps * (sizeof(W2Step) > sizeof(SmallTile) ? sizeof(W2Step) : sizeof(SmallTile));
+// More than half of an SM's shared memory, which keeps the blocks one to an SM.
+// They are set up while the forward blocks still hold most SMs; three to each
+// of the free ones, a batch of 4,096 took 36 us instead of 22.
+constexpr size_t kReduceSmem = 118 * 1024;
+static_assert(kReduceSmem >= kSteps * sizeof(W2Step) && kReduceSmem >= kSteps * sizeof(SmallTile) &&
+                  kReduceSmem + sizeof(FbSmem) + 2048 <= 228 * 1024,
+              "a reducing block beside a forward one");
 
 __global__ void __launch_bounds__(kReduceThreads) mlp_grad_reduce_kernel(int B, Scratch s)
 {
+    wait_for_chain();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int t = threadIdx.x;
     const bool small = blockIdx.x >= kW2Blocks;
@@ -316,26 +352,28 @@ __global__ void __launch_bounds__(kReduceThreads) mlp_grad_reduce_kernel(int B, 
 constexpr int kParamThreads = 128;
 constexpr int kParamBlocks = (kParams + kParamThreads - 1) / kParamThreads;
 
+// kParts values in order, all loads in flight at once.
+template <int kParts>
+__device__ __forceinline__ float sum_parts(const float* p, int stride)
+{
+    float x[kParts], r = 0.0f;
+#pragma unroll
+    for (int u = 0; u < kParts; ++u) x[u] = __ldcg(p + u * stride);
+#pragma unroll
+    for (int u = 0; u < kParts; ++u) r += x[u];
+    return r;
+}
+
 // Parameter k's gradient from the partial sums, added in part order.
 __device__ __forceinline__ float grad_of(const Scratch& s, int k)
 {
     if (k >= kOffW2 && k < kOffB2) {
         const float* p = s.p_w2 + (k - kOffW2);
         constexpr int n = kHid * kHid;
-        return (p[0] + p[n]) + (p[2 * n] + p[3 * n]);
+        return (__ldcg(p) + __ldcg(p + n)) + (__ldcg(p + 2 * n) + __ldcg(p + 3 * n));
     }
-    const float* p;
-    int parts, stride;
-    if (k < kOffB1) {
-        p = s.p_w1 + k; parts = 32; stride = kHid * kFeat;
-    } else {
-        const int e = k < kOffW2 ? k - kOffB1 : kHid + (k - kOffB2);
-        p = s.p_b + e; parts = 64; stride = kBiasParts;
-    }
-    float r = 0.0f;
-#pragma unroll 16
-    for (int u = 0; u < parts; ++u) r += p[u * stride];
-    return r;
+    if (k < kOffB1) return sum_parts<32>(s.p_w1 + k, kHid * kFeat);
+    return sum_parts<64>(s.p_b + (k < kOffW2 ? k - kOffB1 : kHid + (k - kOffB2)), kBiasParts);
 }
 
 // The batch's loss from the per-32-sample sums, by one warp: groups of four,
@@ -350,14 +388,14 @@ __device__ __forceinline__ void sum_loss(const Scratch& s, int B, float inv_b, f
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int u = u0 + 4 * lane + k;
-            t += u < np ? s.loss_part[u] : 0.0f;
+            t += u < np ? __ldcg(s.loss_part + u) : 0.0f;
         }
 #pragma unroll
         for (int k = 0; k < 32; ++k) l += __shfl_sync(0xffffffffu, t, k);  // past the end: + 0
     }
     if (lane == 0) {
         loss_out[0] = l * inv_b;
-        loss_out[1] += l * inv_b;
+        loss_out[1] = __ldcg(loss_out + 1) + l * inv_b;
     }
 }
 
@@ -371,22 +409,27 @@ __global__ void grad_kernel(int B, float inv_b, Scratch s, float* __restrict__ g
     if (k < kParams) g[k] = grad_of(s, k);
 }
 
-__global__ void adam_kernel(int B, float inv_b, Scratch s, float* __restrict__ P, float* __restrict__ m,
-                            float* __restrict__ v, float lr, float b1, float b2, float c1, float c2, float eps,
-                            float* __restrict__ loss_out)
+__global__ void __launch_bounds__(kParamThreads) adam_kernel(int B, float inv_b, Scratch s, float* P, float* m,
+                                                             float* v, float lr, float b1, float b2, float c1,
+                                                             float c2, float eps, float* loss_out)
 {
+    // The parameter and its moments are those of the step before, which has
+    // completed (the kernels between have waited for it).
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = k < kParams;
+    const float p0 = live ? __ldcg(P + k) : 0.0f, m0 = live ? __ldcg(m + k) : 0.0f, v0 = live ? __ldcg(v + k) : 0.0f;
+    wait_for_chain();
     if (blockIdx.x == kParamBlocks) {
         if (threadIdx.x < 32) sum_loss(s, B, inv_b, loss_out);
         return;
     }
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= kParams) return;
+    if (!live) return;
     const float gk = grad_of(s, k);
-    const float mk = b1 * m[k] + (1.0f - b1) * gk;
-    const float vk = b2 * v[k] + (1.0f - b2) * gk * gk;
+    const float mk = fmaf(1.0f - b1, gk, b1 * m0);
+    const float vk = fmaf((1.0f - b2) * gk, gk, b2 * v0);
     m[k] = mk;
     v[k] = vk;
-    P[k] -= lr * (mk * c1) / (sqrtf(vk * c2) + eps);
+    P[k] = p0 - lr * (mk * c1) / (sqrtf(vk * c2) + eps);
 }
 
 // Standardisation of the features and labels (FP64 sums, as the scaling's
@@ -543,11 +586,10 @@ int fwd_bwd(const float* X, const float* T, const int32_t* idx, int64_t off, int
                                      (int)sizeof(FbSmem)));
     BH_CUDA_TRY(cudaFuncSetAttribute(mlp_grad_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kReduceSmem));
-    mlp_fwd_bwd_kernel<<<(B + kFbSamples - 1) / kFbSamples, kFbThreads, sizeof(FbSmem), st>>>(X, T, idx, off, B,
-                                                                                           1.0f / (float)B, P, s);
-    BH_CUDA_TRY(cudaGetLastError());
-    mlp_grad_reduce_kernel<<<kW2Blocks + kSmallBlocks, kReduceThreads, kReduceSmem, st>>>(B, s);
-    BH_CUDA_TRY(cudaGetLastError());
+    BH_CUDA_TRY(launch_in_chain(mlp_fwd_bwd_kernel, (B + kFbSamples - 1) / kFbSamples, kFbThreads, sizeof(FbSmem), st, X,
+                                T, idx, off, B, 1.0f / (float)B, P, s));
+    BH_CUDA_TRY(launch_in_chain(mlp_grad_reduce_kernel, kW2Blocks + kSmallBlocks, kReduceThreads, kReduceSmem, st, B,
+                                s));
     return BH_OK;
 }
 
@@ -647,8 +689,8 @@ extern "C" int bh_mlp_train(const float* features, const float* labels, int64_t 
             ++step;
             const float c1 = 1.0f / (1.0f - std::pow(b1, (float)step));
             const float c2 = 1.0f / (1.0f - std::pow(b2, (float)step));
-            adam_kernel<<<kParamBlocks + 1, kParamThreads>>>(B, 1.0f / (float)B, s, dP, dM, dV, lr, b1, b2, c1, c2, eps, dL);
-            BH_CUDA_TRY(cudaGetLastError());
+            BH_CUDA_TRY(launch_in_chain(adam_kernel, kParamBlocks + 1, kParamThreads, 0, 0, B, 1.0f / (float)B, s, dP,
+                                        dM, dV, lr, b1, b2, c1, c2, eps, dL));
         }
         // the next epoch's order, while the device works on this one
         if (e + 1 < epochs) std::shuffle(order.begin(), order.end(), rng);
