@@ -330,8 +330,13 @@ int step_graph(bh_context* ctx, double dt, double theta, double G, int mode)
     BH_CUDA_TRY(cudaGraphLaunch(g.exec, ctx->stream));
     bh::swap_body_sets(ctx);
     ctx->launches += g.launches;
+    // What the replayed build leaves, as step_once records it: the far-field
+    // forms write the FP32 node records and no FP64 ones.
     ctx->tree_far = mode >= BH_MODE_FP32_FAR;
     ctx->tree_moments = mode == BH_MODE_LEARNED;
+    ctx->tree_rec = !ctx->tree_far;
+    ctx->fnodes_fused = true;
+    ctx->fnodes_G = G;
     return BH_OK;
 }
 
