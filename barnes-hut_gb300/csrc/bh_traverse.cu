@@ -26,12 +26,12 @@
 // bounds this (two lanes per cycle: 16 to 19 cycles of the SM per warp
 // instruction), so the products, the square root and the reciprocal run as
 // integer code beside it (bh_soft64.cuh): 11 FP64 instructions per 32 terms
-// are left (the differences, two squares, the sum of squares and the P
+// are left at P = 4 (the differences, two squares, the sum of squares and the P
 // additions) instead of 36.
 //
 // Measured (theta 1.05, ms of forces; before: one node per pass, 32 bodies
 // per warp, IEEE operations on the FP64 pipe):
-//   300,149 bodies 12.66 -> 2.86, 19,054 7.71 -> 1.12, 1,000 1.23 -> 0.071.
+//   300,149 bodies 12.66 -> 2.84, 19,054 7.71 -> 1.11, 1,000 1.23 -> 0.071.
 #include <climits>
 
 #include "bh_internal.cuh"
@@ -93,8 +93,8 @@ constexpr int kSoftStk = kStk - 21 * 8 - 8;
 // FP32 tests: a relative margin on the squares (eight roundings of 2^-24 each
 // and a square root's 2^-22 are below 1e-6) with an absolute one against
 // underflow (of squares below 2^-126, which sqrt_est takes as zero, too), and
-// the error of a group-relative distance relative to the coordinates' magnitudes: each
-// component of a difference is off by at most 2^-24 (3 |c| + 2 |r|), so the
+// the error of a group-relative distance relative to the coordinates'
+// magnitudes: each component of a difference is off by at most 2^-24 (3 |c| + 2 |r|), so the
 // distance by sqrt(3) times that, below 3.2e-7 (|c| + |r|); the hi + lo
 // split of an absolute coordinate adds 2^-46 of it, so sqrt(3) 2^-46, below
 // 2.5e-14, of the group's distance from the origin (and of |c|).
@@ -119,7 +119,11 @@ struct ExactSmem {
     static constexpr int kCap = 128;  // a power of two, over 33
     int2 stack[kTravWarps][kStk];
     int plist[kTravWarps][kCap][kBodies];
-    double term[kTravWarps][3][32];  // the terms of one step of an evaluation
+    // A warp to a body: the block's warps evaluate together, and the first takes
+    // the sums of all.
+    static constexpr bool kShare = P == 32;
+    static constexpr int kSumBodies = kShare ? kTravWarps * kBodies : kBodies;
+    double term[kShare ? 2 : 1][kTravWarps][3][32];  // the terms of one step of an evaluation
     // Nodes the box cannot decide: {centre, allowance}, {depth of the test,
     // node, leaf id or -1, a chain above the leaf}.
     float4 und[kTravWarps][32];
@@ -161,8 +165,11 @@ __device__ __forceinline__ void exact_term(const double4_32a& r, double px, doub
     }
 }
 
+// Blocks per SM of the form that loads records ahead.
+constexpr int kAheadBlocks = 5;
+
 template <int P, bool kSoft, bool kAhead>
-__global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams p)
+__global__ void __launch_bounds__(kTravThreads, kAhead ? kAheadBlocks : 0) traverse_exact_kernel(TravParams p)
 {
     using Smem = ExactSmem<P>;
     constexpr int kBodies = Smem::kBodies;
@@ -176,11 +183,11 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t group = (int64_t)blockIdx.x * kTravWarps + w;
     const int64_t base = group * kBodies;
-    if (base >= p.n) return;  // whole warp past the end
+    if (!Smem::kShare && base >= p.n) return;  // whole warp past the end
     const int body = lane / P, phase = lane % P;
     const int64_t i = base + body;
     const bool valid = i < p.n;
-    const int64_t ii = valid ? i : base;
+    const int64_t ii = valid ? i : base < p.n ? base : 0;
     const double px = p.px[ii], py = p.py[ii], pz = p.pz[ii];
     const int my_leaf = valid ? p.body_leaf[i] : -2;
     const double theta2 = p.theta2, soft2 = p.soft2;
@@ -212,12 +219,10 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
     int (*PL)[kBodies] = sm.plist[w];
     const unsigned lt = (1u << lane) - 1u;
 
-    // Lane l < 3 kBodies sums the component l / kBodies of body l % kBodies.
-    double sum = 0.0;
     // This body's list: entries done .. cnt - 1, in slots modulo kCap.
     int cnt = 0, done = 0;
-    int sp = 1;
     const unsigned full = __ballot_sync(0xffffffffu, valid) & Smem::kFirst;
+    int sp = full ? 1 : 0;
     const double one = __shfl_sync(0xffffffffu, p.one, 0);
     if (lane == 0) stk[0] = make_int2(0, (int)full);
     __syncwarp();
@@ -226,39 +231,72 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
 
     // Evaluates the bodies' lists in order until none holds more than `left`
     // entries.  P lanes evaluate P consecutive terms of a body.  The sums run
-    // over them one after the other, each waiting for the one before (about
-    // 100 cycles), so they take the terms of the step before while the next
-    // ones are evaluated (19,054 bodies 1.18 -> 1.15 ms, 8,000 0.46 -> 0.42).
-    auto T = sm.term[w];
-    const double* const sums = &T[lane < 3 * kBodies ? lane / kBodies : 2][lane % kBodies * P];
-    T[0][lane] = T[1][lane] = T[2][lane] = 0.0;
-    __syncwarp();
+    // over them one after the other, each waiting for the one before (68
+    // cycles), so they take the terms of the step before while the next ones
+    // are evaluated (19,054 bodies 1.18 -> 1.15 ms, 8,000 0.46 -> 0.42).
+    // Lane l < 3 kSumBodies sums the component l / kSumBodies of a body.  An
+    // addition takes the FP64 pipe 19 cycles however few lanes it is for, and a
+    // warp's own sums are P of them a step, at P = 32 32 of 39 FP64
+    // instructions: there the block's four warps evaluate together, a barrier
+    // to a step, and the first takes the sums of all (2,000 bodies 0.135 ->
+    // 0.103 ms, 4,000 0.285 -> 0.170; with 16 lanes 0.208 -> 0.238, with 8
+    // 0.27 -> 0.29).
+    constexpr int kSumBodies = Smem::kSumBodies;
+    const bool sums = !Smem::kShare || w == 0;
+    const int sum_body = lane % kSumBodies;  // of the block, or of the warp
+    const int sum_comp = lane < 3 * kSumBodies ? lane / kSumBodies : 2;
+    double sum = 0.0;
+    int par = 0;  // the half of `term` the next step fills
+    for (int h = 0; h < (Smem::kShare ? 2 : 1); ++h)
+        sm.term[h][w][0][lane] = sm.term[h][w][1][lane] = sm.term[h][w][2][lane] = 0.0;
+    if (Smem::kShare) __syncthreads();
+    else __syncwarp();
+    // where they stand in a half of `term`
+    const int from = (Smem::kShare ? sum_body / kBodies : w) * 96 + sum_comp * 32 + sum_body % kBodies * P;
+    constexpr int kHalf = kTravWarps * 96;
     auto add = [&] {
+        const double* t = &sm.term[0][0][0][0] + from + (Smem::kShare ? (par ^ 1) * kHalf : 0);
 #pragma unroll
-        for (int k = 0; k < P; ++k) sum = fma(sum, one, sums[k]);
+        for (int k = 0; k < P; ++k) sum = fma(sum, one, t[k]);
     };
-    auto flush = [&](int left) {
+    auto record = [&](int q) { return p.tree.d4[q < cnt ? PL[q & (Smem::kCap - 1)][body] : 0]; };
+    auto step = [&](double4_32a& next, auto beside) {
+        const int q = done + phase;
+        const bool on = q < cnt;
+        const double4_32a r = kAhead ? next : record(q);
+        if (kAhead) next = record(q + P);
+        double tx, ty, tz;
+        exact_term<kSoft>(r, px, py, pz, soft2, on, one, tx, ty, tz, beside);
+        if (!Smem::kShare) __syncwarp();
+        // (a sum is never -0, so adding +0 leaves it as it is)
+        auto T = sm.term[Smem::kShare ? par : 0][w];
+        T[0][lane] = on ? tx : 0.0;
+        T[1][lane] = on ? ty : 0.0;
+        T[2][lane] = on ? tz : 0.0;
+        done = min(done + P, cnt);
+    };
+    // kShare: every warp of the block calls it equally often, walking or not;
+    // returns whether any still walks.
+    auto flush = [&](int left, bool walking) {
+        if (Smem::kShare) {
+            while (__syncthreads_or(cnt - done > left)) {
+                double4_32a none;
+                if (sums) step(none, add);
+                else step(none, [] {});
+                par ^= 1;
+            }
+            return __syncthreads_or(walking) != 0;
+        }
         int most = cnt - done;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
-        auto record = [&](int q) { return p.tree.d4[q < cnt ? PL[q & (Smem::kCap - 1)][body] : 0]; };
         double4_32a next;
         if (kAhead) next = record(done + phase);
         for (; most > left; most -= P) {
-            const int q = done + phase;
-            const bool on = q < cnt;
-            const double4_32a r = kAhead ? next : record(q);
-            if (kAhead) next = record(q + P);
-            double tx, ty, tz;
-            exact_term<kSoft>(r, px, py, pz, soft2, on, one, tx, ty, tz, add);
+            step(next, add);
             __syncwarp();
-            // (a sum is never -0, so adding +0 leaves it as it is)
-            T[0][lane] = on ? tx : 0.0;
-            T[1][lane] = on ? ty : 0.0;
-            T[2][lane] = on ? tz : 0.0;
-            __syncwarp();
-            done = min(done + P, cnt);
         }
+        return false;
     };
 
     while (sp > 0) {
@@ -402,7 +440,7 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
         if (em) {
             if (__any_sync(0xffffffffu, cnt - done > Smem::kCap - 33)) {
                 __syncwarp();
-                flush(Smem::kCap / 4);
+                flush(Smem::kCap / 4, true);
             }
             // Body by body: the lanes whose item it takes append it.
 #pragma unroll
@@ -416,15 +454,14 @@ __global__ void __launch_bounds__(kTravThreads) traverse_exact_kernel(TravParams
         }
         __syncwarp();
     }
-    flush(0);
+    while (flush(0, false)) {}
     add();
     if (overflow && lane == 0) atomicOr(p.err, kErrOverflow);
-    if (lane < 3 * kBodies) {
-        const int c = lane / kBodies;
-        const int64_t k = base + lane % kBodies;
+    if (sums && lane < 3 * kSumBodies) {
+        const int64_t k = (Smem::kShare ? (int64_t)blockIdx.x * kTravWarps * kBodies : base) + sum_body;
         if (k < p.n) {
-            double* a = c == 0 ? p.ax : c == 1 ? p.ay : p.az;
-            double* v = c == 0 ? p.vx : c == 1 ? p.vy : p.vz;
+            double* a = sum_comp == 0 ? p.ax : sum_comp == 1 ? p.ay : p.az;
+            double* v = sum_comp == 0 ? p.vx : sum_comp == 1 ? p.vy : p.vz;
             a[k] = sum;
             if (p.kick_h > 0.0) v[k] = __dadd_rn(v[k], __dmul_rn(p.kick_h, sum));
         }
@@ -487,18 +524,17 @@ int launch_exact_walk(bh_context* ctx, const ExactTree& tree, double theta, doub
     // Lanes to a body: 4 (the evaluation's sums fill 24 lanes and the bodies
     // share a walk) while that gives the chip 12 warps per SM, and more below,
     // where a warp's own latency counts.  Forces in ms with 4 / 8 / 16 / 32
-    // lanes: 300,149 bodies 2.86 / 3.67 / 5.36 / -, 19,054 1.15 / 1.18 / 1.30 /
-    // 2.19, 8,000 0.65 / 0.42 / 0.42 / 0.72, 4,000 0.41 / 0.27 / 0.21 / 0.28,
-    // 1,000 0.19 / 0.12 / 0.086 / 0.071.  With 4 lanes and less than two rounds
-    // of warps (24 to an SM) the next step's records are loaded ahead: 19,054
-    // bodies 1.15 -> 1.12, 50,000 0.516 -> 0.510, but 100,000 0.931 -> 0.940
-    // (registers); with more lanes it is slower from the start (4,000 0.21 ->
-    // 0.22).
+    // lanes: 300,149 bodies 2.84 / 3.67 / 5.36 / -, 19,054 1.11 / 1.18 / 1.30 /
+    // 1.29, 14,000 0.90 / 0.72 / - / 0.88, 8,000 0.63 / 0.41 / 0.42 / 0.43, 7,000
+    // - / 0.36 / - / 0.39, 4,000 0.40 / 0.27 / 0.21 / 0.17, 2,000 0.27 / 0.17 / 0.13 / 0.10, 1,000 0.18 /
+    // 0.12 / 0.086 / 0.071 (16 is not built: never ahead of both neighbours by
+    // more than 1 %).  With 4 lanes and all blocks on the chip at once, five to an
+    // SM, the next step's records are loaded ahead, which takes 92 registers
+    // for 72 (19,054 bodies 1.15 -> 1.11; 30,000 0.312 -> 0.344, in two rounds).
     const int64_t want = 12 * (int64_t)num_sms() * 32;
-    if (n * 4 >= 4 * want) return launch_exact_p<4>(ctx, p);
+    if (n > kAheadBlocks * kTravWarps * 8 * (int64_t)num_sms()) return launch_exact_p<4>(ctx, p);
     if (n * 4 >= want) return launch_exact_p<4, true>(ctx, p);
-    if (n * 8 >= want) return launch_exact_p<8>(ctx, p);
-    if (n * 16 >= want) return launch_exact_p<16>(ctx, p);
+    if (n * 8 >= want - want / 8) return launch_exact_p<8>(ctx, p);
     return launch_exact_p<32>(ctx, p);
 }
 

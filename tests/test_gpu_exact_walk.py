@@ -1,7 +1,7 @@
 """The FP64 walks at the sizes where their splits change.
 
-The bit-exact walk at the sizes where its split changes (lanes per body:
-32 below 3,648 bodies, 16, 8 and 4 from 14,592 on, with 152 SMs), at partly
+The bit-exact walk at the sizes where its split changes (lanes per body: 32
+below 6,384 bodies, 8, and 4 from 14,592 on, with 152 SMs), at partly
 filled warps, with softening, at theta 0 and for a planar system, against the
 oracle bit for bit.  The masked walks with one warp per group and with teams
 of 16 (up to 9,728 bodies), 8 (24,320, FP32) and 4 (48,640 list, 87,552 group,
@@ -39,10 +39,12 @@ def test_sizes(bh, port, n):
     compare(bh, port, pos[:n], vel[:n], mass[:n], ids[:n], 1.05)
 
 
-@pytest.mark.parametrize("n", [58367, 58369])
-def test_records_loaded_ahead(bh, port, n):
-    """Below 58,368 bodies the evaluation loads the next step's records ahead."""
-    pos, vel, mass, ids = bh.generate_system(n, n, 0.1, 0.05)
+@pytest.mark.parametrize("n", [3, 127, 129, 6383, 6385, 24320, 24321])
+def test_shared_sums_and_records_ahead(bh, port, n):
+    """Up to 6,383 bodies a block's warps share the sums of their four bodies
+    (partly filled blocks among them), and up to 24,320 with 4 lanes to a body
+    the evaluation loads the next step's records ahead."""
+    pos, vel, mass, ids = bh.generate_system(n, max(n, 10), 0.1, 0.05)
     compare(bh, port, pos[:n], vel[:n], mass[:n], ids[:n], 1.05)
 
 
