@@ -30,9 +30,9 @@ constexpr int kRadix = 256;
 constexpr int kSortThreads = 512;      // onesweep tile: 512 threads x 8 keys
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;
-constexpr int kClusterSortMax = 65536;  // keys one cluster sorts (8 blocks x 8192; 16-bit payloads)
-// Whether launch_sort reads the digit histograms of launch_keys / launch_hist.
-inline bool sort_uses_hist(int64_t n) { return n > kClusterSortMax; }
+// Whether the sort of n keys reads the digit histograms of launch_keys,
+// launch_hist or prepare_sort_raw (else one cluster sorts them).
+bool sort_uses_hist(int64_t n);
 
 // SM count of the current device (cudaDevAttrMultiProcessorCount), read once
 // per device and cached; grids are sized in multiples of it.  1 when the

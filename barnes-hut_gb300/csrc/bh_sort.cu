@@ -11,8 +11,8 @@
 // in the look-back is bounded; on expiry the kernel raises kErrTimeout
 // and still publishes, so no tile can wait forever.
 //
-// Up to kClusterSortMax keys one thread-block cluster sorts in distributed
-// shared memory instead (cluster_sort_kernel below).
+// Up to some 100,000 keys one thread-block cluster sorts in distributed shared
+// memory instead (cluster_sort_kernel below).
 #include <cooperative_groups.h>
 
 #include <utility>
@@ -258,11 +258,17 @@ constexpr int kCThreads = 1024;
 constexpr int kCWarps = kCThreads / 32;
 constexpr int kCMax = 16;      // blocks, where the device takes clusters beyond the portable 8
 constexpr int kCPortable = 8;
+constexpr int kBlockKeys = 8192;
+// With 16 blocks the cluster is ahead of the onesweep passes up to here (sort and
+// key phases together, us: 65,537 keys 102 / 59, 98,304 103 / 74, 110,000 107 /
+// 82 with a step 1 % faster, 131,000 108 / 91 with a step 2 % slower); three
+// rounds, where long ties are left, take three times as long.
+constexpr int64_t kClusterSortMax = 98304;
 constexpr int kTieRun = 16;
 constexpr int kHistRow = kRadix + 2;  // 129 words: the four quarters of a digit's column fall in four bank groups
 
 struct ClusterSmem {
-    uint64_t words[kClusterSortMax / kCPortable];  // 32 bits of the key over the key's index
+    uint64_t words[kBlockKeys];  // 32 bits of the key over the key's index
     uint16_t warp_hist[kCWarps][kHistRow];
     uint32_t warp_mask[kCWarps][kRadix];
     uint32_t totals[kCMax][kRadix];  // every block's digit counts
@@ -284,7 +290,7 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
     const int start = r * per;
     const int cnt = n - start < 0 ? 0 : (n - start < per ? n - start : per);
     const unsigned lt = (1u << lane) - 1u;
-    // g / per for g < 2^16, per <= 2^13 (exact: the excess of the reciprocal
+    // g / per for g < 2^17, per <= 2^13 (exact: the excess of the reciprocal
     // times g stays below 2^32; per == 1 is a single key, 2^32 wraps to 0)
     const uint32_t recip = (uint32_t)(((1ull << 32) + per - 1) / per);
     const auto sync = [&] {
@@ -455,36 +461,51 @@ int launch_cluster_sort_items(int n, int C, int per, const uint64_t* in, uint64_
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (C > kCPortable) {
-        // A device without room for the large cluster takes the portable one.
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, cluster_sort_kernel<I>, &cfg) != cudaSuccess || clusters < 1) {
-            cudaGetLastError();
-            return BH_ERR_CAPACITY;
-        }
-    }
     BH_CUDA_TRY(cudaLaunchKernelEx(&cfg, cluster_sort_kernel<I>, n, per, in, out, vals));
     return BH_OK;
 }
 
-int launch_cluster_sort_blocks(int n, int C, const uint64_t* in, uint64_t* out, uint32_t* vals, cudaStream_t stream)
+// Blocks of the largest cluster: kCMax where the device has room for one.
+int cluster_blocks_max()
 {
+    static const int most = [] {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kCMax);
+        cfg.blockDim = dim3(kCThreads);
+        cfg.dynamicSmemBytes = sizeof(ClusterSmem);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kCMax;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        const bool fits =
+            cudaFuncSetAttribute(cluster_sort_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(ClusterSmem)) == cudaSuccess &&
+            cudaFuncSetAttribute(cluster_sort_kernel<8>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, cluster_sort_kernel<8>, &cfg) == cudaSuccess && clusters > 0;
+        cudaGetLastError();
+        return fits ? kCMax : kCPortable;
+    }();
+    return most;
+}
+
+// 1 <= n, !sort_uses_hist(n); in and out may be the same.
+int launch_cluster_sort(int64_t n64, const uint64_t* in, uint64_t* out, uint32_t* vals, cudaStream_t stream)
+{
+    const int n = (int)n64, most = cluster_blocks_max();
+    int C = 1;
+    while (C < most && C * kCThreads < n) C *= 2;
     const int per = (n + C - 1) / C;
     if (per <= kCThreads) return launch_cluster_sort_items<1>(n, C, per, in, out, vals, stream);
     if (per <= 2 * kCThreads) return launch_cluster_sort_items<2>(n, C, per, in, out, vals, stream);
     if (per <= 3 * kCThreads) return launch_cluster_sort_items<3>(n, C, per, in, out, vals, stream);
     if (per <= 4 * kCThreads) return launch_cluster_sort_items<4>(n, C, per, in, out, vals, stream);
+    if (per <= 6 * kCThreads) return launch_cluster_sort_items<6>(n, C, per, in, out, vals, stream);
     return launch_cluster_sort_items<8>(n, C, per, in, out, vals, stream);
-}
-
-// 1 <= n <= kClusterSortMax; in and out may be the same.
-int launch_cluster_sort(int64_t n, const uint64_t* in, uint64_t* out, uint32_t* vals, cudaStream_t stream)
-{
-    int C = 1;
-    while (C < kCMax && (int64_t)C * kCThreads < n) C *= 2;
-    int rc = launch_cluster_sort_blocks((int)n, C, in, out, vals, stream);
-    if (rc == BH_ERR_CAPACITY) rc = launch_cluster_sort_blocks((int)n, kCPortable, in, out, vals, stream);
-    return rc;
 }
 
 constexpr int kPermThreads = 256;
@@ -514,6 +535,12 @@ __global__ void __launch_bounds__(kPermThreads) permute_kernel(
 }  // namespace
 
 size_t sort_smem_bytes() { return sizeof(SortSmem); }
+
+bool sort_uses_hist(int64_t n)
+{
+    const int64_t room = (int64_t)cluster_blocks_max() * kBlockKeys;
+    return n > (room < kClusterSortMax ? room : kClusterSortMax);
+}
 
 int launch_sort(bh_context* ctx)
 {

@@ -25,7 +25,8 @@ def _keys(kind, n, rng):
     raise ValueError(kind)
 
 
-@pytest.mark.parametrize("n", [2, 33, 1023, 1024, 1025, 4097, 8192, 8193, 19054, 24577, 40001, 65535, 65536, 65537])
+@pytest.mark.parametrize("n", [2, 33, 1023, 1024, 1025, 4097, 8192, 8193, 19054, 24577, 40001, 65535, 65536, 65537,
+                               98303, 98304, 98305])
 @pytest.mark.parametrize("kind", ["random", "top_bit", "short_ties", "long_ties", "equal", "reversed"])
 def test_sort_matches_a_stable_sort(bh, kind, n):
     rng = np.random.default_rng(n)
