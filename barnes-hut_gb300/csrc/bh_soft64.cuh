@@ -225,8 +225,9 @@ BH_SOFT double square(uint64_t d)
 //   i = RN(1/RN(sqrt(r2))), i3 = RN(RN(i i) i), sc = RN(gm i3),
 //   t = RN(sc d) per component (0 where d = +-0).
 // Returns false (t unset) outside r^2 in 2^+-200, G m in 2^+-300 and |d| = 0
-// or at least 2^-300 (where every product stays in the normal range), and in
-// the odd cases above.
+// or in [2^-300, 2^401) (where every product stays in the normal range), and in
+// the odd cases above.  The upper end is for an r^2 formed with square(): past
+// its range it may wrap to any value, one inside r^2's range among them.
 BH_SOFT bool term(double dx, double dy, double dz, double r2, double gm, double& tx, double& ty, double& tz)
 {
     const uint64_t br = bits_of(r2), bg = bits_of(gm);
@@ -242,7 +243,7 @@ BH_SOFT bool term(double dx, double dy, double dz, double r2, double gm, double&
         const uint64_t d = bits_of(dk);
         const bool zero = is_zero(d);
         const Sig s = unpack(d);
-        odd_case = odd_case || (!zero && (low_zero(s) || s.e < -300));
+        odd_case = odd_case || (!zero && (low_zero(s) || (uint32_t)(s.e + 300) > 700u));
         const uint64_t v = mul_bits(sc.a, s.a, sc.e + s.e) | (d & 0x8000000000000000ull);
         return from_bits(zero ? 0ull : v);
     };
