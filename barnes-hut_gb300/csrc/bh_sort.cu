@@ -81,7 +81,7 @@ __device__ uint32_t scan256(uint32_t v, uint32_t* tmp)
     if (lane == 31) tmp[w] = x;
     __syncwarp();
     // 8 warps: a tiny serial pass by each thread over the warp totals.
-    asm volatile("bar.sync 1, 256;");
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     uint32_t before = 0;
     for (int k = 0; k < w; ++k) before += tmp[k];
     return before + x - v;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) onesweep_kernel(
 #pragma unroll
         for (int k = 0; k < kSortItems; ++k)
             val[k] = kFirst ? (uint32_t)base + first + k * 32 : first + k * 32 < cnt ? vals_in[base + first + k * 32] : 0;
-        asm volatile("bar.sync 2, %0;" ::"n"(kSortThreads));
+        asm volatile("bar.sync 2, %0;" ::"n"(kSortThreads) : "memory");
         // Two threads per digit: exclusive prefix over the warps.
         const int d = threadIdx.x >> 1, h = threadIdx.x & 1;
         uint32_t sum = 0;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) onesweep_kernel(
     __syncthreads();
     if (ranks) {
         // ... and the digits' starts from the other warps.
-        asm volatile("bar.sync 3, %0;" ::"n"(kTileThreads));
+        asm volatile("bar.sync 3, %0;" ::"n"(kTileThreads) : "memory");
         // Into shared memory in tile-sorted order.
 #pragma unroll
         for (int k = 0; k < kSortItems; ++k) {
