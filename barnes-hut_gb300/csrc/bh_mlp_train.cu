@@ -207,13 +207,14 @@ __global__ void __launch_bounds__(kFbThreads) mlp_fwd_bwd_kernel(const float* __
 __device__ __forceinline__ void copy16(void* smem, const void* global)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
-                 "l"(global));
+                 "l"(global)
+                 : "memory");
 }
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n"); }
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void copy_wait()
 {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 // The gradient's sums over the batch, to partial sums (one term after the

@@ -19,7 +19,7 @@ def statements():
             yield path.name, m.group(0)
 
 
-@pytest.mark.parametrize("mnemonic", ["bar.", "griddepcontrol."])
+@pytest.mark.parametrize("mnemonic", ["bar.", "griddepcontrol.", "cp.async."])
 def test_ordering_asm_clobbers_memory(mnemonic):
     found = [(name, s) for name, s in statements() if mnemonic in s]
     assert found
