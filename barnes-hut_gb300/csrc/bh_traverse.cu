@@ -32,6 +32,7 @@
 // Measured (theta 1.05, ms of forces; before: one node per pass, 32 bodies
 // per warp, IEEE operations on the FP64 pipe):
 //   300,149 bodies 12.66 -> 2.84, 19,054 7.71 -> 1.11, 1,000 1.23 -> 0.071.
+#include <cfloat>
 #include <climits>
 
 #include "bh_internal.cuh"
@@ -100,9 +101,14 @@ constexpr int kSoftStk = kStk - 21 * 8 - 8;
 // 2.5e-14, of the group's distance from the origin (and of |c|).
 constexpr float kMargin = 2e-6f, kTiny = 1e-36f;
 constexpr float kAbsErr = 4e-7f;
+// Where a square or a product overflows (distances above 1.8e19), an infinite
+// bound says nothing about one that is finite in FP64: sure_below asks for a
+// finite right side, and the table's side^2 ends at FLT_MAX, which sure_below
+// never accepts and sure_above still bounds from below.
 __device__ __forceinline__ bool sure_below(float side2, float theta2, float dist2)  // side^2 < theta^2 dist^2
 {
-    return fmaf(side2, 1.0f + kMargin, kTiny) < theta2 * dist2;
+    const float right = theta2 * dist2;
+    return fmaf(side2, 1.0f + kMargin, kTiny) < right && right <= FLT_MAX;
 }
 __device__ __forceinline__ bool sure_above(float side2, float theta2, float dist2)  // side^2 > theta^2 dist^2
 {
@@ -177,7 +183,7 @@ __global__ void __launch_bounds__(kTravThreads, kAhead ? kAheadBlocks : 0) trave
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     fill_side2(p.bbox, sm.side2);
     __syncthreads();
-    if (threadIdx.x <= kMaxDepth) sm.side2f[threadIdx.x] = (float)sm.side2[threadIdx.x];
+    if (threadIdx.x <= kMaxDepth) sm.side2f[threadIdx.x] = fminf((float)sm.side2[threadIdx.x], FLT_MAX);
     __syncthreads();
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
