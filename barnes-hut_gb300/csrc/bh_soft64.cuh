@@ -213,11 +213,15 @@ BH_SOFT Sig rcp_sqrt(const Sig& x, bool& odd_case)
 }
 
 // d d rounded, for d = 0 or |d| in [2^-400, 2^400] with a significand that
-// does not end in 32 zero bits.
+// does not end in 32 zero bits.  Larger |d|, infinities and NaN give at least
+// 2^800 or no number, as the exponent stops at 511: an r^2 with such a square
+// in it is outside term()'s range.  (The bound here, not on term()'s components:
+// forces at 19,054 bodies 1.105 ms, 1.123 there, 1.100 without one.)
 BH_SOFT double square(uint64_t d)
 {
     const Sig s = unpack(d);
-    return from_bits(is_zero(d) ? 0ull : mul_bits(s.a, s.a, 2 * s.e));
+    const int e = s.e < 511 ? s.e : 511;
+    return from_bits(is_zero(d) ? 0ull : mul_bits(s.a, s.a, 2 * e));
 }
 
 // The reference's interaction term (src/traversal.cpp:82-88) from the
@@ -225,9 +229,8 @@ BH_SOFT double square(uint64_t d)
 //   i = RN(1/RN(sqrt(r2))), i3 = RN(RN(i i) i), sc = RN(gm i3),
 //   t = RN(sc d) per component (0 where d = +-0).
 // Returns false (t unset) outside r^2 in 2^+-200, G m in 2^+-300 and |d| = 0
-// or in [2^-300, 2^401) (where every product stays in the normal range), and in
-// the odd cases above.  The upper end is for an r^2 formed with square(): past
-// its range it may wrap to any value, one inside r^2's range among them.
+// or at least 2^-300 (where every product stays in the normal range; r^2 bounds
+// |d| from above), and in the odd cases above.
 BH_SOFT bool term(double dx, double dy, double dz, double r2, double gm, double& tx, double& ty, double& tz)
 {
     const uint64_t br = bits_of(r2), bg = bits_of(gm);
@@ -243,7 +246,7 @@ BH_SOFT bool term(double dx, double dy, double dz, double r2, double gm, double&
         const uint64_t d = bits_of(dk);
         const bool zero = is_zero(d);
         const Sig s = unpack(d);
-        odd_case = odd_case || (!zero && (low_zero(s) || (uint32_t)(s.e + 300) > 700u));
+        odd_case = odd_case || (!zero && (low_zero(s) || s.e < -300));
         const uint64_t v = mul_bits(sc.a, s.a, sc.e + s.e) | (d & 0x8000000000000000ull);
         return from_bits(zero ? 0ull : v);
     };
