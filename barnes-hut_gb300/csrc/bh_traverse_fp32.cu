@@ -113,6 +113,20 @@ __device__ __noinline__ bool own_chain_accepts(double dx, double dy, double dz, 
     return side2 < __dmul_rn(theta2, r2);
 }
 
+// The list form's FP32 tests, sides clamped to FLT_MAX: false where the margin
+// (with an absolute one for squares below 2^-126, which sqrt_est takes as zero)
+// leaves a doubt, and where the right side overflowed.
+constexpr float kTiny = 1e-36f;
+__device__ __forceinline__ bool sure_below(float side2, float theta2, float dist2)  // side^2 < theta^2 dist^2
+{
+    const float right = theta2 * dist2;
+    return fmaf(side2, 1.0f + kMargin, kTiny) < right && right <= FLT_MAX;
+}
+__device__ __forceinline__ bool sure_above(float side2, float theta2, float dist2)  // side^2 > theta^2 dist^2
+{
+    return side2 * (1.0f - kMargin) > fmaf(theta2, dist2, kTiny);
+}
+
 // kTeam > 1: a block of kTeam warps walks one group, for systems with too few
 // groups to fill the chip.  The warps take ranges from one stack in rounds
 // (kTeamPop each from its top, eight lanes to a range), push the opened nodes'
@@ -138,7 +152,7 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
         if (L < dz) L = dz;
         const double side = __ddiv_rn(L, (double)(1ull << threadIdx.x));
         sm.side2d[threadIdx.x] = __dmul_rn(side, side);
-        const float s2f = (float)sm.side2d[threadIdx.x];
+        const float s2f = kFP64 ? fminf((float)sm.side2d[threadIdx.x], FLT_MAX) : (float)sm.side2d[threadIdx.x];
         sm.side2f[threadIdx.x] = s2f;
         if (!kFP64) {
             // The FP32 walk's group-test distances: a node of this depth is
@@ -335,9 +349,9 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                     nerr = err;
                     if (kFP64) {
                         s2 = sm.side2f[depth];
-                        const float dlo = fmaxf(sqrt_est(dmin2) - err, 0.0f), dhi = sqrt_est(dmax2 + FLT_MIN) + err;
-                        if (s2 * (1.0f + kMargin) < theta2f * dlo * dlo) A = M;
-                        else if (s2 * (1.0f - kMargin) > theta2f * dhi * dhi) A = 0;
+                        const float dlo = fmaxf(sqrt_est(dmin2) - err, 0.0f), dhi = sqrt_est(dmax2) + err;
+                        if (sure_below(s2, theta2f, dlo * dlo)) A = M;
+                        else if (sure_above(s2, theta2f, dhi * dhi)) A = 0;
                         else mixed = true;
                     } else {
                         // The same tests squared on the distance side:
@@ -420,11 +434,11 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                     const float cz = __shfl_sync(0xffffffffu, e.z, j);
                     const float ej = 2.0f * __shfl_sync(0xffffffffu, nerr, j);
                     const float dxf = cx - rx, dyf = cy - ry, dzf = cz - rz;
-                    const float df = sqrt_est(dxf * dxf + dyf * dyf + dzf * dzf + FLT_MIN);
+                    const float df = sqrt_est(dxf * dxf + dyf * dyf + dzf * dzf);
                     const float lo = fmaxf(df - ej, 0.0f), hi = df + ej;
                     const float s2j = sm.side2f[dj], sf = (float)soft2;
-                    const bool sure_acc = s2j * (1.0f + kMargin) < theta2f * (lo * lo + sf);
-                    const bool sure_rej = s2j * (1.0f - kMargin) > theta2f * (hi * hi + sf * (1.0f + kMargin));
+                    const bool sure_acc = sure_below(s2j, theta2f, lo * lo + sf);
+                    const bool sure_rej = sure_above(s2j, theta2f, hi * hi + sf);
                     acc = sure_acc;
                     if (((Mj >> lane) & 1u) && !sure_acc && !sure_rej) {
                         const TreeRec r = p.rec[nj];
