@@ -350,8 +350,9 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                     if (kFP64) {
                         s2 = sm.side2f[depth];
                         const float dlo = fmaxf(sqrt_est(dmin2) - err, 0.0f), dhi = sqrt_est(dmax2) + err;
-                        if (sure_below(s2, theta2f, dlo * dlo)) A = M;
-                        else if (sure_above(s2, theta2f, dhi * dhi)) A = 0;
+                        const float sf = (float)soft2;
+                        if (sure_below(s2, theta2f, dlo * dlo + sf)) A = M;
+                        else if (sure_above(s2, theta2f, dhi * dhi + sf)) A = 0;
                         else mixed = true;
                     } else {
                         // The same tests squared on the distance side:
