@@ -26,7 +26,7 @@
 //   displacement's bits on the integer pipes, to within an ulp
 //   (soft::scale); six FP64 instructions per 32 pairs are left of 13 (the
 //   differences and the accumulating FMAs).  300,149 bodies, theta 1.05:
-//   3.27 -> 1.88 ms of forces.
+//   3.27 -> 1.76 ms of forces.
 // BH_MODE_FP32_FAR: precision form.  The bodies with id < num_direct (Sun and
 //   planets) are taken out of the tree (masses zeroed before the build) and
 //   summed directly in FP64.  Far-field interactions run in FP32 on
@@ -95,13 +95,11 @@ __global__ void direct_extract_kernel(int64_t n, const double* __restrict__ px, 
 
 namespace {
 
-// G m r^-3 on the FP64 pipe, for the pairs soft::scale leaves out.  A call of
-// its own: inlined, it becomes predicated instructions that take the FP64 pipe
-// although no lane needs them.
-__device__ __noinline__ double fp64_scale(double dx, double dy, double dz, double soft2, double gm)
-{
-    return gm * rcube_hh(fma(dx, dx, fma(dy, dy, fma(dz, dz, soft2))));
-}
+// G m r^-3 from r^2 on the FP64 pipe, for the pairs soft::scale leaves out and
+// with softening.  A call of its own: inlined, it becomes predicated
+// instructions that take the FP64 pipe although no lane needs them (softened,
+// 300,149 bodies: 3.37 ms of forces, inlined 4.9).
+__device__ __noinline__ double fp64_scale(double r2, double gm) { return gm * rcube_hh(r2); }
 
 // Whether a cell of depth 20 accepts, with the reference's rounding
 // (traversal.cpp:78); a call for the same reason.
@@ -134,7 +132,7 @@ __device__ __forceinline__ bool sure_above(float side2, float theta2, float dist
 // for all 32 bodies; the bodies' sums over the warps are added in warp order.
 // Every body meets the nodes it meets with one warp, and the result does not
 // depend on timing.
-template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1>
+template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1, bool kSoft = false>
 __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_masked_kernel(FParams p)
 {
     static_assert(kTeam == 1 || kLearn == kLearnNone, "collection records one warp per group");
@@ -204,7 +202,6 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
     }
     const float theta2f = (float)p.theta2;
     const double theta2 = p.theta2, soft2 = p.soft2;
-    const bool nosoft = (__double_as_longlong(soft2) << 1) == 0;  // soft2 is +-0
     if (kFP64) {
         sm.bpos[w][0][lane] = x;
         sm.bpos[w][1][lane] = y;
@@ -659,8 +656,8 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
                                    own_chain_accepts(dx, dy, dz, soft2, theta2, sm.side2d[kMaxDepth - 1]);
                     }
                     double sc;
-                    if (!(soft::scale(dx, dy, dz, r.w, sc) && nosoft) && take)
-                        sc = fp64_scale(dx, dy, dz, soft2, r.w);
+                    if ((kSoft || !soft::scale(dx, dy, dz, r.w, sc)) && take)
+                        sc = fp64_scale(fma(dx, dx, fma(dy, dy, fma(dz, dz, kSoft ? soft2 : 0.0))), r.w);
                     if (!take) sc = 0.0;
                     sx = fma(sc, dx, sx);
                     sy = fma(sc, dy, sy);
@@ -811,10 +808,10 @@ int grid_n(int64_t n)
     return (int)(b > 8 * bh::num_sms() ? 8 * bh::num_sms() : b);
 }
 
-template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1>
+template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1, bool kSoft = false>
 int launch_walk(bh_context* ctx, const FParams& p)
 {
-    auto kernel = traverse_masked_kernel<kFP64, kLearn, kGroup, kTeam>;
+    auto kernel = traverse_masked_kernel<kFP64, kLearn, kGroup, kTeam, kSoft>;
     const size_t smem = sizeof(WalkSmem<kFP64, kLearn, kGroup, kTeam>);
     BH_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // The plain walks keep their working set in shared memory and L2 (L1
@@ -829,6 +826,17 @@ int launch_walk(bh_context* ctx, const FParams& p)
     kernel<<<(unsigned)blocks, kTeam > 1 ? 32 * kTeam : kThreads, smem, ctx->stream>>>(p);
     BH_LAUNCH_CHECK(ctx);
     return BH_OK;
+}
+
+// The list form: with softening r^-3 comes from the FP64 pipe (soft::scale
+// forms r^2 from the displacement alone).  One kernel for both formed it twice:
+// forces at 300,149 bodies 3.65 -> 3.37 ms with softening, 1.89 -> 1.76 without;
+// at 19,054 1.09 -> 0.97 and 0.72 -> 0.71.
+template <int kTeam>
+int launch_list(bh_context* ctx, const FParams& p)
+{
+    return p.soft2 == 0.0 ? launch_walk<true, kLearnNone, false, kTeam>(ctx, p)
+                          : launch_walk<true, kLearnNone, false, kTeam, true>(ctx, p);
 }
 
 }  // namespace
@@ -922,9 +930,9 @@ int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2
     //     0.083 / 0.072.
     const int64_t per_sm = (ctx->n + 32 * (int64_t)num_sms() - 1) / (32 * (int64_t)num_sms());
     if (fp64) {
-        if (per_sm <= 2) return launch_walk<true, kLearnNone, false, 16>(ctx, p);
-        if (per_sm <= 10) return launch_walk<true, kLearnNone, false, 4>(ctx, p);
-        return launch_walk<true, kLearnNone>(ctx, p);
+        if (per_sm <= 2) return launch_list<16>(ctx, p);
+        if (per_sm <= 10) return launch_list<4>(ctx, p);
+        return launch_list<1>(ctx, p);
     }
     if (group) {
         if (per_sm <= 2) return launch_walk<false, kLearnNone, true, 16>(ctx, p);
