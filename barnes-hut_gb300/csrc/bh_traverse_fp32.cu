@@ -272,11 +272,11 @@ __global__ void __launch_bounds__(kTeam > 1 ? 32 * kTeam : kThreads) traverse_ma
             unsigned m_r = 0;
             bool has;
             if (kTeam > 1) {
-                R = sp < kTeamPop * kTeam ? sp : kTeamPop * kTeam;
-                const int r = sp - 1 - (kTeamPop * w + (lane >> 3));
+                R = sp > team_soft(kTeam) ? 1 : sp < kTeamPop * kTeam ? sp : kTeamPop * kTeam;
+                const int r = kTeamPop * w + (lane >> 3);
                 has = false;
-                if (r >= 0) {
-                    const int2 ent = stk[r];
+                if (r < R) {
+                    const int2 ent = stk[sp - 1 - r];
                     has = (lane & 7) <= (int)((unsigned)ent.x >> kSlotBits);
                     node = (ent.x & ((1 << kSlotBits) - 1)) + (lane & 7);
                     m_r = (unsigned)ent.y;

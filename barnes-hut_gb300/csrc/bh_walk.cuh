@@ -31,9 +31,16 @@ constexpr float kAbsErr = 1e-6f;  // bound on FP32 coordinate error, relative to
 enum { kLearnNone = 0, kLearnInfer = 1, kLearnCollect = 2 };
 
 // A team of warps sharing one group's walk (see traverse_masked_kernel): its
-// sibling ranges, of which the warps take kTeamPop each per round.
+// sibling ranges, of which the warps take kTeamPop each per round.  A range is
+// of at most eight nodes and leaves one range for each, so a round adds at most
+// 7 kTeamPop team of them.  Above team_soft() it takes one range only, which is
+// a depth-first walk: at most 7 more for each of the 21 branching depths.  So
+// the stack cannot pass kTeamStack.  (Uniform lattices of pairs at theta 0
+// reach 960 ranges; full nodes stacked round after round pass any bound without
+// this.)
 constexpr int kTeamStack = 2048;
 constexpr int kTeamPop = 4;
+constexpr int team_soft(int team) { return kTeamStack - 7 * kTeamPop * team - 7 * kMaxDepth; }
 
 // Per-block shared memory of the walk.  Tables a variant does not use shrink
 // to one element, so that the FP32 walk fits 8 blocks (32 warps) per SM; the
