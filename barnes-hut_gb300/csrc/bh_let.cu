@@ -1098,7 +1098,6 @@ extern "C" int bh_let_direct_accelerations(bh_context* ctx, const uint64_t* pref
                                                          ctx->ax, ctx->ay, ctx->az);
         BH_LAUNCH_CHECK(ctx);
     }
-    if (acc_out) return bh::download_accelerations(ctx, acc_out);
-    BH_CUDA_TRY(cudaStreamSynchronize(st));
-    return BH_OK;
+    if (acc_out && (rc = bh::download_accelerations(ctx, acc_out))) return rc;
+    return bh::finish(ctx, "bh_let_direct_accelerations");
 }
