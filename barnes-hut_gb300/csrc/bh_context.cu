@@ -2,7 +2,6 @@
 // transfers, the hot path stage by stage, the step loop and the stateless
 // host-buffer entry points.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -11,6 +10,7 @@
 #include <vector>
 
 #include "bh_internal.cuh"
+#include "bh_per_device.h"
 
 namespace {
 
@@ -149,15 +149,13 @@ void collect_phases(bh_context* ctx);
 // Waits for the stream and turns a raised device error word into a status.
 int bh::num_sms()
 {
-    constexpr int kMaxDevices = 64;
-    static std::atomic<int> cache[kMaxDevices];
+    static bh::PerDevice sms;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 1;
-    int v = cache[dev].load(std::memory_order_relaxed);
-    if (v > 0) return v;
-    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) return 1;
-    cache[dev].store(v, std::memory_order_relaxed);
-    return v;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    return sms.get(dev, 1, [dev] {
+        int v = 0;
+        return cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? v : 0;
+    });
 }
 
 int bh::finish(bh_context* ctx, const char* fn)

@@ -18,6 +18,7 @@
 #include <utility>
 
 #include "bh_internal.cuh"
+#include "bh_per_device.h"
 
 namespace bh {
 namespace {
@@ -465,10 +466,14 @@ int launch_cluster_sort_items(int n, int C, int per, const uint64_t* in, uint64_
     return BH_OK;
 }
 
-// Blocks of the largest cluster: kCMax where the device has room for one.
+// Blocks of the current device's largest cluster: kCMax where it has room for
+// one; asked once per device.
 int cluster_blocks_max()
 {
-    static const int most = [] {
+    static PerDevice most;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+    return most.get(dev, kCPortable, [] {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kCMax);
         cfg.blockDim = dim3(kCThreads);
@@ -489,8 +494,7 @@ int cluster_blocks_max()
             cudaOccupancyMaxActiveClusters(&clusters, cluster_sort_kernel<8>, &cfg) == cudaSuccess && clusters > 0;
         cudaGetLastError();
         return fits ? kCMax : kCPortable;
-    }();
-    return most;
+    });
 }
 
 // 1 <= n, !sort_uses_hist(n); in and out may be the same.
