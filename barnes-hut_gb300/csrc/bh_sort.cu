@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) onesweep_kernel(
     }
 }
 
-// Small sets: one cluster of 1 to 8 blocks holds all keys in its shared
+// Small sets: one cluster of 1 to 16 blocks holds all keys in its shared
 // memory.  The onesweep passes above cost a launch, a look-back chain and a
 // trip through memory each, 60 us and more however few the keys are; here a
 // pass is two cluster barriers around a scatter over the blocks' shared
@@ -248,10 +248,17 @@ __global__ void __launch_bounds__(kTileThreads, 2) onesweep_kernel(
 //
 // The high 32 bits of the key are sorted first, in four passes.  Morton keys
 // equal there share a cell of the tenth level, so in most sets few are left to
-// order: runs of equal high bits up to kTieRun long are ordered by insertion (stable, as the passes
-// are), and a set with a longer run is sorted again by all eight digits.
-// Sort phase per step, before -> after: 1,000 keys 71 -> 15 us, 19,054 92 -> 29,
-// 65,536 95 -> 47 (68 with 8 blocks, 79 with key and payload as two words).
+// order.  Runs of equal high bits are then ordered in place: up to kTieRun keys
+// by a thread's insertion (stable, as the passes are), up to kTieWarp by a
+// warp.  With a longer run the set is sorted by all eight digits instead; where
+// a sample of the keys shows that (an outlier makes the box wide for the rest,
+// and the LET codes of the upper cells have no high bits), at once.
+// Sort phase per step, us, before -> after: 1,000 keys 71 -> 14, 19,054 92 -> 28,
+// 65,536 95 -> 48 (68 with 8 blocks, 79 with key and payload as two words).
+// With one body at 200 / 1,000 / 10,000 AU (runs of 20 / 331 / 33,623 keys at
+// 65,537): 60 / 70 / 69 (onesweep 93), and 103 / 102 / 97 when every run above
+// kTieRun had the set sorted by four digits and then by eight; at 98,304 83 / 86
+// / 84 (93), and 129 / 127 / 120 so.
 // At the large end the remote stores bound it (a block's 4,096 words in 2.3 us
 // a pass); staging a pass's words in digit order before they leave the block
 // gained nothing.
@@ -261,11 +268,17 @@ constexpr int kCMax = 16;      // blocks, where the device takes clusters beyond
 constexpr int kCPortable = 8;
 constexpr int kBlockKeys = 8192;
 // With 16 blocks the cluster is ahead of the onesweep passes up to here (sort and
-// key phases together, us: 65,537 keys 102 / 59, 98,304 103 / 74, 110,000 107 /
-// 82 with a step 1 % faster, 131,000 108 / 91 with a step 2 % slower); three
-// rounds, where long ties are left, take three times as long.
+// key phases together, us: 65,537 keys 102 / 59, 98,304 103 / 75, 110,000 107 /
+// 82 with a step 1 % faster, 131,000 108 / 91 with a step 2 % slower; with
+// long ties 98,304 107 / 100).
 constexpr int64_t kClusterSortMax = 98304;
 constexpr int kTieRun = 16;
+constexpr int kTieWarp = 256;  // the words of a warp's row of warp_mask
+constexpr int kSampleSlots = 2 * kCMax * kRadix;  // 16-bit counters in `totals`
+// The sample takes 1 to 2 us.  Below three keys to a thread (32,768) all twelve
+// passes stay under the onesweep ones without it (19,054 keys 63 and 91 us).
+constexpr int kSampleItems = 3;
+constexpr int kMaxTieRuns = kBlockKeys / (kTieRun + 1) + 1;  // longer than kTieRun, starting in one block
 constexpr int kHistRow = kRadix + 2;  // 129 words: the four quarters of a digit's column fall in four bank groups
 
 struct ClusterSmem {
@@ -276,7 +289,9 @@ struct ClusterSmem {
     uint32_t base[kRadix];           // where the block's keys of a digit go
     uint32_t scan[kRadix / 32];
     int flags[kCMax];
+    int tied, runs;
 };
+static_assert(kMaxTieRuns <= kCMax * kRadix, "the list of runs in `totals`");
 
 template <int I>
 __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per, const uint64_t* keys_in,
@@ -287,6 +302,7 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
     ClusterSmem& s = *reinterpret_cast<ClusterSmem*>(smem_raw);
     const cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks(), r = (int)cluster.block_rank();
+    constexpr bool kSample = I >= kSampleItems;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int start = r * per;
     const int cnt = n - start < 0 ? 0 : (n - start < per ? n - start : per);
@@ -304,19 +320,33 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
     };
     const auto half = [&](int g) { return (uint32_t)(*at(g) >> 32); };
     // A run of equal high halves that starts at g: its length up to
-    // kTieRun + 1, 0 if none starts here or it is one key.
+    // kTieWarp + 1, 0 if none starts here or it is one key.
     const auto run_at = [&](int g) {
         const uint32_t t = half(g);
         if (g + 1 >= n || half(g + 1) != t || (g > 0 && half(g - 1) == t)) return 0;
         int e = g + 2;
         while (e < n && e - g <= kTieRun && half(e) == t) ++e;
+        if (e - g <= kTieRun || e == n || half(e) != t) return e - g;
+        int end = n < g + kTieWarp + 1 ? n : g + kTieWarp + 1;  // e is in the run; [e + 1, end] holds its end
+        for (++e; e < end;) {
+            const int mid = (e + end) / 2;
+            if (half(mid) == t) e = mid + 1;
+            else end = mid;
+        }
         return e - g;
     };
 
     for (int k = threadIdx.x; k < kCWarps * kRadix; k += kCThreads) (&s.warp_mask[0][0])[k] = 0;
+    if (threadIdx.x == 0) s.runs = 0;
+    if (kSample) {
+        for (int k = threadIdx.x; k < kSampleSlots / 2; k += kCThreads) (&s.totals[0][0])[k] = 0;
+        __syncthreads();
+    }
     // Round 0 sorts by the high halves; rounds 1 and 2, where needed, by the
     // low and then by the high halves.
     for (int round = 0; round < 3; ++round) {
+        uint32_t sample = 0;  // the high half of one of the thread's keys
+        bool sampled = false;
 #pragma unroll
         for (int k = 0; k < I; ++k) {
             const int i = k * kCThreads + threadIdx.x;
@@ -324,9 +354,28 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
                 const uint32_t v = round == 2 ? (uint32_t)s.words[i] : (uint32_t)(start + i);
                 const uint64_t key = keys_in[v];
                 s.words[i] = (round == 1 ? key << 32 : key >> 32 << 32) | v;
+                if (k == (int)(threadIdx.x % I)) {
+                    sample = (uint32_t)(key >> 32);
+                    sampled = true;
+                }
             }
         }
+        if (kSample && round == 0) {
+            // Long ties show in a sample of one key in I, evenly spread: the
+            // keys of a high half (or, rarely, of two that share a counter)
+            // are then as many as half of kTieWarp neighbours would give.
+            uint32_t* slots = &s.totals[0][0];
+            const uint32_t h = sample * 0x9E3779B1u >> 19;
+            static_assert(kSampleSlots == 1 << 13 && kCThreads < 1 << 16, "13 bits of the hash, 16-bit counters");
+            if (sampled) atomicAdd(&slots[h >> 1], 1u << 16 * (h & 1));
+            __syncthreads();
+            const int count = sampled ? (int)(slots[h >> 1] >> 16 * (h & 1) & 0xFFFFu) : 0;
+            const int tied = __syncthreads_or(I * count > kTieWarp / 2);
+            if (threadIdx.x == 0) s.tied = tied;
+        }
         sync();
+        if (kSample && round == 0 && __syncthreads_or((int)threadIdx.x < C && *cluster.map_shared_rank(&s.tied, threadIdx.x)))
+            continue;
         for (int shift = 32; shift < 64; shift += 8) {
             // Warp w holds positions w*32*I + k*32 + lane of the block.
             uint64_t word[I];
@@ -391,12 +440,15 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
         }
         if (round != 0) continue;
 
-        // Ties of the high halves: a thread takes the runs that start at its
-        // positions.  flags: 1 a short run, 2 a long one.
+        // Ties of the high halves: a thread looks for runs that start at its
+        // positions.  flags: 1 up to kTieWarp long, 2 longer.  Runs above
+        // kTieRun go to a list (in `totals`), for the warps.
         int f = 0;
         for (int i = threadIdx.x; i < cnt; i += kCThreads) {
             const int len = run_at(start + i);
-            if (len) f |= len > kTieRun ? 2 : 1;
+            if (len) f |= len > kTieWarp ? 2 : 1;
+            if (len > kTieRun && len <= kTieWarp)
+                (&s.totals[0][0])[atomicAdd(&s.runs, 1)] = (uint32_t)(start + i) | (uint32_t)len << 17;
         }
         const int shorts = __syncthreads_or(f & 1), longs = __syncthreads_or(f & 2);
         if ((int)threadIdx.x < C)
@@ -408,6 +460,7 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
         if (any) {
             for (int i = threadIdx.x; i < cnt; i += kCThreads) {
                 const int g = start + i, len = run_at(g);
+                if (len > kTieRun) continue;
                 for (int e = g + 1; e < g + len; ++e) {
                     const uint64_t x = *at(e);
                     const uint32_t xl = (uint32_t)keys_in[(uint32_t)x];
@@ -419,6 +472,36 @@ __global__ void __launch_bounds__(kCThreads) cluster_sort_kernel(int n, int per,
                     }
                     *at(j) = x;
                 }
+            }
+            // A warp to a run: a key's place is the number of keys before it,
+            // by the low halves and then by the order they stand in.
+            for (int k = w; k < s.runs; k += kCWarps) {
+                const uint32_t run = (&s.totals[0][0])[k];
+                const int g = (int)(run & 0x1FFFFu), len = (int)(run >> 17);
+                uint32_t* low = s.warp_mask[w];
+                constexpr int kPer = kTieWarp / 32;
+                uint64_t x[kPer];
+                uint32_t mine[kPer], place[kPer] = {};
+#pragma unroll
+                for (int q = 0; q < kPer; ++q) {
+                    const int i = 32 * q + lane;
+                    if (i >= len) continue;
+                    x[q] = *at(g + i);
+                    low[i] = mine[q] = (uint32_t)keys_in[(uint32_t)x[q]];
+                }
+                __syncwarp();
+                for (int j = 0; j < len; ++j) {
+                    const uint32_t v = low[j];
+#pragma unroll
+                    for (int q = 0; q < kPer; ++q) {
+                        if (32 * q >= len) break;
+                        if (32 * q + lane < len && (v < mine[q] || (v == mine[q] && j < 32 * q + lane))) ++place[q];
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < kPer; ++q)
+                    if (32 * q + lane < len) *at(g + (int)place[q]) = x[q];
+                __syncwarp();
             }
         }
         sync();
