@@ -919,8 +919,13 @@ int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2
     // fill the chip, a team where they do not (forces in ms, theta 1.05, with
     // teams of 1 / 4 / 8 / 16):
     //   FP64 list: 45,000 bodies 0.49 / 0.45 / 0.64 / 1.10 (65,537: 0.54 /
-    //     0.62), 19,054 1.83 / 0.76 / 0.83 / 0.87, 12,000 1.50 / 0.59 / 0.59 /
-    //     0.53, 1,000 0.40 / 0.16 / 0.12 / 0.08;
+    //     0.62); without an outer belt and with one, 4 / 8 / 16: 19,054 0.71 /
+    //     0.74 / 1.28 and 0.19 / 0.26 / 0.53, 12,000 0.57 / 0.54 / 0.78 and 0.18 /
+    //     0.20 / 0.35, 9,800 0.50 / 0.35 / 0.64 and 0.17 / 0.15 / 0.29, 9,000 0.48 /
+    //     0.31 / 0.59 and 0.18 / 0.15 / 0.28, 1,000 0.16 / 0.12 / 0.13 and 0.10 /
+    //     0.09 / 0.12: 8 up to 72 bodies to an SM (10,944), ahead or even at theta
+    //     0.7 as well; softened (FP64 factors), 4,864 0.41 / 0.27 / 0.21 and 0.14 /
+    //     0.13 / 0.13, 6,000 0.46 / 0.34 / 0.35 and 0.15 / 0.14 / 0.20;
     //   FP32: 200,000 0.285 / 0.275 / 0.36 / 0.64 (300,149: 0.370 / 0.395),
     //     30,000 0.128 / 0.069 / 0.083 / 0.118, 19,054 0.45 / 0.20 / 0.15 /
     //     0.16, 8,000 0.32 / 0.14 / 0.09 / 0.08, 1,000 0.11 / 0.06 / 0.045 /
@@ -930,7 +935,8 @@ int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2
     //     0.083 / 0.072.
     const int64_t per_sm = (ctx->n + 32 * (int64_t)num_sms() - 1) / (32 * (int64_t)num_sms());
     if (fp64) {
-        if (per_sm <= 2) return launch_list<16>(ctx, p);
+        if (per_sm <= 1 && soft2 != 0.0) return launch_walk<true, kLearnNone, false, 16, true>(ctx, p);
+        if (ctx->n <= 72 * (int64_t)num_sms()) return launch_list<8>(ctx, p);
         if (per_sm <= 10) return launch_list<4>(ctx, p);
         return launch_list<1>(ctx, p);
     }

@@ -52,7 +52,7 @@ def bodies(leaves, n):
 
 
 # team, rounds of piling up, bodies, form
-@pytest.mark.parametrize("team,rounds,n,mode", [(16, 4, 4612, "list"), (16, 5, 9728, "far"), (16, 4, 5000, "group"),
+@pytest.mark.parametrize("team,rounds,n,mode", [(8, 8, 4612, "list"), (16, 5, 9728, "far"), (16, 4, 5000, "group"),
                                                 (8, 8, 9729, "far"), (8, 9, 24320, "group")])
 def test_full_stack(bh, team, rounds, n, mode):
     leaves, most = piled_up(team, rounds)
