@@ -28,7 +28,7 @@ and seeded (the reference's 300k CSV is not part of its repository).
   against the FP32 far field over a theta sweep (1.05-2.0) and FP32 + learned
   criterion at several per-body error budgets (network trained first on 20
   seeded 1M-body systems, ~10M pairs, by the engine's GPU kernels); the
-  line's top-level benchmark spec object summarises it (learned against plain
+  the benchmark spec object summarises it (learned against plain
   FP64 at equal or lower error, and against the fastest theta-only run at
   the learned run's error) with the FP32 walk's roofline.
 * learned_eval: the learned criterion on 5 unseen 1M-body systems at the
@@ -48,6 +48,9 @@ and seeded (the reference's 300k CSV is not part of its repository).
   split over 8 ranks, against the oracle on the host cores.
 * csv_ingest: readCSV of a 1M-body file on the GPU against the host reader.
   --no-extras skips these seven blocks; --blocks a,b runs only those.
+
+The result is one JSON line on standard output; hbm_phases, the benchmark spec and the
+blocks are one JSON line each on standard error, before it.
 
 Multi-GPU: the path does not shard on one GPU per rank; ranks run replicas
 (weak scaling) and value is the sum of their body-steps over the slowest
@@ -1021,7 +1024,6 @@ def run_ours(args, rank, ws, local):
                      "traffic_unit": "bytes per launch (ncu)",
                      "hbm_view": hbm_view(TRAFFIC_BYTES.get((args.mode, n)), force_ms)},
         "phases_ms_per_step": {kk: v / k for kk, v in phases.items()},
-        "hbm_phases": hbm_phases({kk: v / k for kk, v in phases.items()}, n),
         "interactions_per_body": inter_per_step / n,
         "interactions_per_s": inter_per_step / (force_ms * 1e-3),
         "accuracy": accuracy,
@@ -1030,6 +1032,9 @@ def run_ours(args, rank, ws, local):
         "gpu_launches": launches,
         "clocks": clk.summary((w0, w1)),
         "cpu_baseline": cpu,
+    }
+    print_result(line, {
+        "hbm_phases": hbm_phases({kk: v / k for kk, v in phases.items()}, n),
         "north_star": ns.get("north_star") if ns else None,
         "forms_4m": ns,
         "learned_eval": le,
@@ -1038,8 +1043,25 @@ def run_ours(args, rank, ws, local):
         "long_runs": runs,
         "let_exchange": let,
         "csv_ingest": ingest,
-    }
-    print(json.dumps(line), flush=True)
+    })
+
+
+def rounded(x):
+    """x with every number below the first level to six significant digits."""
+    if isinstance(x, dict):
+        return {k: rounded(v) for k, v in x.items()}
+    if isinstance(x, list):
+        return [rounded(v) for v in x]
+    return float(f"{x:.6g}") if isinstance(x, float) else x
+
+
+def print_result(line, blocks):
+    """The result as one line of a few KB on standard output (records keep only
+    the end of a long one), after the blocks, one line each on standard error."""
+    for name, block in blocks.items():
+        if block is not None:
+            print(json.dumps({name: block}), file=sys.stderr, flush=True)
+    print(json.dumps({k: v if isinstance(v, float) else rounded(v) for k, v in line.items()}), flush=True)
 
 
 def barrier(ws):
