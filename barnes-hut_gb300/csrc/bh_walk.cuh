@@ -45,7 +45,7 @@ constexpr int team_soft(int team) { return kTeamStack - 7 * kTeamPop * team - 7 
 // Per-block shared memory of the walk.  Tables a variant does not use shrink
 // to one element, so that the FP32 walk fits 8 blocks (32 warps) per SM; the
 // FP64 walk fits 5 (6 with shorter lists ran slower: 1.92 ms against 1.87 at
-// 300,149 bodies).
+// 300,149 bodies, in the kernel that served softened calls as well).
 template <bool kFP64, int kLearn, bool kGroup = false, int kTeam = 1>
 struct WalkSmem {
     static constexpr int kWarps = kTeam > 1 ? kTeam : bh::kWarps;  // per block

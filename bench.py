@@ -699,8 +699,8 @@ def forms_4m(args, dev, params, scale, info):
 # DRAM traffic per launch of the force kernel (dram__bytes_read.sum +
 # dram__bytes_write.sum) from one ncu --set full capture of that kernel on
 # that workload, keyed by (mode, bodies).
-TRAFFIC_BYTES = {("fp64_list", 300_149): 44.91e6 + 0.41e6, ("fp32", 4_000_000): 482.41e6 + 183.02e6,
-                 ("fp32_group", 4_000_000): 483.43e6 + 183.40e6}
+TRAFFIC_BYTES = {("fp64_list", 300_149): 44.92e6 + 0.45e6, ("fp32", 4_000_000): 483.24e6 + 182.95e6,
+                 ("fp32_group", 4_000_000): 482.85e6 + 183.18e6}
 
 # Algorithmic bytes per body of the HBM-bound phases: the minimum traffic of
 # each phase's work (reads + writes of its inputs and outputs once).
@@ -1019,7 +1019,8 @@ def run_ours(args, rank, ws, local):
         "roofline": {"kernel": KERNEL[mode], "bound": fp, "achieved": achieved,
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "peak_source": f"measured in-process: {fp.upper()} FMA chains (bh_measure_fma_peak)",
-                     "work": f"{FLOPS_PER_INTERACTION} flops x {inter_per_step:.4g} interactions per launch",
+                     "work": f"{FLOPS_PER_INTERACTION} flops x {inter_per_step:.4g} interactions per launch"
+                             + (", most of them on the integer pipes" if mode <= 1 else ""),
                      "traffic": TRAFFIC_BYTES.get((args.mode, n)),
                      "traffic_unit": "bytes per launch (ncu)",
                      "hbm_view": hbm_view(TRAFFIC_BYTES.get((args.mode, n)), force_ms)},
