@@ -915,40 +915,51 @@ int launch_traverse_masked(bh_context* ctx, double theta, double G, double soft2
     int rc = prepare_walk(ctx, theta, G, soft2, fp64, p);
     if (rc) return rc;
     p.kick_h = kick_h;
-    // Warps per group, by the groups of 32 bodies each SM gets: one where they
-    // fill the chip, a team where they do not (forces in ms, theta 1.05, with
-    // teams of 1 / 4 / 8 / 16):
-    //   FP64 list: 45,000 bodies 0.49 / 0.45 / 0.64 / 1.10 (65,537: 0.54 /
-    //     0.62); without an outer belt and with one, 4 / 8 / 16: 19,054 0.71 /
-    //     0.74 / 1.28 and 0.19 / 0.26 / 0.53, 12,000 0.57 / 0.54 / 0.78 and 0.18 /
-    //     0.20 / 0.35, 9,800 0.50 / 0.35 / 0.64 and 0.17 / 0.15 / 0.29, 9,000 0.48 /
-    //     0.31 / 0.59 and 0.18 / 0.15 / 0.28, 1,000 0.16 / 0.12 / 0.13 and 0.10 /
-    //     0.09 / 0.12: 8 up to 72 bodies to an SM (10,944), ahead or even at theta
-    //     0.7 as well; softened (FP64 factors), 4,864 0.41 / 0.27 / 0.21 and 0.14 /
-    //     0.13 / 0.13, 6,000 0.46 / 0.34 / 0.35 and 0.15 / 0.14 / 0.20;
-    //   FP32: 200,000 0.285 / 0.275 / 0.36 / 0.64 (300,149: 0.370 / 0.395),
-    //     30,000 0.128 / 0.069 / 0.083 / 0.118, 19,054 0.45 / 0.20 / 0.15 /
-    //     0.16, 8,000 0.32 / 0.14 / 0.09 / 0.08, 1,000 0.11 / 0.06 / 0.045 /
-    //     0.039;
-    //   FP32 group: 65,537 0.115 / 0.107 / 0.14 / 0.22 (100,003: 0.141 /
-    //     0.145), 30,000 0.100 / 0.063 / 0.083 / 0.119, 8,000 0.22 / 0.11 /
-    //     0.083 / 0.072.
-    const int64_t per_sm = (ctx->n + 32 * (int64_t)num_sms() - 1) / (32 * (int64_t)num_sms());
+    // Warps per group: one where the groups of 32 bodies fill the chip, a team
+    // where they do not.  A team's rounds leave lanes idle, which costs the more
+    // the shorter the walk is: at a wide angle, and in systems without the long
+    // walks that the planets' places give an inner belt.  Forces with a team over
+    // those with one warp, without an outer belt / with one / with one and a body
+    // at 1,000 AU / in a uniform cube:
+    //   FP32, theta 1.05, 4 warps: 30,000 bodies 0.51 / 0.57 / 0.72 / 0.72, 70,000
+    //     0.72 / 0.87 / 0.94 / 1.00, 120,000 0.87 / 0.97 / 1.05 / 1.23, 204,288 0.87
+    //     / 1.02 / 1.16 / 1.25; theta 1.3: 70,000 0.73 / 0.92 / 1.07 / 1.21, 120,000
+    //     0.85 / 1.04 / 1.12 / 1.44; theta 0.8: 204,288 0.90 / 0.94 / 1.03 / 1.08;
+    //     8 warps: 19,054 0.34 / 0.57 / 0.65 / 0.69 (4: 0.46 / 0.60 / 0.66 / 0.68),
+    //     24,320 0.44 / 0.74 / 0.93 / 1.02 (4: 0.48 / 0.60 / 0.67 / 0.71), 9,728
+    //     0.30 / 0.51 / 0.59 / 0.65 (16: 0.24 / 0.52 / 0.63 / 0.70);
+    //   FP32 group, theta 1.05, 4 warps: 30,000 0.60 / 0.67 / 0.81 / 0.82, 70,000
+    //     0.81 / 0.99 / 1.08 / 1.24, 87,552 0.89 / 1.05 / 1.20 / 1.28; theta 1.3:
+    //     40,000 0.69 / 1.01 / 1.14 / 1.22; 8 and 16 warps as above;
+    //   FP64 list, theta 1.05, 4 warps: 30,000 0.66 / 0.71 / 0.84 / 0.95, 48,640
+    //     0.85 / 0.99 / 1.12 / 1.24; theta 1.3: 40,000 0.68 / 0.92 / 1.16 / 1.48,
+    //     48,640 0.86 / 1.11 / 1.44 / 1.55; 8 warps: 9,728 0.25 / 0.45 / 0.54 /
+    //     0.58 (4: 0.38 / 0.55 / 0.54 / 0.60; 16: 0.46 / 0.88 / 1.09 / 1.36), 10,944
+    //     0.36 / 0.54 / 0.67 / 0.83 (4: 0.40 / 0.51 / 0.53 / 0.59); softened (FP64
+    //     factors), ms with 4 / 8 / 16: 4,864 0.41 / 0.27 / 0.21 and 0.14 / 0.13 /
+    //     0.13, 6,000 0.46 / 0.34 / 0.35 and 0.15 / 0.14 / 0.20.
+    // The lines are where the systems without an outer belt and with one, taken
+    // together, break even up to theta 1.3.  Above it the walks get shorter (theta
+    // 2, with an outer belt, 4 warps: FP32 30,000 bodies 0.88, 40,000 1.1, 150,000
+    // 1.33; group 30,000 0.92; list 19,054 0.98, 24,320 1.28) and the lines move
+    // with it.
+    const double bodies = (double)ctx->n / num_sms();  // to an SM
+    const double wide = theta > 1.3 ? theta * theta / (1.3 * 1.3) : 1.0;
     if (fp64) {
-        if (per_sm <= 1 && soft2 != 0.0) return launch_walk<true, kLearnNone, false, 16, true>(ctx, p);
-        if (ctx->n <= 72 * (int64_t)num_sms()) return launch_list<8>(ctx, p);
-        if (per_sm <= 10) return launch_list<4>(ctx, p);
+        if (bodies <= 32.0 && soft2 != 0.0) return launch_walk<true, kLearnNone, false, 16, true>(ctx, p);
+        if (bodies <= 64.0) return launch_list<8>(ctx, p);
+        if (bodies * wide <= 320.0) return launch_list<4>(ctx, p);
         return launch_list<1>(ctx, p);
     }
     if (group) {
-        if (per_sm <= 2) return launch_walk<false, kLearnNone, true, 16>(ctx, p);
-        if (per_sm <= 5) return launch_walk<false, kLearnNone, true, 8>(ctx, p);
-        if (per_sm <= 18) return launch_walk<false, kLearnNone, true, 4>(ctx, p);
+        if (bodies <= 64.0) return launch_walk<false, kLearnNone, true, 16>(ctx, p);
+        if (bodies <= 128.0) return launch_walk<false, kLearnNone, true, 8>(ctx, p);
+        if (bodies * wide * wide <= 576.0) return launch_walk<false, kLearnNone, true, 4>(ctx, p);
         return launch_walk<false, kLearnNone, true>(ctx, p);
     }
-    if (per_sm <= 2) return launch_walk<false, kLearnNone, false, 16>(ctx, p);
-    if (per_sm <= 5) return launch_walk<false, kLearnNone, false, 8>(ctx, p);
-    if (per_sm <= 42) return launch_walk<false, kLearnNone, false, 4>(ctx, p);
+    if (bodies <= 64.0) return launch_walk<false, kLearnNone, false, 16>(ctx, p);
+    if (bodies <= 128.0) return launch_walk<false, kLearnNone, false, 8>(ctx, p);
+    if (bodies * wide * wide <= 1344.0) return launch_walk<false, kLearnNone, false, 4>(ctx, p);
     return launch_walk<false, kLearnNone>(ctx, p);
 }
 
